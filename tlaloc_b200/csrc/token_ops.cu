@@ -1,62 +1,131 @@
 // Token ids into rows and rows into token ids (ir/.../inference/HfDecoderGraph.kt: embedding :904-909; greedy next token): what every
 // model of the framework begins and ends a step with.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace tlaloc_b200 {
 namespace {
 
-template <typename TT>
-__global__ void EmbeddingKernel(const TT* table, const int* ids, float* out, int vocab, int dim)
+namespace cg = cooperative_groups;
+constexpr int kEmbedThreads = 128, kArgmaxThreads = 512, kArgmaxCluster = 8;
+
+// A row of the table widened to f32, sixteen bytes of it per thread: blockIdx.y counts stretches of the row.  A single CTA walking a row
+// element by element was a chain of dim / 256 dependent trips (128 rows of 8192: 16.7 us; this form 3.8 us, 5.2 MB of traffic).
+template <typename TT, bool VEC>
+__global__ void __launch_bounds__(kEmbedThreads) EmbeddingKernel(const TT* table, const int* ids, float* out, int vocab, int dim)
 {
+  constexpr int kPer = 16 / static_cast<int>(sizeof(TT));
   GridDependencySync();
-  const int p = blockIdx.x;
+  const int p = blockIdx.x, d0 = (blockIdx.y * kEmbedThreads + threadIdx.x) * kPer;
+  if (d0 >= dim) return;
   int v = __ldg(ids + p);
   v = v < 0 ? 0 : (v >= vocab ? vocab - 1 : v);
-  const TT* src = table + static_cast<size_t>(v) * dim;
-  for (int d = threadIdx.x; d < dim; d += blockDim.x) out[static_cast<size_t>(p) * dim + d] = ToF32(src[d]);
+  const TT* src = table + static_cast<size_t>(v) * dim + d0;
+  float* dst = out + static_cast<size_t>(p) * dim + d0;
+  if (VEC) {
+    const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(src));  // L2: an f32 table may be rows that the kernel before has written
+    const TT* e = reinterpret_cast<const TT*>(&raw);
+#pragma unroll
+    for (int i = 0; i < kPer; i += 4) {
+      *reinterpret_cast<float4*>(dst + i) = make_float4(ToF32(e[i]), ToF32(e[i + 1]), ToF32(e[i + 2]), ToF32(e[i + 3]));
+    }
+  } else {
+    for (int i = 0; i < kPer && d0 + i < dim; ++i) dst[i] = ToF32(src[i]);
+  }
 }
 
-// One CTA per row; the first index of the maximum wins (DxirInterpreter.kt:2414-2426).
-__global__ void __launch_bounds__(256) ArgmaxKernel(const float* x, int* out, int n)
+// The larger of two candidates, the lower index of two equal ones.  NaN is never larger.
+__device__ __forceinline__ void TakeLarger(float& best, int& idx, float v, int j)
+{
+  if (v > best || (v == best && j < idx)) {
+    best = v;
+    idx = j;
+  }
+}
+
+// A cluster per row; the first index of the maximum wins (DxirInterpreter.kt:2414-2426).  The row is bound by latency, not by its bytes
+// (32768 columns are 128 KB), so it is spread over up to eight CTAs whose threads have all their 16-byte loads in flight at once; one CTA a
+// row, reading 128 elements a thread one after the other, took 30 us where this takes 4.
+__global__ void __launch_bounds__(kArgmaxThreads) ArgmaxKernel(const float* x, int* out, int n, int per, int vec)
 {
   GridDependencySync();
-  __shared__ float bv[8];
-  __shared__ int bi[8];
+  constexpr int kWarps = kArgmaxThreads / 32, kUnroll = 8;
+  __shared__ float bv[kWarps];
+  __shared__ int bi[kWarps];
+  __shared__ float cv[kArgmaxCluster];
+  __shared__ int ci[kArgmaxCluster];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank()), ranks = static_cast<int>(cluster.num_blocks());
   const float* xr = x + static_cast<size_t>(blockIdx.x) * n;
+  const int lo = rank * per, hi = min(n, lo + per), tid = threadIdx.x;
   float best = -INFINITY;
   int idx = 0x7fffffff;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const float v = xr[j];
-    if (v > best || (v == best && j < idx)) {
-      best = v;
-      idx = j;
-    }
-  }
+  if (vec) {
+    for (int j0 = lo + tid * 4; j0 < hi; j0 += kArgmaxThreads * 4 * kUnroll) {
+      float4 v[kUnroll];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ov > best || (ov == best && oi < idx)) {
-      best = ov;
-      idx = oi;
+      for (int u = 0; u < kUnroll; ++u) {
+        const int j = j0 + u * kArgmaxThreads * 4;
+        if (j < hi) v[u] = __ldcg(reinterpret_cast<const float4*>(xr + j));
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int j = j0 + u * kArgmaxThreads * 4;
+        if (j < hi) {
+          TakeLarger(best, idx, v[u].x, j);
+          TakeLarger(best, idx, v[u].y, j + 1);
+          TakeLarger(best, idx, v[u].z, j + 2);
+          TakeLarger(best, idx, v[u].w, j + 3);
+        }
+      }
     }
+  } else {
+    for (int j = lo + tid; j < hi; j += kArgmaxThreads) TakeLarger(best, idx, xr[j], j);
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
+  auto across = [&](int from) {
+    for (int o = from; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+      TakeLarger(best, idx, ov, oi);
+    }
+  };
+  across(16);
   if (lane == 0) {
     bv[warp] = best;
     bi[warp] = idx;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
-      if (bv[w] > best || (bv[w] == best && bi[w] < idx)) {
-        best = bv[w];
-        idx = bi[w];
-      }
-    }
-    // A row of NaNs (or an empty comparison) leaves idx unset: the interpreter's answer is index 0.
-    out[blockIdx.x] = idx == 0x7fffffff ? 0 : idx;
+  if (warp == 0) {
+    best = lane < kWarps ? bv[lane] : -INFINITY;
+    idx = lane < kWarps ? bi[lane] : 0x7fffffff;
+    across(kWarps / 2);
   }
+  if (ranks > 1) {
+    cluster.sync();  // rank 0 runs: its shared memory may be written
+    if (tid == 0) {
+      cluster.map_shared_rank(cv, 0)[rank] = best;
+      cluster.map_shared_rank(ci, 0)[rank] = idx;
+    }
+    cluster.sync();
+    if (rank != 0) return;
+    if (tid == 0) {
+      for (int r = 1; r < ranks; ++r) TakeLarger(best, idx, cv[r], ci[r]);
+    }
+  }
+  // A row of NaNs (or an empty comparison) leaves idx unset: the interpreter's answer is index 0.
+  if (tid == 0) out[blockIdx.x] = idx == 0x7fffffff ? 0 : idx;
+}
+
+template <typename TT>
+cudaError_t LaunchEmbedding(const void* table, const int32_t* ids, float* out, int positions, int vocab, int dim, cudaStream_t st)
+{
+  constexpr int kPer = 16 / static_cast<int>(sizeof(TT));
+  const dim3 grid(positions, (dim + kEmbedThreads * kPer - 1) / (kEmbedThreads * kPer));
+  const TT* t = static_cast<const TT*>(table);
+  return dim % kPer == 0 && Aligned16(table) && Aligned16(out) ? LaunchChained(EmbeddingKernel<TT, true>, grid, kEmbedThreads, 0, st, t, ids, out, vocab, dim)
+                                                             : LaunchChained(EmbeddingKernel<TT, false>, grid, kEmbedThreads, 0, st, t, ids, out, vocab, dim);
 }
 
 }  // namespace
@@ -72,12 +141,8 @@ extern "C" int tlaloc_b200_embedding(const void* table, int32_t table_dtype, con
   if (positions < 0 || vocab < 1 || dim < 1) return Fail(kInvalid, "EMBEDDING: bad sizes");
   if (positions == 0) return kOk;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
-  if (table_dtype == TLALOC_B200_F32) {
-    e = LaunchChained(EmbeddingKernel<float>, positions, 256, 0, st, static_cast<const float*>(table), ids, out, vocab, dim);
-  } else {
-    e = LaunchChained(EmbeddingKernel<__nv_bfloat16>, positions, 256, 0, st, static_cast<const __nv_bfloat16*>(table), ids, out, vocab, dim);
-  }
+  const cudaError_t e = table_dtype == TLALOC_B200_F32 ? LaunchEmbedding<float>(table, ids, out, positions, vocab, dim, st)
+                                                       : LaunchEmbedding<__nv_bfloat16>(table, ids, out, positions, vocab, dim, st);
   if (e != cudaSuccess) return CudaFail("EMBEDDING launch", e);
   CountLaunches(1);
   return kOk;
@@ -88,7 +153,18 @@ extern "C" int tlaloc_b200_argmax(const float* logits, int32_t* out, int32_t row
   if (!logits || !out) return Fail(kInvalid, "ARGMAX: a required device pointer is null");
   if (rows < 0 || n < 1) return Fail(kInvalid, "ARGMAX: bad sizes");
   if (rows == 0) return kOk;
-  const cudaError_t e = LaunchChained(ArgmaxKernel, rows, 256, 0, static_cast<cudaStream_t>(stream), logits, out, n);
+  // At least 4096 columns a CTA: two 16-byte loads per thread, below which another CTA costs more than it takes over.
+  int ranks = 1;
+  while (ranks < kArgmaxCluster && n >= ranks * 2 * 4096) ranks *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows, ranks);
+  cfg.blockDim = dim3(kArgmaxThreads);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attrs[2];
+  cfg.numAttrs = ChainAttributes(attrs, ranks);
+  cfg.attrs = attrs;
+  const int per = ((n + ranks - 1) / ranks + 3) / 4 * 4;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, ArgmaxKernel, logits, out, static_cast<int>(n), per, n % 4 == 0 && Aligned16(logits) ? 1 : 0);
   if (e != cudaSuccess) return CudaFail("ARGMAX launch", e);
   CountLaunches(1);
   return kOk;
