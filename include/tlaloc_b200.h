@@ -327,8 +327,8 @@ typedef struct tlaloc_b200_dense_problem {
 
 /*
  * `count` (1 or 2) projections of the same m rows (or of `rows` of their own) in one launch where a tensor-core kernel takes them, else one launch
- * each.  dtype: F32 or BF16, the type of x and w of every problem; y is F32 or BF16 per problem.  F32 runs in true f32 (FMA,
- * no reduced-precision products).  flags: TLALOC_B200_GEMM_WEIGHTS_CONST.  Two problems of one call must not depend on
+ * each.  dtype: F32 or BF16, the type of x and w of every problem; y is F32 or BF16 per problem.  F32 products are exact
+ * to the last place of f32 (on the tensor cores: each operand as three bf16 parts, the sums no further from 64 bits than f32 FMAs in k order).  flags: TLALOC_B200_GEMM_WEIGHTS_CONST.  Two problems of one call must not depend on
  * each other's results.
  */
 int tlaloc_b200_dense_gemm(const tlaloc_b200_dense_problem* problems, int32_t count, int32_t dtype, int32_t m, int32_t flags,

@@ -1,0 +1,96 @@
+"""The f32 projection on the tensor cores against f64: edges of its tiles, chunks and slices, its distance from f64 beside the plain kernel's, operands
+that its parts cannot hold (needs a B200)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(autouse=True)
+def no_wait_runs_out():
+    yield
+    from tlaloc_b200 import _native
+
+    torch.cuda.synchronize()
+    assert _native.lib().tlaloc_b200_device_status() == 0
+
+
+def ops():
+    from tlaloc_b200 import ops as o
+
+    return o
+
+
+def rand(*shape, seed=0):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed + sum(shape))
+    return torch.randn(shape, device=DEV, generator=g)
+
+
+def bound(x, w):
+    """Every addition loses at most 2^-23 of what it holds: k / 32 rounded ones of chunks, and 16 inside a chunk, whose size is at most the
+    sum of magnitudes."""
+    k = x.shape[-1]
+    return (k / 32 + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().transpose(-1, -2)) + 1e-30
+
+
+# rows: one tile of 16 .. 208, then equal parts; n, k: remainders of 128 columns and of chunks of 32 and 64, two chunks and fewer
+@pytest.mark.parametrize("m", [1, 15, 17, 32, 33, 64, 65, 127, 129, 193, 208, 209, 500])
+@pytest.mark.parametrize("n,k", [(1, 4), (128, 64), (200, 100), (1344, 192), (130, 1028)])
+def test_tiles_and_chunks(m, n, k):
+    x, w, b, r = rand(m, k), rand(n, k, seed=1), rand(n, seed=2), rand(m, n, seed=3)
+    y = torch.full((m + 1, n), 7.0, device=DEV)
+    ops().dense_gemm(ops().dense(x, w, y[:m]))
+    want = x.double() @ w.double().T
+    assert bool(((y[:m].double() - want).abs() <= bound(x, w)).all()) and bool((y[m] == 7).all())
+    want = (want + b.double()).clamp_min(0) ** 2 + r.double()
+    tol = bound(x, w) * (2 * want.abs().sqrt() + 1) + 2.0 ** -20 * (want.abs() + 1)
+    ops().dense_gemm(ops().dense(x, w, r, bias=b, act=1, residual=r), weights_const=True)
+    assert bool(((r.double() - want).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("m", [3, 40, 100, 203])
+@pytest.mark.parametrize("k", [2048, 10304])
+def test_no_further_from_f64_than_plain_sums(m, k):
+    x, w = rand(m, k), rand(256, k, seed=1)
+    want = x.double() @ w.double().T
+    y, plain = torch.empty((m, 256), device=DEV), torch.empty((m, 256), device=DEV)
+    ops().dense_gemm(ops().dense(x, w, y))
+    before = ops().set_order_faithful(True)
+    try:
+        ops().dense_gemm(ops().dense(x, w, plain))
+    finally:
+        ops().set_order_faithful(before)
+    assert float((y - want).norm()) <= float((plain - want).norm())
+
+
+@pytest.mark.parametrize("m", [5, 150])
+def test_what_the_parts_cannot_hold(m):
+    """Infinities, NaN, f32's largest numbers and subnormal ones give what f32 gives, in their rows and columns alone."""
+    x, w = rand(m, 96), rand(140, 96, seed=1)
+    x[0, 3], x[1, 5], x[2, 7], x[3] = float("inf"), float("nan"), 3.4e38, x[3] * 1e-36
+    w[:, 7] *= 0.1
+    w[17, 9], w[18] = -float("inf"), 0.0
+    y = torch.empty((m, 140), device=DEV)
+    ops().dense_gemm(ops().dense(x, w, y))
+    want = x.double() @ w.double().T
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf()) and torch.equal(y[y.isinf()].double(), want[want.isinf()])
+    fine = want.isfinite()
+    assert bool(((y.double() - want).abs() <= bound(x, w).nan_to_num(0, 0, 0))[fine].all())
+
+
+@pytest.mark.parametrize("sizes", [[0, 3, 40, 0, 70, 1], [5] * 64, [300, 0]])
+@pytest.mark.parametrize("act", [0, 2])
+def test_groups(sizes, act):
+    o, n, k = ops(), 192, 160
+    rows = sum(sizes)
+    x, w = rand(rows, k), rand(len(sizes), n, k, seed=1)
+    offsets = torch.tensor([0] + sizes, device=DEV).cumsum(0).int()
+    y = torch.full((rows + 1, n // 2 if act else n), 7.0, device=DEV)
+    o.dense_gemm(o.grouped_dense(x, w, y[:rows], offsets, act=act))
+    z = torch.cat([x[a:b].double() @ w[e].double().T for e, (a, b) in enumerate(zip(offsets[:-1].tolist(), offsets[1:].tolist()))])
+    if act:
+        z = z.view(rows, -1, 2, 16)
+        z = (z[:, :, 0] * torch.sigmoid(z[:, :, 0]) * z[:, :, 1]).reshape(rows, -1)
+    assert float((y[:rows].double() - z).norm() / z.norm()) < 1e-6 and bool((y[rows] == 7).all())

@@ -2,8 +2,8 @@
 // tlaloc_b200_dense_gemm): the entry point, and the kernel that takes any size and type.
 //
 // DenseGemmTiled: 64 x 64 output tiles, 256 threads with 4 x 4 outputs each, k in steps of 16 through shared memory as
-// f32, plain FMA in k order.  It is the whole of the f32 path (true f32 products and sums) and the fallback of the bf16
-// path for sizes and strides the tensor-core kernels do not take.
+// f32, plain FMA in k order: order-faithful runs, and the sizes and strides that the tensor-core kernels (dense_gemm_tc.cu for bf16,
+// dense_gemm_f32.cu) do not take.
 #include "common.cuh"
 #include "dense_gemm.cuh"
 
@@ -120,7 +120,13 @@ extern "C" int tlaloc_b200_dense_gemm(const tlaloc_b200_dense_problem* problems,
     e = LaunchDenseGemmTc(problems, count, m, (flags & TLALOC_B200_GEMM_WEIGHTS_CONST) != 0, st);
     launches = 1;
   }
-  for (int i = 0; i < count && e == cudaSuccess && !tc; ++i) {
+  bool split = dtype == TLALOC_B200_F32 && !OrderFaithful();
+  for (int i = 0; i < count; ++i) split = split && DenseGemmF32Applies(problems[i], m);
+  if (split) {
+    e = LaunchDenseGemmF32(problems, count, m, (flags & TLALOC_B200_GEMM_WEIGHTS_CONST) != 0, st);
+    launches = 1;
+  }
+  for (int i = 0; i < count && e == cudaSuccess && !tc && !split; ++i) {
     e = dtype == TLALOC_B200_F32 ? LaunchTiled<float>(problems[i], m, st) : LaunchTiled<__nv_bfloat16>(problems[i], m, st);
     ++launches;
   }

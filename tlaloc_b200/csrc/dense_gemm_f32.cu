@@ -1,0 +1,658 @@
+// The f32 projection on the tensor cores (include/tlaloc_b200.h, tlaloc_b200_dense_gemm): every f32 operand is the exact sum of three
+// bf16 numbers (8 + 8 + 8 bits of its 24), and the six products of parts that reach f32's last place run as tcgen05.mma kind::f16.
+//
+// Accuracy.  Products of parts are exact; what is left out (middle x low, low x low) is below 2^-26 of a product and of either sign.  An
+// accumulator in TMEM holds one chunk of 32 k only, its small products first and its large ones last; the chunks are summed in registers with
+// rounding to nearest.  So a sum of k products has k / 32 rounded additions where the plain kernel (dense_gemm.cu) has k, and its error
+// against 64 bits (2-norm, relative) is the smaller one at every k: k = 128: 0.7e-7 and the plain kernel's 2.0e-7; 2048: 1.2e-7, 8.1e-7; 10304: 1.6e-7, 1.8e-6.
+// An infinity, a NaN or a number above bf16's largest makes a part infinite and the sum NaN or infinite, and a sum below 1e-28 may have met
+// parts in bf16's subnormal range: such an output is computed again with plain FMAs.
+//
+// D[n, m] = sum_k W[n, k] X[m, k]: 128 weight rows are the MMA's M, a tile of up to 208 activation rows its N.
+//   producer lane boxes of 32 k of both operands by TMA (f32, 128-byte swizzle), two to eight stages ahead
+//   sixteen warps split a chunk of 32 k into the three planes (128-byte swizzle; a buffer is one half of the planes' rows)
+//   MMA lane      the six products of a chunk, into one of two accumulators
+//   eight warps   add the finished accumulator to sums in registers (104 a thread at 208 rows, hence the register split), and write the tile
+//   persistent    a CTA walks tiles;   K slices   the slices of a tile are a cluster and sum their partial tiles in rank order
+// Bound at 208 rows by the split and the six products, which run side by side (each alone takes about 100 us of the 115 us of 203 rows, n 18944, k 2048),
+// at few rows by the way of a chunk through the three kinds of warps (0.85 us each).  203 rows, n 2048, k 10304: 86 us, 1414 us with plain FMAs; one
+// row, n 32768, k 2048: 113 us, 443 us.  Every mbarrier wait is bounded.
+#include <cuda.h>
+
+#include "common.cuh"
+#include "dense_gemm.cuh"
+#include "tc_common.cuh"
+
+namespace tlaloc_b200 {
+namespace {
+
+using namespace tc;
+
+constexpr int kBN = 128, kBK = 32, kSumWarps = 8, kSplitWarps = 16, kMmaWarp = kSumWarps + kSplitWarps, kProducerWarp = kMmaWarp + 1;
+constexpr int kThreads = (kMmaWarp + 4) * 32;
+
+// BT: most activation rows of a tile.
+template <int BT>
+struct Layout {
+  static constexpr int kPlane = (kBN + BT) * 128;  // 64 k a row: two buffers of 32
+  static constexpr int kRaw = 3 * kPlane;
+  static constexpr int kStage = (kBN + BT) * 128;
+  static constexpr int kStages = BT == 208 ? 2 : BT == 128 ? 3 : BT == 64 ? 6 : 8;
+  static constexpr int kTileStride = kBN + 4;  // a slice's partial tile [BT][kTileStride] f32, aliases the planes
+  static_assert(kRaw >= BT * kTileStride * 4, "the partial tile aliases the planes");
+  static constexpr int kBars = kRaw + kStages * kStage;
+  static constexpr int kSlot = kBars + 8 * (6 + 2 * kStages);
+  static constexpr int kBytes = kSlot + 8 + 1024;  // slack to align to 1024
+  // Registers a thread of the three kinds of warpgroups; 128 * (2 * sum + 4 * split + mma) is the 896 * 72 of the launch.
+  static constexpr int kSumRegs = 152, kSplitRegs = 40, kMmaRegs = 40;
+  static_assert(128 * (2 * kSumRegs + 4 * kSplitRegs + kMmaRegs) <= kThreads * 72, "more registers than the launch has");
+  static constexpr int kUnits = BT / 16;           // groups of eight activation rows a thread sums
+  static constexpr int kAcc = BT <= 32 ? 32 : BT <= 64 ? 64 : BT <= 128 ? 128 : 256;  // TMEM columns of an accumulator
+};
+
+struct F32Args {
+  tlaloc_b200_dense_problem p[2];
+  int M[2], tiles_m[2], tiles_n[2];
+  int swap_x[2];  // the activations' map has the batch before the rows
+  int tiles0, tiles, ks, bt, weights_const, groups;  // groups: of the last problem, whose tiles are not counted here
+};
+
+__device__ int g_f32_status = 0;  // nonzero after an mbarrier wait timed out (sticky until read)
+
+struct Tile {
+  int pr, n0, m0, b, M;  // M: first row that is not the tile's to write
+};
+__device__ __forceinline__ Tile TileAt(const F32Args& a, int id, const int* start)
+{
+  Tile t;
+  t.pr = id >= a.tiles0 ? 1 : 0;
+  if (t.pr) id -= a.tiles0;
+  const tlaloc_b200_dense_problem& p = a.p[t.pr];
+  if (p.row_offsets != nullptr) {
+    int lo = 0, hi = a.groups;  // start[lo] <= id < start[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (start[mid] <= id) lo = mid;
+      else hi = mid;
+    }
+    id -= start[lo];
+    t.b = lo;
+    const int tiles_m = (start[lo + 1] - start[lo]) / a.tiles_n[t.pr];
+    t.M = min(p.row_offsets[lo + 1], a.M[t.pr]);
+    t.m0 = p.row_offsets[lo] + (id % tiles_m) * a.bt;
+    t.n0 = (id / tiles_m) * kBN;
+    return t;
+  }
+  t.M = a.M[t.pr];
+  t.m0 = (id % a.tiles_m[t.pr]) * a.bt;  // activation tiles of one weight tile run side by side: the weights leave HBM once
+  id /= a.tiles_m[t.pr];
+  t.n0 = (id % a.tiles_n[t.pr]) * kBN;
+  t.b = id / a.tiles_n[t.pr];
+  return t;
+}
+
+// Two f32 as the exact sum of three pairs of bf16, each rounded to nearest from what the parts before it leave.
+__device__ __forceinline__ void Split2(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l)
+{
+  auto pack = [](float u, float v) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(u, v);
+    return *reinterpret_cast<const uint32_t*>(&b);
+  };
+  h = pack(x, y);
+  const float r = x - __uint_as_float(h << 16), s = y - __uint_as_float(h & 0xffff0000u);
+  m = pack(r, s);
+  l = pack(r - __uint_as_float(m << 16), s - __uint_as_float(m & 0xffff0000u));
+}
+
+// One output with plain FMAs; a NaN stays one.
+__device__ __noinline__ float PlainDot(const float* x, const float* w, int k)
+{
+  float v = 0.f;
+  for (int i = 0; i < k && v == v; i += 4) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(x + i)), b = __ldcg(reinterpret_cast<const float4*>(w + i));
+    v = fmaf(a.x, b.x, v);
+    v = fmaf(a.y, b.y, v);
+    v = fmaf(a.z, b.z, v);
+    v = fmaf(a.w, b.w, v);
+  }
+  return v;
+}
+__device__ __forceinline__ bool Doubtful(float v) { return !(fabsf(v) <= 3.4e38f) || (v != 0.f && fabsf(v) < 1e-28f); }
+
+__device__ __forceinline__ const float* XRow(const tlaloc_b200_dense_problem& p, const Tile& t, int m)
+{
+  return static_cast<const float*>(p.x) + (p.row_offsets != nullptr ? 0 : p.batch_x * t.b) + static_cast<size_t>(m) * p.ld_x;
+}
+__device__ __forceinline__ const float* WRow(const tlaloc_b200_dense_problem& p, const Tile& t, int n)
+{
+  return static_cast<const float*>(p.w) + p.batch_w * t.b + static_cast<size_t>(n) * p.k;
+}
+__device__ __forceinline__ void Put(const tlaloc_b200_dense_problem& p, size_t at, float v)
+{
+  if (p.y_dtype == TLALOC_B200_F32) static_cast<float*>(p.y)[at] = v;
+  else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
+}
+
+// CH finished sums of column n (a warp's lanes hold 32 consecutive columns), rows m, m + step, ... below end: epilogue and store.
+template <int CH>
+__device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const Tile& t, int n, int m, int step, int end, float* v)
+{
+  const size_t out = p.row_offsets != nullptr ? 0 : p.batch_y * t.b;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int r = m + c * step;
+    if (n < p.n && r < end && Doubtful(v[c])) v[c] = PlainDot(XRow(p, t, r), WRow(p, t, n), p.k);
+  }
+  if (IsGated(p.act)) {  // gate and other factor are sixteen lanes apart
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int r = m + c * step;
+      const float other = __shfl_xor_sync(0xffffffffu, v[c], kGateBlock);
+      if (n < p.n && r < end && (n & kGateBlock) == 0) {
+        Put(p, out + static_cast<size_t>(r) * p.ld_y + (n >> 5) * kGateBlock + (n & 15), GatedValue(p.act, v[c], other));
+      }
+    }
+    return;
+  }
+  if (n >= p.n) return;
+  const float bias = p.bias != nullptr ? __ldg(p.bias + n) : 0.f;
+  float res[CH];
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int r = m + c * step;
+    res[c] = p.residual != nullptr && r < end ? p.residual[static_cast<size_t>(r) * p.ld_res + n] : 0.f;
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int r = m + c * step;
+    if (r < end) Put(p, out + static_cast<size_t>(r) * p.ld_y + n, DenseActivation(p.act, v[c] + bias) + res[c]);
+  }
+}
+
+__device__ __forceinline__ void ClusterSync()
+{
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void TcLd8(uint32_t taddr, uint32_t* r)
+{
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+
+// The chunks of a tile that a CTA sums: all of them, or the slice of its cluster rank.
+__device__ __forceinline__ int Chunks(const F32Args& a, const Tile& t, int& first)
+{
+  const int nb = (a.p[t.pr].k + kBK - 1) / kBK;
+  if (a.ks <= 1) {
+    first = 0;
+    return nb;
+  }
+  const int per = (nb + a.ks - 1) / a.ks;
+  first = static_cast<int>(blockIdx.y) * per;
+  return max(0, min(per, nb - first));
+}
+
+// x (the k coordinate) is a multiple of 32 f32: always a 16-byte boundary.
+__device__ __forceinline__ void TmaBox3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar, uint64_t policy)
+{
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar), "l"(policy)
+      : "memory");
+}
+
+template <int BT>
+__global__ void __launch_bounds__(kThreads, 1)
+    DenseGemmF32Kernel(const __grid_constant__ CUtensorMap w0, const __grid_constant__ CUtensorMap x0, const __grid_constant__ CUtensorMap w1,
+                       const __grid_constant__ CUtensorMap x1, const __grid_constant__ F32Args a)
+{
+  using L = Layout<BT>;
+  constexpr int S = L::kStages;
+  constexpr uint32_t kCols = 2 * L::kAcc;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ int s_start[kMaxGroups + 1];
+  const uint32_t base = (SmemAddr(smem_raw) + 1023u) & ~1023u;  // the swizzle is a function of address bits 4..9
+  unsigned char* smem = smem_raw + (base - SmemAddr(smem_raw));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t full = base + L::kBars, done = full + 16, empty = done + 16;  // planes written; a chunk's MMAs through; its accumulator added
+  const uint32_t landed = empty + 16, freed = landed + 8 * S;                                      // a stage's boxes are there; split
+  volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(smem + L::kSlot);
+  volatile uint32_t* abort_word = slot + 1;
+  if (tid == 0) {
+    *abort_word = 0u;
+    for (int i = 0; i < 2; ++i) {
+      MbarInit(full + 8 * i, kSplitWarps);
+      MbarInit(done + 8 * i, 1);
+      MbarInit(empty + 8 * i, kSumWarps);
+    }
+    for (int i = 0; i < S; ++i) {
+      MbarInit(landed + 8 * i, 1);
+      MbarInit(freed + 8 * i, kSplitWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(base + L::kSlot), "r"(kCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = *slot;
+  const bool early = a.weights_const != 0 && a.groups == 0;  // the first weights travel before the dependency wait
+  if (!early || warp != kProducerWarp) GridDependencySync();
+  int tiles = a.tiles;
+  if (a.groups > 0) {
+    const int pr = a.p[1].row_offsets != nullptr ? 1 : 0;
+    const int* offsets = a.p[pr].row_offsets;
+    if (warp == 0) {
+      int total = 0;
+      for (int e0 = 0; e0 < a.groups; e0 += 32) {
+        const int e = e0 + lane;
+        int v = e < a.groups ? max(0, (min(offsets[e + 1], a.M[pr]) - offsets[e] + a.bt - 1) / a.bt) * a.tiles_n[pr] : 0;
+        const int own = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += u;
+        }
+        if (e < a.groups) s_start[e] = total + v - own;
+        total += __shfl_sync(0xffffffffu, v, 31);
+      }
+      if (lane == 0) s_start[a.groups] = total;
+    }
+    __syncthreads();
+    tiles += s_start[a.groups];
+  }
+  bool ok = true;
+  int it = 0;  // chunks so far: chunk `it` has buffer and accumulator it & 1
+
+  if (warp >= kMmaWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(L::kMmaRegs));
+    if (warp == kMmaWarp && ElectOne()) {
+      // f32 accumulator, bf16 A and B, both K-major, M = 128
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(a.bt >> 3) << 17) | (8u << 24);
+      const uint64_t wd = SmemDesc(base, 16, 1024), xd = SmemDesc(base + kBN * 128, 16, 1024);
+      for (int id = blockIdx.x; id < tiles; id += gridDim.x) {
+        const Tile t = TileAt(a, id, s_start);
+        int first;
+        const int nb = Chunks(a, t, first);
+        for (int c = 0; c < nb; ++c, ++it) {
+          const int b = it & 1;
+          if (it >= 2) ok = MbarWait(empty + 8 * b, ((it >> 1) - 1) & 1, abort_word) && ok;
+          ok = MbarWait(full + 8 * b, (it >> 1) & 1, abort_word) && ok;
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          const uint32_t acc = tmem + b * L::kAcc;
+          constexpr uint32_t P = L::kPlane >> 4;
+          const uint64_t w = wd + 4 * b, x = xd + 4 * b;
+          // planes high, middle, low: small products first
+          TcMmaBf16(acc, w, x + 2 * P, idesc, 0u);
+          TcMmaBf16(acc, w + 2, x + 2 * P + 2, idesc, 1u);
+          TcMmaBf16(acc, w + 2 * P, x, idesc, 1u);
+          TcMmaBf16(acc, w + 2 * P + 2, x + 2, idesc, 1u);
+          TcMmaBf16(acc, w + P, x + P, idesc, 1u);
+          TcMmaBf16(acc, w + P + 2, x + P + 2, idesc, 1u);
+          TcMmaBf16(acc, w, x + P, idesc, 1u);
+          TcMmaBf16(acc, w + 2, x + P + 2, idesc, 1u);
+          TcMmaBf16(acc, w + P, x, idesc, 1u);
+          TcMmaBf16(acc, w + P + 2, x + 2, idesc, 1u);
+          TcMmaBf16(acc, w, x, idesc, 1u);
+          TcMmaBf16(acc, w + 2, x + 2, idesc, 1u);
+          TcCommit(done + 8 * b);
+        }
+      }
+      if (!ok) atomicExch(&g_f32_status, 1);
+    } else if (warp == kProducerWarp && ElectOne()) {
+      uint64_t w_policy, x_policy;
+      if (a.tiles_m[0] == 1) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(w_policy));
+      else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;\n" : "=l"(w_policy));
+      asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(x_policy));
+      const uint32_t bytes = (kBN + a.bt) * 128;
+      int s = 0, round = 0;  // the next stage, and how often the ring has been around
+      bool waited = !early;
+      for (int id = blockIdx.x; id < tiles; id += gridDim.x) {
+        const Tile t = TileAt(a, id, s_start);
+        int first;
+        const int nb = Chunks(a, t, first);
+        auto load_x = [&](int c, int at) {
+          const int z = a.p[t.pr].row_offsets != nullptr ? 0 : t.b;
+          const bool swap = a.swap_x[t.pr] != 0;
+          TmaBox3d(base + L::kRaw + at * L::kStage + kBN * 128, t.pr ? &x1 : &x0, (first + c) * kBK, swap ? z : t.m0, swap ? t.m0 : z, landed + 8 * at, x_policy);
+        };
+        auto load_w = [&](int c, int at) {
+          MbarExpectTx(landed + 8 * at, bytes);
+          TmaBox3d(base + L::kRaw + at * L::kStage, t.pr ? &w1 : &w0, (first + c) * kBK, t.n0, t.b, landed + 8 * at, w_policy);
+        };
+        int c = 0;
+        if (!waited) {  // constant weights of the first stages travel before the dependency wait; activations only after it
+          const int ahead = min(nb, S);
+          for (int i = 0; i < ahead; ++i) load_w(i, i);
+          GridDependencySync();
+          waited = true;
+          for (; c < ahead; ++c) load_x(c, c);
+          s = ahead == S ? 0 : ahead;
+          round = ahead == S ? 1 : 0;
+        }
+        for (; c < nb; ++c) {
+          if (round > 0) ok = MbarWait(freed + 8 * s, (round - 1) & 1, abort_word) && ok;
+          load_w(c, s);
+          load_x(c, s);
+          if (++s == S) {
+            s = 0;
+            ++round;
+          }
+        }
+      }
+      if (!waited) GridDependencySync();
+      if (!ok) {  // given up: let the copies in flight land before the CTA's shared memory goes away
+        atomicExch(&g_f32_status, 1);
+        volatile uint32_t never = 0;
+        for (int i = 0; i < S; ++i) {
+          const int uses = round + (i < s ? 1 : 0);
+          if (uses > 0) MbarWait(landed + 8 * i, (uses - 1) & 1, &never);
+        }
+      }
+    }
+    __syncwarp();
+    if (a.ks > 1) {
+      ClusterSync();
+      ClusterSync();
+    }
+  } else if (warp >= kSumWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(L::kSplitRegs));
+    // A lane's eight k are two 16-byte words of a row of the stage and one of each plane's; four lanes a row, and the two rows of a phase of
+    // eight lanes differ by 5 in their swizzle, so that neither the loads (words 0 2 4 6 of a row) nor the stores (words 0 - 3, or 4 - 7) collide.
+    const int sw = warp - kSumWarps, u = lane & 3, low = (lane >> 3) ^ ((lane & 4) != 0 ? 5 : 0);
+    const uint32_t from0 = base + L::kRaw + low * 128 + (((2 * u) ^ low) << 4), to0 = base + low * 128 + ((u ^ low) << 4);
+    const int groups = (kBN + a.bt) >> 3;  // of eight rows
+    int s = 0, phase = 0;
+    for (int id = blockIdx.x; id < tiles; id += gridDim.x) {
+      const Tile t = TileAt(a, id, s_start);
+      int first;
+      const int nb = Chunks(a, t, first);
+      for (int c = 0; c < nb; ++c, ++it) {
+        ok = MbarWaitWarp(landed + 8 * s, phase, lane, abort_word) && ok;
+        if (it >= 2) ok = MbarWaitWarp(done + 8 * (it & 1), ((it >> 1) - 1) & 1, lane, abort_word) && ok;
+        const uint32_t from = from0 + s * L::kStage, to = to0 ^ ((it & 1) << 6);
+#pragma unroll
+        for (int i = 0; i < (kBN + BT) / 8; i += kSplitWarps) {
+          const int g = i + sw;
+          if (g >= groups) break;
+          float4 f, h;
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "r"(from + g * 1024));
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(h.x), "=f"(h.y), "=f"(h.z), "=f"(h.w) : "r"((from + g * 1024) ^ 16));
+          uint32_t part[3][4];
+          Split2(f.x, f.y, part[0][0], part[1][0], part[2][0]);
+          Split2(f.z, f.w, part[0][1], part[1][1], part[2][1]);
+          Split2(h.x, h.y, part[0][2], part[1][2], part[2][2]);
+          Split2(h.z, h.w, part[0][3], part[1][3], part[2][3]);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(to + g * 1024 + q * L::kPlane), "r"(part[q][0]), "r"(part[q][1]),
+                         "r"(part[q][2]), "r"(part[q][3])
+                         : "memory");
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          MbarArrive(full + 8 * (it & 1));
+          MbarArrive(freed + 8 * s);
+        }
+        if (++s == S) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    if (!ok) atomicExch(&g_f32_status, 1);
+    if (a.ks > 1) {
+      ClusterSync();
+      ClusterSync();
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(L::kSumRegs));
+    const int quad = warp & 3, col0 = (warp >> 2) * (a.bt >> 1), units = a.bt >> 4;  // this warp's lanes and columns of an accumulator
+    for (int id = blockIdx.x; id < tiles; id += gridDim.x) {
+      const Tile t = TileAt(a, id, s_start);
+      const tlaloc_b200_dense_problem& p = a.p[t.pr];
+      int first;
+      const int nb = Chunks(a, t, first);
+      float acc[L::kUnits][8];
+#pragma unroll
+      for (int q = 0; q < L::kUnits; ++q)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[q][e] = 0.f;
+      for (int c = 0; c < nb; ++c, ++it) {
+        ok = MbarWaitWarp(done + 8 * (it & 1), (it >> 1) & 1, lane, abort_word) && ok;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const uint32_t from = tmem + (static_cast<uint32_t>(quad * 32) << 16) + (it & 1) * L::kAcc + col0;
+#pragma unroll
+        for (int q = 0; q < L::kUnits; q += 2) {
+          if (q < units) {
+            uint32_t r[2][8];
+            TcLd8(from + q * 8, r[0]);
+            if (q + 1 < L::kUnits) TcLd8(from + q * 8 + 8, r[1]);  // within the accumulator's columns also where the tile ends before it
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              acc[q][e] += __uint_as_float(r[0][e]);
+              if (q + 1 < L::kUnits) acc[q + 1 < L::kUnits ? q + 1 : q][e] += __uint_as_float(r[1][e]);
+            }
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) MbarArrive(empty + 8 * (it & 1));
+      }
+      if (a.ks <= 1) {
+#pragma unroll
+        for (int q = 0; q < L::kUnits; ++q)
+          if (q < units) Finish<8>(p, t, t.n0 + quad * 32 + lane, t.m0 + col0 + q * 8, 1, t.M, acc[q]);
+      } else {
+        float* tile = reinterpret_cast<float*>(smem);  // over the planes: every MMA of this CTA's one tile is through
+#pragma unroll
+        for (int q = 0; q < L::kUnits; ++q) {
+          if (q < units) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) tile[(col0 + q * 8 + e) * L::kTileStride + quad * 32 + lane] = acc[q][e];
+          }
+        }
+      }
+    }
+    if (!ok) atomicExch(&g_f32_status, 1);
+    if (a.ks > 1) {
+      ClusterSync();  // every slice's tile is in its CTA's shared memory
+      cg::cluster_group cluster = cg::this_cluster();
+      const Tile t = TileAt(a, blockIdx.x, s_start);
+      const tlaloc_b200_dense_problem& p = a.p[t.pr];
+      const int nl = tid & 127, nr = static_cast<int>(cluster.num_blocks()), rows = min(a.bt, t.M - t.m0), step = 2 * nr;
+      float* tile = reinterpret_cast<float*>(smem);
+      constexpr int kU = 8;
+      for (int c0 = static_cast<int>(cluster.block_rank()) + nr * (tid >> 7); c0 < rows; c0 += kU * step) {
+        float v[kU] = {};
+        for (int q = 0; q < nr; ++q) {
+          const float* peer = cluster.map_shared_rank(tile, q) + nl;
+          float w[kU];
+#pragma unroll
+          for (int e = 0; e < kU; ++e) w[e] = c0 + e * step < rows ? peer[(c0 + e * step) * L::kTileStride] : 0.f;
+#pragma unroll
+          for (int e = 0; e < kU; ++e) v[e] += w[e];
+        }
+        Finish<kU>(p, t, t.n0 + nl, t.m0 + c0, step, t.m0 + rows, v);
+      }
+      ClusterSync();  // no CTA leaves while a peer may still read its tile
+    }
+    asm volatile("bar.sync 1, 256;\n" ::: "memory");
+    if (warp == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols) : "memory");
+    }
+  }
+}
+
+// ---- host -----------------------------------------------------------------------------------------------------------
+
+int g_slots[kMaxDevices][9];  // resident CTAs when launched as clusters of ks
+
+cudaError_t PrepareDenseF32()
+{
+  static OncePerDevice once;
+  return once.Run([](int device) {
+    TensorMapEncoder();
+    cudaError_t e = cudaSuccess;
+#define TLALOC_OPT_IN(BT) \
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(DenseGemmF32Kernel<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT>::kBytes)
+    TLALOC_OPT_IN(32);
+    TLALOC_OPT_IN(64);
+    TLALOC_OPT_IN(128);
+    TLALOC_OPT_IN(208);
+#undef TLALOC_OPT_IN
+    if (e != cudaSuccess) return e;
+    for (int ks = 1; ks <= 8; ++ks) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(148, ks, 1);
+      cfg.blockDim = dim3(kThreads, 1, 1);
+      cfg.dynamicSmemBytes = Layout<128>::kBytes;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1;
+      attr[0].val.clusterDim.y = ks;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, DenseGemmF32Kernel<128>, &cfg) != cudaSuccess || clusters <= 0) {
+        cudaGetLastError();
+        clusters = (ks <= 2 ? 148 : ks <= 4 ? 128 : 112) / ks;
+      }
+      g_slots[device][ks] = clusters * ks;
+    }
+    return cudaSuccess;
+  });
+}
+
+int ReadF32Status()
+{
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_f32_status, sizeof(int)) != cudaSuccess) return -1;
+  if (v != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_f32_status, &zero, sizeof(int));
+  }
+  return v;
+}
+KernelSetup g_setup(PrepareDenseF32, ReadF32Status);
+
+// K slices (1..8) of tiles with k of nb times 64, in microseconds: 64 k take 3.6 us at 208 rows and 1.7 us at
+// few; a tile's start and end cost about 3 us, a cluster's sum 2 us and more with its ranks.
+int ChooseSlices(long long tiles, int nb, int bt)
+{
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) device = 0;
+  const double chunk = fmax(1.7, 3.6 * bt / 208);
+  int best = 1;
+  double best_cost = 1e30;
+  for (int ks = 1; ks <= 8; ++ks) {
+    if (ks > 1 && nb / ks < 2) break;
+    const int slots = g_slots[device][ks] > 0 ? g_slots[device][ks] : 148 / ks * ks;
+    const long long waves = (tiles * ks + slots - 1) / slots;
+    const double cost = waves * ((nb + ks - 1) / ks * chunk + 3.0 + (ks > 1 ? 1.5 + 0.2 * ks : 0.0));
+    if (cost < best_cost * 0.97) {
+      best_cost = cost;
+      best = ks;
+    }
+  }
+  return best;
+}
+
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// f32 [batch][rows][k] with strides in elements, boxes of 32 k x box_rows rows; the dimension with the smaller stride comes first (*swap: the batch).
+bool EncodeMatrix(CUtensorMap* map, const void* ptr, int64_t k, int64_t rows, int64_t batch, int64_t ld, int64_t batch_stride, uint32_t box_rows, int* swap)
+{
+  auto encode = reinterpret_cast<EncodeTiledFn>(TensorMapEncoder());
+  if (encode == nullptr) return false;
+  *swap = batch > 1 && batch_stride < ld ? 1 : 0;
+  if (batch == 1) batch_stride = ld;
+  const cuuint64_t r_dim = static_cast<cuuint64_t>(rows), b_dim = static_cast<cuuint64_t>(batch);
+  const cuuint64_t r_str = static_cast<cuuint64_t>(ld) * 4, b_str = static_cast<cuuint64_t>(batch_stride) * 4;
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(k), *swap ? b_dim : r_dim, *swap ? r_dim : b_dim};
+  const cuuint64_t strides[2] = {*swap ? b_str : r_str, *swap ? r_str : b_str};
+  const cuuint32_t box[3] = {kBK, *swap ? 1u : box_rows, *swap ? box_rows : 1u};
+  const cuuint32_t elem[3] = {1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BT>
+cudaError_t Launch(const CUtensorMap* maps, const F32Args& a, int ctas, cudaStream_t st)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas, a.ks, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = Layout<BT>::kBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  cfg.numAttrs = ChainAttributes(attr, a.ks > 1 ? a.ks : 0);
+  cfg.attrs = attr;
+  return cudaLaunchKernelEx(&cfg, DenseGemmF32Kernel<BT>, maps[0], maps[1], maps[2], maps[3], a);
+}
+
+}  // namespace
+
+bool DenseGemmF32Applies(const tlaloc_b200_dense_problem& p, int m)
+{
+  const long long rows = p.rows > 0 ? p.rows : m;
+  return p.k % 4 == 0 && p.ld_x % 4 == 0 && Aligned16(p.x) && Aligned16(p.w) && (p.batch == 1 || (p.batch_x % 4 == 0 && p.batch_w % 4 == 0)) &&
+         (rows / 16 + p.batch + 1) * ((p.n + kBN - 1) / kBN) * (p.row_offsets != nullptr ? 1 : p.batch) < (1ll << 30);
+}
+
+cudaError_t LaunchDenseGemmF32(const tlaloc_b200_dense_problem* problems, int count, int m, bool weights_const, cudaStream_t st)
+{
+  cudaError_t e = PrepareDenseF32();
+  if (e != cudaSuccess) return e;
+  // Rows of a tile: what the problem has in equal parts of up to 208, or what a group has on average (one that has more takes several tiles).
+  int typical = 1, nb = 1 << 30;
+  for (int i = 0; i < count; ++i) {
+    const int rows = problems[i].rows > 0 ? problems[i].rows : m;
+    typical = max(typical, problems[i].row_offsets != nullptr ? (rows + problems[i].batch - 1) / problems[i].batch : rows);
+    nb = min(nb, (problems[i].k + 63) / 64);
+  }
+  const int parts = (typical + 207) / 208;
+  CUtensorMap maps[4];
+  F32Args a = {};
+  a.bt = ((typical + parts - 1) / parts + 15) / 16 * 16;
+  a.weights_const = weights_const ? 1 : 0;
+  for (int i = 0; i < count; ++i) {
+    const tlaloc_b200_dense_problem& s = problems[i];
+    a.p[i] = s;
+    a.M[i] = s.rows > 0 ? s.rows : m;
+    int swap_w = 0;
+    if (!EncodeMatrix(&maps[2 * i], s.w, s.k, s.n, s.batch, s.k, s.batch_w, kBN, &swap_w) || swap_w ||
+        !EncodeMatrix(&maps[2 * i + 1], s.x, s.k, a.M[i], s.row_offsets != nullptr ? 1 : s.batch, s.ld_x, s.batch_x, a.bt, &a.swap_x[i])) {
+      return cudaErrorInvalidValue;
+    }
+    a.tiles_m[i] = (a.M[i] + a.bt - 1) / a.bt;
+    a.tiles_n[i] = (s.n + kBN - 1) / kBN;
+    if (s.row_offsets != nullptr) a.groups = s.batch;
+    else a.tiles += a.tiles_n[i] * a.tiles_m[i] * s.batch;
+    if (i == 0) a.tiles0 = s.row_offsets != nullptr ? 1 << 30 : a.tiles;
+  }
+  if (count == 1) {
+    maps[2] = maps[0];
+    maps[3] = maps[1];
+  }
+  a.ks = a.groups > 0 ? 1 : ChooseSlices(a.tiles, nb, a.bt);
+  const int ctas = a.groups > 0 ? 148 : a.ks > 1 ? a.tiles : min(a.tiles, 148);
+  if (a.bt <= 32) return Launch<32>(maps, a, ctas, st);
+  if (a.bt <= 64) return Launch<64>(maps, a, ctas, st);
+  if (a.bt <= 128) return Launch<128>(maps, a, ctas, st);
+  return Launch<208>(maps, a, ctas, st);
+}
+
+}  // namespace tlaloc_b200
