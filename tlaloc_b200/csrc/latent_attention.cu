@@ -1,5 +1,7 @@
 // Attention of absorbed queries over a paged pool of latents (include/tlaloc_b200.h, tlaloc_b200_latent_attention).
 //
+// LatentAttentionF32: f32 rows of up to 512 + 128 channels, multiples of four.  See there.
+//
 // LatentAttentionGeneric: any sizes, f32 or bf16, plain FMA.  A CTA serves one (row, head): tiles of 128 positions, a warp
 // per position for the scores (lanes over the channels), an online softmax in f32, then a thread per latent channel.
 //
@@ -115,6 +117,266 @@ __global__ void __launch_bounds__(kGenericThreads) LatentAttentionGeneric(Latent
     if (j >= p.kv_rank) break;
     out[j] = FromF32<T>(acc[c] * inv);
   }
+}
+
+// ---- the f32 form -----------------------------------------------------------------------------------------------------
+// Sixteen heads of one row over a slice of its positions.  A tile of 16 positions arrives in shared memory (cp.async, three stages); a warp owns four
+// heads and eight positions of each tile: its lanes hold the four queries and the four outputs spread over the channels, so a cached row is
+// read from shared memory once for the scores and once for the output of four heads, a 16-byte word for 16 FMAs, and the FMA pipe (paired
+// f32x2 FMAs) bounds it.  The 32 scores of a tile meet in the 32 lanes (a reduce-scatter of 31 shuffles).  203 rows of 16 heads, 512 + 64 channels,
+// 300 to 1000 positions: 161 us; 868 us with a CTA per (row, head) that walks every position's row alone (LatentAttentionGeneric).  A test of every word for
+// the row's end instead of zeros behind it: 267 us.
+constexpr int kF32Tile = 16, kF32Heads = 16, kF32Threads = 256, kF32Stages = 3;
+
+struct F32Slices {
+  float* records;  // [slices][T][H][kv_rank + 2], or null: one slice, straight to out
+  int slices, slice_tiles;
+};
+
+__device__ __forceinline__ uint64_t Fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t Pair(float a, float b)
+{
+  return static_cast<uint64_t>(__float_as_uint(a)) | (static_cast<uint64_t>(__float_as_uint(b)) << 32);
+}
+__device__ __forceinline__ float Low(uint64_t a) { return __uint_as_float(static_cast<uint32_t>(a)); }
+__device__ __forceinline__ float High(uint64_t a) { return __uint_as_float(static_cast<uint32_t>(a >> 32)); }
+
+// NW, NV: 16-byte words of a cached row and of its latent part per lane.
+template <int NW, int NV>
+__global__ void __launch_bounds__(kF32Threads, 1) LatentAttentionF32(LatentParams p, F32Slices sp)
+{
+  GridDependencySync();
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ float4 s_p[kF32Threads / 32][8];
+  constexpr int kRow = NW * 32;  // words of a row in shared memory, zeros past its own: no lane asks where the row ends
+  ulonglong2* ring = reinterpret_cast<ulonglong2*>(smem_raw);  // [stages][16 positions][kRow]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
+  const int slice = blockIdx.x, h0 = blockIdx.y * kF32Heads + quad * 4, t = blockIdx.z;
+  const int words = p.row >> 2, vwords = p.kv_rank >> 2;
+  const int2 live = LiveRange(p, t);
+  const int tile0 = live.x / kF32Tile + slice * sp.slice_tiles;
+  const int n = min((live.y + kF32Tile - 1) / kF32Tile, tile0 + sp.slice_tiles) - tile0;
+  if (n <= 0 && sp.records != nullptr) return;  // an empty slice writes nothing
+  const int* table = TableOf(p, t);
+  const float* pool = static_cast<const float*>(p.pool);
+  // Two rows of a tile a warp; where they are is looked up a tile before they are fetched.
+  const float* next[2];
+  auto find = [&](int j) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      next[r] = pool;
+      if (j < n) next[r] += PoolRow(p, table, min(max((tile0 + j) * kF32Tile + warp * 2 + r, live.x), live.y - 1));
+    }
+  };
+  auto fetch = [&](int j) {
+    if (j < n) {
+      const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(ring + (j % kF32Stages) * (kF32Tile * kRow)));
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        for (int w = lane; w < words; w += 32) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + ((warp * 2 + r) * kRow + w) * 16), "l"(next[r] + w * 4) : "memory");
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    find(j + 1);
+  };
+  for (int i = tid; i < kF32Stages * kF32Tile * kRow; i += kF32Threads)
+    if (i % kRow >= words) ring[i] = make_ulonglong2(0, 0);
+  find(0);
+  fetch(0);
+  fetch(1);
+  uint64_t q[4][NW][2], acc[4][NV][2];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const float* src = static_cast<const float*>(p.query) + (static_cast<size_t>(t) * p.H + h0 + h) * p.row;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      const int w = lane + 32 * i;
+      const ulonglong2 v = h0 + h < p.H && w < words ? __ldcg(reinterpret_cast<const ulonglong2*>(src) + w) : make_ulonglong2(0, 0);
+      q[h][i][0] = v.x;
+      q[h][i][1] = v.y;
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) acc[h][i][0] = acc[h][i][1] = 0;
+  }
+  // This lane's score of a tile: position lane >> 2 of the warp's eight, head lane & 3; its running maximum is the head's, its sum its own.
+  float top = -INFINITY, sum = 0.f;
+  for (int j = 0; j < n; ++j) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // tile j is there, and everyone is through with the one whose place j + 2 takes
+    fetch(j + 2);
+    const int pos0 = (tile0 + j) * kF32Tile + half * 8;
+    if (pos0 >= live.y || pos0 + 8 <= live.x) continue;
+    const ulonglong2* tile = ring + ((j % kF32Stages) * kF32Tile + half * 8) * kRow + lane;
+    float s[32];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint64_t d[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const ulonglong2 k = tile[i * kRow + 32 * w];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) d[h] = Fma2(q[h][w][1], k.y, Fma2(q[h][w][0], k.x, d[h]));
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) s[i * 4 + h] = Low(d[h]) + High(d[h]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {  // lane i ends up with the sum of s[i] over the lanes
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const float give = upper ? s[i] : s[i + o], keep = upper ? s[i + o] : s[i];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    const int pos = pos0 + (lane >> 2);
+    const bool seen = pos >= live.x && pos < live.y;
+    const float score = s[0] * p.scale;
+    float most = seen ? score : -INFINITY;
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+    const float next = fmaxf(top, most), keep = expf(top - next), weight = seen ? expf(score - next) : 0.f;
+    top = next;
+    sum = fmaf(sum, keep, weight);
+    reinterpret_cast<float*>(s_p[warp])[lane] = weight;
+    __syncwarp();
+    if (__any_sync(0xffffffffu, keep != 1.f)) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float f = __shfl_sync(0xffffffffu, keep, h);
+        const uint64_t f2 = Pair(f, f);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          acc[h][i][0] = Fma2(acc[h][i][0], f2, 0);
+          acc[h][i][1] = Fma2(acc[h][i][1], f2, 0);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 w4 = s_p[warp][i];  // zeros for a position that is not live, whose row is a live one's
+      const uint64_t w2[4] = {Pair(w4.x, w4.x), Pair(w4.y, w4.y), Pair(w4.z, w4.z), Pair(w4.w, w4.w)};
+#pragma unroll
+      for (int w = 0; w < NV; ++w) {
+        const ulonglong2 v = tile[i * kRow + 32 * w];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          acc[h][w][0] = Fma2(w2[h], v.x, acc[h][w][0]);
+          acc[h][w][1] = Fma2(w2[h], v.y, acc[h][w][1]);
+        }
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  // The second half of the warps hands its positions' part to the first.
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  ulonglong2* other = ring + quad * (4 * NV * 32);
+  if (half == 1) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) other[(h * NV + i) * 32 + lane] = make_ulonglong2(acc[h][i][0], acc[h][i][1]);
+    if (lane < 4) s_p[warp][lane] = make_float4(top, sum, 0.f, 0.f);
+  }
+  __syncthreads();
+  if (half == 1) return;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    if (h0 + h >= p.H) break;
+    const float4 there = s_p[warp + 4][h];
+    const float top_a = __shfl_sync(0xffffffffu, top, h), sum_a = __shfl_sync(0xffffffffu, sum, h);
+    const float all = fmaxf(top_a, there.x);
+    // A half that saw nothing has no part in it.
+    const float fa = top_a == -INFINITY && sum_a == 0.f ? 0.f : expf(top_a - all), fb = there.x == -INFINITY && there.y == 0.f ? 0.f : expf(there.x - all);
+    const float total = sum_a * fa + there.y * fb, inv = sum_a * fa + there.y * fb > 0.f ? 1.f / total : 0.f;
+    const size_t at = static_cast<size_t>(t) * p.H + h0 + h;
+    float* rec = sp.records != nullptr ? sp.records + (static_cast<size_t>(slice) * p.T * p.H + at) * (p.kv_rank + 2) : nullptr;
+    float* out = static_cast<float*>(p.out) + at * p.kv_rank;
+    if (rec != nullptr && lane == 0) {
+      rec[0] = all;
+      rec[1] = total;
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int w = lane + 32 * i;
+      if (w >= vwords) break;
+      const ulonglong2 o = other[(h * NV + i) * 32 + lane];
+      const float r[4] = {fmaf(Low(acc[h][i][0]), fa, Low(o.x) * fb), fmaf(High(acc[h][i][0]), fa, High(o.x) * fb),
+                          fmaf(Low(acc[h][i][1]), fa, Low(o.y) * fb), fmaf(High(acc[h][i][1]), fa, High(o.y) * fb)};
+      if (rec != nullptr) {
+        *reinterpret_cast<float2*>(rec + 2 + 4 * w) = make_float2(r[0], r[1]);
+        *reinterpret_cast<float2*>(rec + 4 + 4 * w) = make_float2(r[2], r[3]);
+      } else {
+        *reinterpret_cast<float4*>(out + 4 * w) = make_float4(r[0] * inv, r[1] * inv, r[2] * inv, r[3] * inv);
+      }
+    }
+  }
+}
+
+// Merges the slices of one (row, head): a thread per two latent channels.
+__global__ void __launch_bounds__(128) LatentCombineF32(LatentParams p, F32Slices sp)
+{
+  GridDependencySync();
+  const int h = blockIdx.x, t = blockIdx.y;
+  const int2 live = LiveRange(p, t);
+  const int tiles = live.y > live.x ? (live.y + kF32Tile - 1) / kF32Tile - live.x / kF32Tile : 0;
+  const int n = (tiles + sp.slice_tiles - 1) / sp.slice_tiles;
+  const float* rec = sp.records + (static_cast<size_t>(t) * p.H + h) * (p.kv_rank + 2);
+  const size_t step = static_cast<size_t>(p.T) * p.H * (p.kv_rank + 2);
+  float top = -INFINITY, sum = 0.f;
+  for (int s = 0; s < n; ++s) top = fmaxf(top, rec[s * step]);
+  for (int s = 0; s < n; ++s) sum += expf(rec[s * step] - top) * rec[s * step + 1];
+  const float inv = sum > 0.f ? 1.f / sum : 0.f;
+  float* out = static_cast<float*>(p.out) + (static_cast<size_t>(t) * p.H + h) * p.kv_rank;
+  for (int c = threadIdx.x * 2; c < p.kv_rank; c += 256) {
+    float a = 0.f, b = 0.f;
+    for (int s = 0; s < n; ++s) {
+      const float w = expf(rec[s * step] - top);
+      const float2 v = *reinterpret_cast<const float2*>(rec + s * step + 2 + c);
+      a = fmaf(w, v.x, a);
+      b = fmaf(w, v.y, b);
+    }
+    *reinterpret_cast<float2*>(out + c) = make_float2(a * inv, b * inv);
+  }
+}
+
+bool F32Applies(const LatentParams& p)
+{
+  return p.kv_rank % 4 == 0 && p.row % 4 == 0 && p.kv_rank <= 512 && p.row <= 640 && p.pool_ld % 4 == 0 && Aligned16(p.query) && Aligned16(p.pool) &&
+         Aligned16(p.out) && p.T <= 65535;
+}
+constexpr int F32Smem(int nw) { return kF32Stages * kF32Tile * nw * 32 * 16; }
+
+// Slices of the positions: waves of CTAs (one an SM) times the tiles of the longest, and what a slice's start and its record cost (in tiles).
+F32Slices ChooseF32Slices(const LatentParams& p, int max_live, void* scratch, size_t scratch_bytes)
+{
+  const int tiles = (max_live + kF32Tile - 1) / kF32Tile + 1, slots = 148;
+  const long long ctas = static_cast<long long>(p.T) * ((p.H + kF32Heads - 1) / kF32Heads);
+  const size_t record = static_cast<size_t>(p.T) * p.H * (p.kv_rank + 2) * sizeof(float);
+  F32Slices best = {nullptr, 1, 0x3fffffff};
+  double best_cost = 1e30;
+  for (int s = 1; s <= std::min(tiles, 64) && (s == 1 || (scratch != nullptr && Aligned16(scratch) && record * s <= scratch_bytes)); ++s) {
+    const int per = (tiles + s - 1) / s;
+    const double waves = static_cast<double>((ctas * s + slots - 1) / slots);
+    const double cost = waves * (per + 3.0) + (s > 1 ? 3.0 + 0.1 * s * static_cast<double>(ctas) / slots : 0.0);
+    if (cost < best_cost * 0.98) {
+      best_cost = cost;
+      best.slices = (tiles + per - 1) / per;
+      best.slice_tiles = s > 1 ? per : 0x3fffffff;
+    }
+  }
+  if (best.slices > 1) best.records = static_cast<float*>(scratch);
+  return best;
 }
 
 // ---- the tensor-core form ---------------------------------------------------------------------------------------------
@@ -602,6 +864,8 @@ cudaError_t PrepareLatentAttention()
     TLALOC_OPT_IN(3);
     TLALOC_OPT_IN(4);
 #undef TLALOC_OPT_IN
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(LatentAttentionF32<5, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Smem(5));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(LatentAttentionF32<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Smem(3));
     return e;
   });
 }
@@ -718,6 +982,18 @@ extern "C" int tlaloc_b200_latent_attention(const void* query, const void* pool,
     sp.records = sp.slices > 1 ? static_cast<float*>(scratch) : nullptr;
     e = LaunchTcForm(map, p, sp, st);
     if (e == cudaSuccess && sp.slices > 1) e = LaunchChained(LatentCombine, dim3(num_heads, num_tokens), 128, 0, st, p, sp);
+    if (e != cudaSuccess) return CudaFail("LATENT_ATTENTION launch", e);
+    CountLaunches(sp.slices > 1 ? 2 : 1);
+    return kOk;
+  }
+  if (dtype == TLALOC_B200_F32 && !OrderFaithful() && F32Applies(p)) {
+    cudaError_t e = PrepareLatentAttention();
+    if (e != cudaSuccess) return CudaFail("LATENT_ATTENTION set-up", e);
+    const F32Slices sp = ChooseF32Slices(p, MaxLive(max_live, window, static_cast<int64_t>(max_blocks) * block_size), scratch, scratch_bytes);
+    const dim3 grid(sp.slices, (num_heads + kF32Heads - 1) / kF32Heads, num_tokens);
+    e = kv_rank <= 256 && p.row <= 384 ? LaunchChained(LatentAttentionF32<3, 2>, grid, kF32Threads, F32Smem(3), st, p, sp)
+                                       : LaunchChained(LatentAttentionF32<5, 4>, grid, kF32Threads, F32Smem(5), st, p, sp);
+    if (e == cudaSuccess && sp.slices > 1) e = LaunchChained(LatentCombineF32, dim3(num_heads, num_tokens), 128, 0, st, p, sp);
     if (e != cudaSuccess) return CudaFail("LATENT_ATTENTION launch", e);
     CountLaunches(sp.slices > 1 ? 2 : 1);
     return kOk;
