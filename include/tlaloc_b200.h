@@ -294,6 +294,10 @@ int tlaloc_b200_swiglu(const float* gate, const float* up, int32_t ld, void* out
 /* Greedy NEXT_TOKEN (DxirInterpreter.kt:2414-2426; triton/kernels/sample.cu greedy arm): first index of the maximum. */
 int tlaloc_b200_argmax(const float* logits, int32_t* out, int32_t rows, int32_t n, void* stream);
 
+/* A step's inputs from one buffer into their own: the counts[0] values at packed go to dst[0], the counts[1] after them to dst[1], and so on
+ * (1 to 16 segments).  packed and the dst[i] are device memory, the arrays dst and counts host memory, read before the call returns. */
+int tlaloc_b200_unpack_i32(const int32_t* packed, int32_t* const* dst, const int32_t* counts, int32_t segments, void* stream);
+
 /* ------------------------------------------------------------------ unquantized projections */
 
 #define TLALOC_B200_ACT_NONE 0

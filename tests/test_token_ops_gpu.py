@@ -47,3 +47,34 @@ def test_embedding_rows(dim, dtype, offset):
     table = torch.randn((9 * dim + offset,), device=DEV).to(dtype)[offset:].view(9, dim)
     ids = torch.tensor([3, -2, 8, 0, 99, 3], dtype=torch.int32, device=DEV)  # ids outside are clamped
     assert torch.equal(ops().embedding(table, ids), table[ids.long().clamp(0, 8)].float())
+
+
+@pytest.mark.parametrize("sizes", [[1], [5, 0, 300, 1], [256, 256], [1] * 16])
+def test_unpacking_of_a_steps_inputs(sizes):
+    packed = torch.randint(-9, 9, (sum(sizes) + 3,), dtype=torch.int32, device=DEV)
+    outs = [torch.full((n + 1,), 77, dtype=torch.int32, device=DEV) for n in sizes]
+    ops().unpack_i32(packed, [o[:n] for o, n in zip(outs, sizes)])
+    at = 0
+    for o, n in zip(outs, sizes):
+        assert torch.equal(o[:n], packed[at:at + n]) and int(o[n]) == 77
+        at += n
+
+
+def test_inputs_of_steps_in_flight_do_not_mix():
+    """More steps than there are pinned buffers, queued behind a busy stream: each finds its own inputs."""
+    from tlaloc_b200.step_model import StepModel
+
+    m = StepModel(50, 50, 8, 30, 16, 100, DEV)
+    seen, sent = [], []
+    a = torch.randn((4096, 4096), device=DEV)
+    for step in range(5):
+        for _ in range(3):
+            a = a @ a * 1e-4
+        rng = np.random.default_rng(step)
+        sent.append([rng.integers(0, 99, size=shape) for shape in ((50,), (50,), (50, 30), (50,), (50,))])
+        m.set_inputs(*sent[-1])
+        seen.append([t.clone() for t in (m.token_ids, m.positions, m.block_tables, m.seq_lens, m.slot_mapping)])
+    for got, want in zip(seen, sent):
+        assert all(np.array_equal(g.cpu().numpy(), w) for g, w in zip(got, want))
+    with pytest.raises(RuntimeError):
+        m.set_inputs(sent[0][0][:7], None, None, None, None)

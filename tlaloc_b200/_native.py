@@ -64,6 +64,7 @@ _SIGNATURES = {
     "tlaloc_b200_rope_kv_write": (ctypes.c_int, [_vp] * 8 + [_i32, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp]),
     "tlaloc_b200_swiglu": (ctypes.c_int, [_vp, _vp, _i32, _vp, _i32, _i32, _i32, _vp]),
     "tlaloc_b200_argmax": (ctypes.c_int, [_vp, _vp, _i32, _i32, _vp]),
+    "tlaloc_b200_unpack_i32": (ctypes.c_int, [_vp, _vp, _vp, _i32, _vp]),
     "tlaloc_b200_dense_gemm": (ctypes.c_int, [ctypes.POINTER(DenseProblem), _i32, _i32, _i32, _i32, _vp]),
     "tlaloc_b200_rmsnorm_pair": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _f32, _vp]),
     "tlaloc_b200_latent_kv_write": (ctypes.c_int, [_vp, _i64, _vp, _vp, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64] + [_i32] * 7 + [_vp]),

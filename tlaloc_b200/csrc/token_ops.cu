@@ -118,6 +118,24 @@ __global__ void __launch_bounds__(kArgmaxThreads) ArgmaxKernel(const float* x, i
   if (tid == 0) out[blockIdx.x] = idx == 0x7fffffff ? 0 : idx;
 }
 
+// The inputs of a step travel to the device as one copy and are handed out to their buffers here: each copy of its own costs about 5 us on the
+// stream, and a step has five to eight of them.
+constexpr int kMaxSegments = 16;
+struct UnpackArgs {
+  int32_t* dst[kMaxSegments];
+  int start[kMaxSegments + 1];
+  int segments;
+};
+__global__ void __launch_bounds__(256) UnpackKernel(const int32_t* packed, const __grid_constant__ UnpackArgs a)
+{
+  GridDependencySync();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= a.start[a.segments]) return;
+  int s = 0;
+  while (i >= a.start[s + 1]) ++s;
+  a.dst[s][i - a.start[s]] = __ldcg(packed + i);
+}
+
 template <typename TT>
 cudaError_t LaunchEmbedding(const void* table, const int32_t* ids, float* out, int positions, int vocab, int dim, cudaStream_t st)
 {
@@ -166,6 +184,27 @@ extern "C" int tlaloc_b200_argmax(const float* logits, int32_t* out, int32_t row
   const int per = ((n + ranks - 1) / ranks + 3) / 4 * 4;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, ArgmaxKernel, logits, out, static_cast<int>(n), per, n % 4 == 0 && Aligned16(logits) ? 1 : 0);
   if (e != cudaSuccess) return CudaFail("ARGMAX launch", e);
+  CountLaunches(1);
+  return kOk;
+}
+
+extern "C" int tlaloc_b200_unpack_i32(const int32_t* packed, int32_t* const* dst, const int32_t* counts, int32_t segments, void* stream)
+{
+  if (!packed || !dst || !counts) return Fail(kInvalid, "UNPACK: a required pointer is null");
+  if (segments < 1 || segments > kMaxSegments) return Fail(kInvalid, "UNPACK: 1 to %d segments", kMaxSegments);
+  UnpackArgs a = {};
+  a.segments = segments;
+  long long total = 0;
+  for (int i = 0; i < segments; ++i) {
+    if (counts[i] < 0 || (counts[i] > 0 && !dst[i])) return Fail(kInvalid, "UNPACK: bad segment %d", i);
+    a.dst[i] = dst[i];
+    total += counts[i];
+    if (total > (1 << 30)) return Fail(kInvalid, "UNPACK: too many values");
+    a.start[i + 1] = static_cast<int>(total);
+  }
+  if (total == 0) return kOk;
+  const cudaError_t e = LaunchChained(UnpackKernel, static_cast<unsigned>((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), packed, a);
+  if (e != cudaSuccess) return CudaFail("UNPACK launch", e);
   CountLaunches(1);
   return kOk;
 }

@@ -363,9 +363,14 @@ class Decoder(StepModel):
         return self.peer.status() if self.peer is not None else 0
 
     def run(self, step: RaggedStep, want) -> torch.Tensor:
-        self.set_inputs(*self._padded(step, self.batch))
+        ids, positions, tables, lens, slots = self._padded(step, self.batch)
+        rows = self._wanted(want, self.batch)
+        self._put_all([(self.token_ids, ids), (self.positions, positions), (self.block_tables, tables), (self.seq_lens, lens), (self.slot_mapping, slots),
+                       (self.want_rows[:len(rows)], rows) if rows is not None else (self.want_rows, None)])
         self.step()
-        return self.logits[torch.as_tensor(want, dtype=torch.long, device=self.device)]
+        if rows is None:
+            return self.logits[torch.as_tensor(want, dtype=torch.long, device=self.device)]
+        return ops.embedding(self.logits, self.want_rows[:len(rows)]) if len(rows) else self.logits[:0]
 
     # ------------------------------------------------------------------ traffic model
 

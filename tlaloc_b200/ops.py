@@ -6,6 +6,8 @@ a tensor that is not on a CUDA device is refused.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _native as N
@@ -243,6 +245,16 @@ def argmax(logits, out=None):
     _out("ARGMAX out", out, (rows,), torch.int32, logits)
     N.check(N.lib().tlaloc_b200_argmax(_ptr(logits), _ptr(out), rows, n, _stream(logits)))
     return out
+
+
+def unpack_i32(packed, outs):
+    """The values of packed [n], in order, into the int32 tensors `outs` (contiguous, up to 16)."""
+    _dev(packed, *outs)
+    if packed.dtype != torch.int32 or any(t.dtype != torch.int32 for t in outs) or packed.numel() < sum(t.numel() for t in outs):
+        raise ValueError("UNPACK: int32 tensors, and as many values as they hold")
+    dst = (ctypes.c_void_p * len(outs))(*[t.data_ptr() for t in outs])
+    counts = (ctypes.c_int32 * len(outs))(*[t.numel() for t in outs])
+    N.check(N.lib().tlaloc_b200_unpack_i32(_ptr(packed), dst, counts, len(outs), _stream(packed)))
 
 
 # ---------------------------------------------------------------------- unquantized projections, latent attention

@@ -35,6 +35,12 @@ class StepModel:
         self.block_tables = torch.zeros((tables, max_blocks_per_seq), **i32)
         self.seq_lens = torch.ones((rows,), **i32)
         self.slot_mapping = torch.full((rows,), PADDING_SLOT, **i32)
+        self.want_rows = torch.zeros((tables,), **i32)  # rows whose logits are asked for
+        # a step's inputs on their way: two pinned copies in turn (one is filled while the other travels) and where they arrive
+        self._pinned: list[torch.Tensor] = []
+        self._sent: list[torch.cuda.Event] = []
+        self._packed: torch.Tensor | None = None
+        self._turn = 0
         self._graphs: dict[int, torch.cuda.CUDAGraph] = {}
 
     def _run_step(self, rows: int) -> None:
@@ -42,9 +48,8 @@ class StepModel:
 
     def set_inputs(self, token_ids, positions, block_tables, seq_lens, slot_mapping) -> None:
         """Host (NumPy or pinned torch) step inputs -> the device buffers the graph reads."""
-        for dst, src in ((self.token_ids, token_ids), (self.positions, positions), (self.block_tables, block_tables),
-                         (self.seq_lens, seq_lens), (self.slot_mapping, slot_mapping)):
-            self._put(dst, src)
+        self._put_all([(self.token_ids, token_ids), (self.positions, positions), (self.block_tables, block_tables),
+                       (self.seq_lens, seq_lens), (self.slot_mapping, slot_mapping)])
 
     @staticmethod
     def _put(dst: torch.Tensor, src) -> None:
@@ -53,6 +58,44 @@ class StepModel:
         if isinstance(src, np.ndarray):
             src = torch.from_numpy(np.ascontiguousarray(src, dtype=np.int32))
         dst.copy_(src.reshape(dst.shape), non_blocking=True)
+
+    def _put_all(self, pairs) -> None:
+        """Host sources into device buffers [(buffer, source or None)], all with one copy: the buffers are contiguous."""
+        pairs = [(dst, src) for dst, src in pairs if src is not None]
+        if self.device.type != "cuda" or torch.cuda.is_current_stream_capturing() or any(isinstance(src, torch.Tensor) and src.is_cuda for _, src in pairs):
+            for dst, src in pairs:
+                self._put(dst, src)
+            return
+        host = [src.numpy() if isinstance(src, torch.Tensor) else np.asarray(src) for _, src in pairs]
+        for (dst, _), src in zip(pairs, host):
+            if src.size != dst.numel():
+                raise RuntimeError(f"an input of shape {src.shape} does not fit {tuple(dst.shape)}")
+        total = sum(src.size for src in host)
+        if total == 0:
+            return
+        if self._packed is None:
+            most = 6 * self.rows + self.block_tables.numel() + self.max_sequences
+            self._pinned = [torch.empty((most,), dtype=torch.int32, pin_memory=True) for _ in range(2)]
+            self._sent = [torch.cuda.Event() for _ in range(2)]
+            self._packed = torch.empty((most,), dtype=torch.int32, device=self.device)
+        turn = self._turn
+        self._turn ^= 1
+        self._sent[turn].synchronize()  # the copy before last has left
+        pinned, at = self._pinned[turn].numpy(), 0
+        for src in host:
+            pinned[at:at + src.size] = src.reshape(-1)
+            at += src.size
+        with torch.cuda.device(self.device):
+            self._packed[:total].copy_(self._pinned[turn][:total], non_blocking=True)
+            self._sent[turn].record()
+            ops.unpack_i32(self._packed[:total], [dst for dst, _ in pairs])
+
+    def _wanted(self, want, rows: int):
+        """Indices as a list takes them (negative ones from the end), as int32; None where they do not fit `want_rows`."""
+        want = np.asarray(want, np.int64).reshape(-1)
+        if want.size and (want.min() < -rows or want.max() >= rows):
+            raise IndexError(f"rows {want.tolist()} of {rows}")
+        return np.where(want < 0, want + rows, want).astype(np.int32) if want.size <= self.max_sequences else None
 
     def capture(self, rows: int | None = None) -> None:
         """Capture the step over `rows` rows into a CUDA graph (after one eager warm-up step on a side stream)."""
@@ -152,21 +195,23 @@ class RaggedModel(StepModel):
             raise ValueError(f"a step of {n} tokens of {s} sequences; this model takes {self.max_tokens} of {self.max_sequences}")
         if n == s and trace is None:
             return self._run_decode(step, want)
-        self._inputs(step)
+        rows = np.asarray(want, np.int32).reshape(-1)
+        fits = rows.size <= self.max_sequences
+        self._inputs(step, rows if fits else None)
         self._hidden(n, [(int(a), int(b), r, int(step.positions[a])) for r, (a, b) in enumerate(zip(step.starts[:-1], step.starts[1:]))], trace)
+        if fits:
+            return self._head(ops.embedding(self.x[:n], self.want_rows[:rows.size])) if rows.size else self.logits[:0]
         out = []
         for k in range(0, len(want), self.max_sequences):
             rows = torch.as_tensor(np.asarray(want[k:k + self.max_sequences], np.int32), device=self.device)
-            out.append(self._head(ops.embedding(self.x[:n], rows)))
-            if len(want) > self.max_sequences:
-                out[-1] = out[-1].clone()
-        return torch.cat(out) if len(out) > 1 else out[0] if out else self.logits[:0]
+            out.append(self._head(ops.embedding(self.x[:n], rows)).clone())
+        return torch.cat(out)
 
-    def _inputs(self, step: RaggedStep) -> None:
-        for dst, src in ((self.token_ids, step.token_ids), (self.positions, step.positions), (self.seq_lens, step.seq_lens),
-                         (self.slot_mapping, step.slot_mapping), (self.row_tables, step.row_tables), (self.row_states, step.row_states),
-                         (self.block_tables, step.block_tables)):
-            self._put(dst[:src.shape[0]], src)
+    def _inputs(self, step: RaggedStep, want=None) -> None:
+        pairs = ((self.token_ids, step.token_ids), (self.positions, step.positions), (self.seq_lens, step.seq_lens),
+                 (self.slot_mapping, step.slot_mapping), (self.row_tables, step.row_tables), (self.row_states, step.row_states),
+                 (self.block_tables, step.block_tables), (self.want_rows, want))
+        self._put_all([(dst[:src.shape[0]], src) for dst, src in pairs if src is not None])
 
     def _run_decode(self, step: RaggedStep, want) -> torch.Tensor:
         """One token of every sequence: the batch is padded to a power of two, and a size that comes up again is captured into a
@@ -190,7 +235,6 @@ class RaggedModel(StepModel):
     def set_decode_inputs(self, token_ids, positions, block_tables, seq_lens, slot_mapping, row_states=None) -> None:
         """Inputs of a step of one token per sequence, as many as there are ids; row r uses block table r."""
         rows = token_ids.shape[0]
-        for dst, src in ((self.token_ids, token_ids), (self.positions, positions), (self.block_tables, block_tables),
-                         (self.seq_lens, seq_lens), (self.slot_mapping, slot_mapping), (self.row_tables, np.arange(rows, dtype=np.int32)),
-                         (self.row_states, row_states)):
-            self._put(dst[:rows], src)
+        self._put_all([(dst[:rows], src) for dst, src in (
+            (self.token_ids, token_ids), (self.positions, positions), (self.block_tables, block_tables), (self.seq_lens, seq_lens),
+            (self.slot_mapping, slot_mapping), (self.row_tables, np.arange(rows, dtype=np.int32)), (self.row_states, row_states))])
