@@ -298,12 +298,33 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
 
 // ------------------------------------------------------------------------------------------
 
-template <typename XT>
-__global__ void ToBf16Kernel(const XT* x, __nv_bfloat16* out, size_t n)
+// Eight values a thread (n is a multiple of eight here: k is), by 16-byte words where x allows.
+__global__ void __launch_bounds__(256) ToBf16Kernel(const float* x, __nv_bfloat16* out, size_t n, int vec)
 {
   GridDependencySync();
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = __float2bfloat16_rn(ToF32(x[i]));
+  const size_t i = (static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x) * 8;
+  if (i >= n) return;
+  float v[8];
+  if (vec) {
+    *reinterpret_cast<float4*>(v) = __ldcg(reinterpret_cast<const float4*>(x + i));
+    *reinterpret_cast<float4*>(v + 4) = __ldcg(reinterpret_cast<const float4*>(x + i) + 1);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = x[i + e];
+  }
+  uint4 o;
+  uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    w[e] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  *reinterpret_cast<uint4*>(out + i) = o;
+}
+cudaError_t LaunchToBf16(const void* x, void* out, size_t count, cudaStream_t st)
+{
+  return LaunchChained(ToBf16Kernel, static_cast<unsigned>((count / 8 + 255) / 256), 256, 0, st, static_cast<const float*>(x), static_cast<__nv_bfloat16*>(out),
+                       count, Aligned16(x) ? 1 : 0);
 }
 
 // y[i, j] = (sum over p ascending of x[i, p] * w[p, j], f32, separate multiply and add, x == 0 skipped) * scale[j]
@@ -526,8 +547,7 @@ extern "C" int tlaloc_b200_int8_gemm(const void* x, int32_t x_dtype, const int8_
     }
     if (!Aligned16(scratch)) return Fail(kInvalid, "%s: scratch must be 16-byte aligned", op);
     const size_t count = static_cast<size_t>(m) * k;
-    e = LaunchChained(ToBf16Kernel<float>, static_cast<unsigned>((count + 255) / 256), 256, 0, st,
-                      static_cast<const float*>(x), reinterpret_cast<__nv_bfloat16*>(scratch), count);
+    e = LaunchToBf16(x, scratch, count, st);
     if (e != cudaSuccess) return CudaFail("INT8_PROJ activation cast", e);
     CountLaunches(1);
     xb = reinterpret_cast<const __nv_bfloat16*>(scratch);
@@ -639,8 +659,7 @@ extern "C" int tlaloc_b200_int8_gemm_swiglu(const void* x, int32_t x_dtype, cons
       return Fail(kInvalid, "%s: an f32 x needs %zu bytes of 16-byte aligned scratch for its bf16 copy, got %zu", op, need, scratch_bytes);
     }
     const size_t count = static_cast<size_t>(m) * k;
-    e = LaunchChained(ToBf16Kernel<float>, static_cast<unsigned>((count + 255) / 256), 256, 0, st, static_cast<const float*>(x),
-                      reinterpret_cast<__nv_bfloat16*>(scratch), count);
+    e = LaunchToBf16(x, scratch, count, st);
     if (e != cudaSuccess) return CudaFail("INT8_PROJ_SWIGLU activation cast", e);
     CountLaunches(1);
     xb = reinterpret_cast<const __nv_bfloat16*>(scratch);
