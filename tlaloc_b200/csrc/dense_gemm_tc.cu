@@ -37,11 +37,11 @@ template <int BT>
 struct Layout {
   static constexpr int kXBytes = BT * kBK * 2;
   static constexpr int kStage = kWBytes + kXBytes;
-  static constexpr int kStages = BT == 256 ? 4 : BT == 128 ? 6 : 8;
+  static constexpr int kStages = BT >= 224 ? 4 : BT >= 160 ? 5 : BT == 128 ? 6 : 8;
   static constexpr int kPipe = kStages * kStage;
   static constexpr int kTileStride = kBN + 4;  // the slice's partial tile [BT][kTileStride] f32, aliases the ring
-  static_assert(kPipe >= BT * kTileStride * 4 || BT == 256, "the partial tile aliases the ring");
-  static constexpr int kRows = BT / 2 < 32 ? BT / 2 : 32;          // activation rows an epilogue group takes at a time
+  static_assert(kPipe >= BT * kTileStride * 4 || BT > 128, "the partial tile aliases the ring");
+  static constexpr int kRows = BT % 64 == 0 ? 32 : 16;             // activation rows an epilogue group takes at a time
   static constexpr int kOut = kPipe;                               // two groups' bf16 output rows [kRows][128]
   static constexpr int kBars = kOut + 2 * kRows * kBN * 2;
   static constexpr int kSlot = kBars + 8 * (2 * kStages + 4);
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 {
   using L = Layout<BT>;
   constexpr int S = L::kStages;
-  constexpr uint32_t kCols = SPLIT ? (BT < 32 ? 32 : BT) : 2 * BT;
+  constexpr uint32_t kCols = SPLIT ? BT : BT > 128 ? 512 : 2 * BT;  // a power of two
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (SmemAddr(smem_raw) + 1023u) & ~1023u;  // the swizzle is a function of address bits 4..9
   unsigned char* smem = smem_raw + (base - SmemAddr(smem_raw));
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     if (!GROUPED) GridDependencySync();
     const int quad = warp & 3, half = warp >> 2;
-    constexpr int kHalf = BT / 2, CH = kHalf < 32 ? kHalf : 32;
+    constexpr int kHalf = BT / 2, CH = L::kRows;
     int lt = 0;
     for (int id = blockIdx.x; id < tiles; id += gridDim.x, ++lt) {
       const Tile t = TileAt<GROUPED>(a, id, BT, s_start);
@@ -502,6 +502,9 @@ cudaError_t PrepareDenseTc()
     TLALOC_OPT_IN(32, false);
     TLALOC_OPT_IN(64, false);
     TLALOC_OPT_IN(128, false);
+    TLALOC_OPT_IN(160, false);
+    TLALOC_OPT_IN(192, false);
+    TLALOC_OPT_IN(224, false);
     TLALOC_OPT_IN(256, false);
     TLALOC_OPT_IN(32, true);
     TLALOC_OPT_IN(64, true);
@@ -570,6 +573,30 @@ int ChooseSlices(int tiles, int nb)
   return best;
 }
 
+// Rows of a tile of more than 128 rows, in units of one 64-k block of 256 rows: waves * (blocks of a tile * (0.15 + 0.85 rows / 256) + what a tile's
+// start and end cost).  A block of 128 rows takes 0.57 of one of 256 (measured), the heights between are there to fill the last wave: 2048 rows,
+// n 2560, k 2560 and 6400: 160 tiles of 256 rows are 1.08 waves, 320 of 128 rows 2.16, 260 of 160 rows 1.76: 57 us with 128 rows, 46 with 160.
+int ChooseHeight(const tlaloc_b200_dense_problem* problems, int count, int rows)
+{
+  long long columns = 0;
+  int nb = 0;
+  for (int i = 0; i < count; ++i) {
+    columns += static_cast<long long>((problems[i].n + kBN - 1) / kBN) * problems[i].batch;
+    nb = max(nb, (problems[i].k + kBK - 1) / kBK);
+  }
+  int best = 256;
+  double best_cost = 1e30;
+  for (int height : {256, 224, 192, 160, 128}) {
+    const long long waves = (columns * ((rows + height - 1) / height) + 147) / 148;
+    const double cost = static_cast<double>(waves) * (nb * (0.15 + 0.85 * height / 256) + 4.6);
+    if (cost < best_cost * 0.97) {
+      best_cost = cost;
+      best = height;
+    }
+  }
+  return best;
+}
+
 template <int BT, bool SPLIT, bool GROUPED = false>
 cudaError_t Launch(const CUtensorMap* maps, const TcArgs& a, int ctas, cudaStream_t st)
 {
@@ -606,12 +633,7 @@ cudaError_t LaunchDenseGemmTc(const tlaloc_b200_dense_problem* problems, int cou
     grouped = grouped || s.row_offsets != nullptr;
   }
   int bt = typical <= 32 ? 32 : typical <= 64 ? 64 : typical <= 128 ? 128 : 256;
-  if (bt == 256 && !grouped) {  // half the rows a tile where that fills the last wave of CTAs better by more than its own loss (about a seventh)
-    int columns = 0;
-    for (int i = 0; i < count; ++i) columns += (problems[i].n + kBN - 1) / kBN * problems[i].batch;
-    auto waves = [&](int rows) { return (columns * ((typical + rows - 1) / rows) + 147) / 148; };
-    if (waves(128) * 128 * 1.15 < waves(256) * 256) bt = 128;
-  }
+  if (bt == 256 && !grouped) bt = ChooseHeight(problems, count, typical);
   CUtensorMap maps[4];
   TcArgs a = {};
   a.weights_const = weights_const ? 1 : 0;
@@ -659,7 +681,7 @@ cudaError_t LaunchDenseGemmTc(const tlaloc_b200_dense_problem* problems, int cou
       default: return Launch<256, false, true>(maps, a, 148, st);
     }
   }
-  a.ks = bt <= 128 && a.p[0].tiles_m == 1 && (count == 1 || a.p[1].tiles_m == 1) ? ChooseSlices(a.tiles, nb) : 1;
+  a.ks = typical <= 128 ? ChooseSlices(a.tiles, nb) : 1;
   if (a.ks > 1) {
     switch (bt) {
       case 32: return Launch<32, true>(maps, a, a.tiles, st);
@@ -672,6 +694,9 @@ cudaError_t LaunchDenseGemmTc(const tlaloc_b200_dense_problem* problems, int cou
     case 32: return Launch<32, false>(maps, a, ctas, st);
     case 64: return Launch<64, false>(maps, a, ctas, st);
     case 128: return Launch<128, false>(maps, a, ctas, st);
+    case 160: return Launch<160, false>(maps, a, ctas, st);
+    case 192: return Launch<192, false>(maps, a, ctas, st);
+    case 224: return Launch<224, false>(maps, a, ctas, st);
     default: return Launch<256, false>(maps, a, ctas, st);
   }
 }
