@@ -88,6 +88,13 @@ __device__ __forceinline__ void GridDependencySync()
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Ahead of GridDependencySync(): the n values at p (a norm's gain, read only once a row's sum is known) on their way from HBM into L2 while the
+// previous kernel drains.  A hint without a result, at the point of coherence: a kernel in flight may even be writing them.
+__device__ __forceinline__ void PrefetchL2(const float* p, int n)
+{
+  if (p == nullptr || blockIdx.x >= 4) return;
+  for (int i = threadIdx.x * 32; i < n; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+}
 bool PdlEnabled();
 // The launch attributes every kernel gets; `attrs` must have room for 2.  Returns the count.
 inline int ChainAttributes(cudaLaunchAttribute* attrs, int cluster_y = 0)

@@ -21,6 +21,7 @@ __device__ __forceinline__ float BlockSum(float v, float* red)
 
 // One CTA per row: x * rsqrt(mean(x^2) + eps) * gain.  mean = sum / n, rsqrt in double then narrowed, and the two
 // multiplies kept separate, as the interpreter evaluates the graph's nodes (DxirInterpreter.kt:567-572,1791-1807).
+// A few rows are bound by the chain of launch, row, sum, gain, store; the gain is in L2 by the time it is asked for (PrefetchL2).
 // Rows of up to 8192 values (a multiple of 4) are read once with 16-byte loads, all in flight together, and kept
 // in registers for the second pass; other rows take the two-pass loop.
 __device__ __forceinline__ float BlockMax(float v, float* red)
@@ -43,6 +44,7 @@ template <typename OT, bool PLANES>
 __global__ void __launch_bounds__(256) RmsNormKernel(const float* x, const float* gain, OT* out, int n, float eps, int8_t* hi,
                                                      int8_t* lo, float* steps)
 {
+  PrefetchL2(gain, n);
   GridDependencySync();
   __shared__ float red[8];
   const float* xr = x + static_cast<size_t>(blockIdx.x) * n;
@@ -70,10 +72,22 @@ __global__ void __launch_bounds__(256) RmsNormKernel(const float* x, const float
         const float a = __fmul_rn(v[i].x, rsq), b = __fmul_rn(v[i].y, rsq), c = __fmul_rn(v[i].z, rsq), d = __fmul_rn(v[i].w, rsq);
         const float r0 = gain != nullptr ? __fmul_rn(a, g.x) : a, r1 = gain != nullptr ? __fmul_rn(b, g.y) : b;
         const float r2 = gain != nullptr ? __fmul_rn(c, g.z) : c, r3 = gain != nullptr ? __fmul_rn(d, g.w) : d;
-        o[4 * j] = FromF32<OT>(r0);
-        o[4 * j + 1] = FromF32<OT>(r1);
-        o[4 * j + 2] = FromF32<OT>(r2);
-        o[4 * j + 3] = FromF32<OT>(r3);
+        if constexpr (sizeof(OT) == 2) {
+          if ((reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+            const __nv_bfloat162 lo2 = __floats2bfloat162_rn(r0, r1), hi2 = __floats2bfloat162_rn(r2, r3);
+            *reinterpret_cast<uint2*>(o + 4 * j) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo2), *reinterpret_cast<const uint32_t*>(&hi2));
+          } else {
+            o[4 * j] = FromF32<OT>(r0);
+            o[4 * j + 1] = FromF32<OT>(r1);
+            o[4 * j + 2] = FromF32<OT>(r2);
+            o[4 * j + 3] = FromF32<OT>(r3);
+          }
+        } else {
+          o[4 * j] = FromF32<OT>(r0);
+          o[4 * j + 1] = FromF32<OT>(r1);
+          o[4 * j + 2] = FromF32<OT>(r2);
+          o[4 * j + 3] = FromF32<OT>(r3);
+        }
         if constexpr (PLANES) {
           v[i] = make_float4(Bf16Value(r0), Bf16Value(r1), Bf16Value(r2), Bf16Value(r3));
           const float m4 = fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));

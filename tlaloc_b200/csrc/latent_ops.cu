@@ -39,6 +39,8 @@ template <typename OT, bool VEC>
 __global__ void __launch_bounds__(256) RmsNormPairKernel(const float* x, const float* gain_a, OT* out_a, const float* gain_b,
                                                          OT* out_b, int n, float eps)
 {
+  PrefetchL2(gain_a, n);
+  PrefetchL2(gain_b, n);
   GridDependencySync();
   __shared__ float red[8];
   const size_t row = static_cast<size_t>(blockIdx.x) * n;
@@ -92,6 +94,8 @@ __global__ void __launch_bounds__(256) LatentKvWriteKernel(const float* in, int6
                                                            T* cq, T* pool, int64_t pool_ld, int q_rank, int kv_rank, int rot_dim,
                                                            int rot_dims, int num_slots, int max_pos)
 {
+  PrefetchL2(q_gain, q_rank);
+  PrefetchL2(kv_gain, kv_rank);
   GridDependencySync();
   __shared__ float red[8], red2[8];
   const int t = blockIdx.x, tid = threadIdx.x;
