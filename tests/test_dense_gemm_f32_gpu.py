@@ -28,11 +28,22 @@ def rand(*shape, seed=0):
     return torch.randn(shape, device=DEV, generator=g)
 
 
+def in_order(x, w):
+    """The product by the plain kernel: f32 FMAs in k order."""
+    y = torch.empty((x.shape[0], w.shape[0]), device=DEV)
+    before = ops().set_order_faithful(True)
+    try:
+        ops().dense_gemm(ops().dense(x, w, y))
+    finally:
+        ops().set_order_faithful(before)
+    return y
+
+
 def bound(x, w):
     """Every addition loses at most 2^-23 of what it holds: k / 32 rounded ones of chunks, and 16 inside a chunk, whose size is at most the
     sum of magnitudes."""
     k = x.shape[-1]
-    return (k / 32 + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().transpose(-1, -2)) + 1e-30
+    return (k / 32 + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().transpose(-1, -2)) + 2.0 ** -148
 
 
 # rows: one tile of 16 .. 208, then equal parts; n, k: remainders of 128 columns and of chunks of 32 and 64, two chunks and fewer
@@ -55,14 +66,39 @@ def test_tiles_and_chunks(m, n, k):
 def test_no_further_from_f64_than_plain_sums(m, k):
     x, w = rand(m, k), rand(256, k, seed=1)
     want = x.double() @ w.double().T
-    y, plain = torch.empty((m, 256), device=DEV), torch.empty((m, 256), device=DEV)
+    y = torch.empty((m, 256), device=DEV)
     ops().dense_gemm(ops().dense(x, w, y))
-    before = ops().set_order_faithful(True)
-    try:
-        ops().dense_gemm(ops().dense(x, w, plain))
-    finally:
-        ops().set_order_faithful(before)
-    assert float((y - want).norm()) <= float((plain - want).norm())
+    assert float((y - want).norm()) <= float((in_order(x, w) - want).norm())
+
+
+# k 2048: slices of k; n 19000: none
+@pytest.mark.parametrize("m,n,k", [(9, 200, 2048), (200, 200, 2048), (9, 19000, 96), (200, 19000, 96)])
+@pytest.mark.parametrize("large", [1.0, 1e10, 1e20, 1e30, 1e38])
+def test_small_operands(m, n, k, large):
+    """Rows from 1e-41 (subnormal) to 1e-33, alone and beside a row of one, against weights of `large`: each row as near to f64 as plain FMAs are, and not
+    zero where those are not."""
+    x, w = rand(m, k), rand(n, k, seed=1).clamp(-3, 3) * large
+    x *= torch.tensor([10.0 ** (r - 41) if r < 9 else 1e-37 for r in range(m)], device=DEV, dtype=torch.float64)[:, None].float()
+    x[4, ::2], x[-1] = 0.0, 0.0
+    y = torch.empty((m, n), device=DEV)
+    ops().dense_gemm(ops().dense(x, w, y))
+    want, plain = x.double() @ w.double().T, in_order(x, w)
+    assert bool(((y - want).norm(dim=1) <= (plain - want).norm(dim=1) + 2.0 ** -149 * n ** 0.5).all())
+    assert bool((y[-1] == 0).all()) and torch.equal(y == 0, want.float() == 0)
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 140, 96), (150, 140, 96), (40, 200, 1024)])
+@pytest.mark.parametrize("size", [1e12, 1e15, 1e19, 1e31, 1e38])
+def test_large_sums(m, n, k, size):
+    """Above what the parts' sums hold the outputs are the plain kernel's, infinities and NaN among them."""
+    x, w = rand(m, k).clamp(-3, 3) * size, rand(n, k, seed=1).clamp(-3, 3) * min(size, 1e19)  # finite: 3e38 is below f32's largest number
+    x[1] *= 1e-30 / size
+    y = torch.empty((m, n), device=DEV)
+    ops().dense_gemm(ops().dense(x, w, y))
+    plain, want = in_order(x, w), x[1:2].double() @ w.double().T
+    large = plain.isnan() | (plain.abs() > 2.0 ** 81)
+    assert torch.equal(y[large].nan_to_num(7.0), plain[large].nan_to_num(7.0)) and torch.equal(y.isnan(), plain.isnan())
+    assert bool(((y[1:2].double() - want).abs() <= bound(x[1:2], w)).all())
 
 
 @pytest.mark.parametrize("m", [5, 150])

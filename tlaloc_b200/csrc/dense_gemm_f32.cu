@@ -5,8 +5,10 @@
 // accumulator in TMEM holds one chunk of 32 k only, its small products first and its large ones last; the chunks are summed in registers with
 // rounding to nearest.  So a sum of k products has k / 32 rounded additions where the plain kernel (dense_gemm.cu) has k, and its error
 // against 64 bits (2-norm, relative) is the smaller one at every k: k = 128: 0.7e-7 and the plain kernel's 2.0e-7; 2048: 1.2e-7, 8.1e-7; 10304: 1.6e-7, 1.8e-6.
-// An infinity, a NaN or a number above bf16's largest makes a part infinite and the sum NaN or infinite, and a sum below 1e-28 may have met
-// parts in bf16's subnormal range: such an output is computed again with plain FMAs.
+// bf16 ends where f32 does (2^-149 is f32's last place there, 2^-126 bf16's smallest normal number), so the parts of small operands would lose
+// their low bits: operands are split after a multiplication by 2^24, which leaves every nonzero part normal, and a finished sum is
+// multiplied by 2^-48.  What gets too large by that (an operand of 2^104, a sum of 2^80 and more), an infinity or a NaN makes a part infinite
+// and the sum NaN or infinite: such an output is computed again with plain FMAs.
 //
 // D[n, m] = sum_k W[n, k] X[m, k]: 128 weight rows are the MMA's M, a tile of up to 208 activation rows its N.
 //   producer lane boxes of 32 k of both operands by TMA (f32, 128-byte swizzle), two to eight stages ahead
@@ -14,8 +16,8 @@
 //   MMA lane      the six products of a chunk, into one of two accumulators
 //   eight warps   add the finished accumulator to sums in registers (104 a thread at 208 rows, hence the register split), and write the tile
 //   persistent    a CTA walks tiles;   K slices   the slices of a tile are a cluster and sum their partial tiles in rank order
-// Bound at 208 rows by the split and the six products, which run side by side (each alone takes about 100 us of the 115 us of 203 rows, n 18944, k 2048),
-// at few rows by the way of a chunk through the three kinds of warps (0.85 us each).  203 rows, n 2048, k 10304: 86 us, 1414 us with plain FMAs; one
+// Bound at 208 rows by the split and the six products, which run side by side (each alone takes about 100 us of the 118 us of 203 rows, n 18944, k 2048),
+// at few rows by the way of a chunk through the three kinds of warps (0.85 us each).  203 rows, n 2048, k 10304: 87 us, 1414 us with plain FMAs; one
 // row, n 32768, k 2048: 113 us, 443 us.  Every mbarrier wait is bounded.
 #include <cuda.h>
 
@@ -91,17 +93,28 @@ __device__ __forceinline__ Tile TileAt(const F32Args& a, int id, const int* star
   return t;
 }
 
-// Two f32 as the exact sum of three pairs of bf16, each rounded to nearest from what the parts before it leave.
-__device__ __forceinline__ void Split2(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l)
+// Two f32 times 2^24 as the exact sum of three pairs of bf16, each rounded to nearest from what the parts before it leave: after it the lowest
+// bit of any f32 is 2^-125 or above, so no part is subnormal.
+constexpr float kDown = 0x1p-48f;  // what a sum is multiplied by
+__device__ __forceinline__ void Split2(uint64_t xy, uint32_t& h, uint32_t& m, uint32_t& l)
 {
-  auto pack = [](float u, float v) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(u, v);
-    return *reinterpret_cast<const uint32_t*>(&b);
+  // v's pair of bf16, and what it leaves of v
+  auto part = [](uint64_t v, uint32_t& out) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+    out = *reinterpret_cast<const uint32_t*>(&b);
+    uint64_t there;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(there) : "r"(out << 16), "r"(out & 0xffff0000u));
+    return there;
   };
-  h = pack(x, y);
-  const float r = x - __uint_as_float(h << 16), s = y - __uint_as_float(h & 0xffff0000u);
-  m = pack(r, s);
-  l = pack(r - __uint_as_float(m << 16), s - __uint_as_float(m & 0xffff0000u));
+  constexpr uint64_t kUp2 = 0x4b8000004b800000ull, kMinus2 = 0xbf800000bf800000ull;  // 2^24 and -1, twice
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(xy) : "l"(kUp2));
+  uint64_t at = part(xy, h);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(xy) : "l"(at), "l"(kMinus2));
+  at = part(xy, m);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(xy) : "l"(at), "l"(kMinus2));
+  part(xy, l);
 }
 
 // One output with plain FMAs; a NaN stays one.
@@ -117,7 +130,7 @@ __device__ __noinline__ float PlainDot(const float* x, const float* w, int k)
   }
   return v;
 }
-__device__ __forceinline__ bool Doubtful(float v) { return !(fabsf(v) <= 3.4e38f) || (v != 0.f && fabsf(v) < 1e-28f); }
+__device__ __forceinline__ bool Doubtful(float v) { return !(fabsf(v) < INFINITY); }
 
 __device__ __forceinline__ const float* XRow(const tlaloc_b200_dense_problem& p, const Tile& t, int m)
 {
@@ -133,7 +146,7 @@ __device__ __forceinline__ void Put(const tlaloc_b200_dense_problem& p, size_t a
   else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
 }
 
-// CH finished sums of column n (a warp's lanes hold 32 consecutive columns), rows m, m + step, ... below end: epilogue and store.
+// CH sums (times 2^48) of column n (a warp's lanes hold 32 consecutive columns), rows m, m + step, ... below end: epilogue and store.
 template <int CH>
 __device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const Tile& t, int n, int m, int step, int end, float* v)
 {
@@ -141,7 +154,7 @@ __device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int r = m + c * step;
-    if (n < p.n && r < end && Doubtful(v[c])) v[c] = PlainDot(XRow(p, t, r), WRow(p, t, n), p.k);
+    v[c] = n < p.n && r < end && Doubtful(v[c]) ? PlainDot(XRow(p, t, r), WRow(p, t, n), p.k) : v[c] * kDown;
   }
   if (IsGated(p.act)) {  // gate and other factor are sixteen lanes apart
 #pragma unroll
@@ -380,14 +393,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < (kBN + BT) / 8; i += kSplitWarps) {
           const int g = i + sw;
           if (g >= groups) break;
-          float4 f, h;
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "r"(from + g * 1024));
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(h.x), "=f"(h.y), "=f"(h.z), "=f"(h.w) : "r"((from + g * 1024) ^ 16));
+          uint64_t v[4];
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[0]), "=l"(v[1]) : "r"(from + g * 1024));
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[2]), "=l"(v[3]) : "r"((from + g * 1024) ^ 16));
           uint32_t part[3][4];
-          Split2(f.x, f.y, part[0][0], part[1][0], part[2][0]);
-          Split2(f.z, f.w, part[0][1], part[1][1], part[2][1]);
-          Split2(h.x, h.y, part[0][2], part[1][2], part[2][2]);
-          Split2(h.z, h.w, part[0][3], part[1][3], part[2][3]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) Split2(v[e], part[0][e], part[1][e], part[2][e]);
 #pragma unroll
           for (int q = 0; q < 3; ++q) {
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(to + g * 1024 + q * L::kPlane), "r"(part[q][0]), "r"(part[q][1]),
