@@ -116,6 +116,30 @@ def test_what_the_parts_cannot_hold(m):
     assert bool(((y.double() - want).abs() <= bound(x, w).nan_to_num(0, 0, 0))[fine].all())
 
 
+# 235 tiles of 148 CTAs; and a gated one, whose pairs are computed again together
+@pytest.mark.parametrize("m,n,k,act", [(208, 30000, 4096, 0), (40, 30016, 1028, 2)])
+def test_tiles_of_infinities_before_finite_ones(m, n, k, act):
+    """A CTA's first tile is infinite throughout: its outputs are the plain kernel's, and no wait of the next tile runs out meanwhile."""
+    x, w = rand(m, k), rand(n, k, seed=1)
+    w[:148 * 128, k - 1] = float("inf")
+    y = torch.empty((m, n // 2 if act else n), device=DEV)
+    ops().dense_gemm(ops().dense(x, w, y, act=act))
+    if act:
+        u = (x @ w.T).view(m, -1, 2, 16)
+        want = (u[:, :, 0].double() / (1 + torch.exp(-u[:, :, 0].double())) * u[:, :, 1]).reshape(m, -1)
+        fine = 148 * 64
+        assert torch.equal(y[:, :fine].isnan(), want[:, :fine].isnan()) and torch.equal(y[:, :fine].isinf(), want[:, :fine].isinf())
+        z = x.double() @ w[2 * fine:].double().T
+        z = z.view(m, -1, 2, 16)
+        want = (z[:, :, 0] * torch.sigmoid(z[:, :, 0]) * z[:, :, 1]).reshape(m, -1)
+        assert float((y[:, fine:].double() - want).norm() / want.norm()) < 1e-6
+    else:
+        plain = x[:, k - 1:].sign() * float("inf")
+        assert torch.equal(y[:, :148 * 128], plain.expand(m, 148 * 128))
+        want = x.double() @ w[148 * 128:].double().T
+        assert bool(((y[:, 148 * 128:].double() - want).abs() <= bound(x, w[148 * 128:])).all())
+
+
 @pytest.mark.parametrize("sizes", [[0, 3, 40, 0, 70, 1], [5] * 64, [300, 0]])
 @pytest.mark.parametrize("act", [0, 2])
 def test_groups(sizes, act):

@@ -16,9 +16,10 @@
 //   MMA lane      the six products of a chunk, into one of two accumulators
 //   eight warps   add the finished accumulator to sums in registers (104 a thread at 208 rows, hence the register split), and write the tile
 //   persistent    a CTA walks tiles;   K slices   the slices of a tile are a cluster and sum their partial tiles in rank order
-// Bound at 208 rows by the split and the six products, which run side by side (each alone takes about 100 us of the 118 us of 203 rows, n 18944, k 2048),
-// at few rows by the way of a chunk through the three kinds of warps (0.85 us each).  203 rows, n 2048, k 10304: 87 us, 1414 us with plain FMAs; one
-// row, n 32768, k 2048: 113 us, 443 us.  Every mbarrier wait is bounded.
+// Bound at 208 rows by the split and the six products, which run side by side (each alone takes about 100 us of the 109 us of 203 rows, n 18944, k 2048),
+// at few rows by the way of a chunk through the three kinds of warps (0.85 us each).  203 rows, n 2048, k 10304: 85 us, 1414 us with plain FMAs; one
+// row, n 32768, k 2048: 113 us, 443 us.  Every mbarrier wait is bounded.  Sums computed again: 203 rows, n 18944, k 2048 with one row of NaN 0.26 ms, all
+// infinite 2.2 ms (DenseGemmTiled 0.85 ms); n 2048, k 10304: 0.80, 2.3 (1.4) ms.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -44,7 +45,7 @@ struct Layout {
   static_assert(kRaw >= BT * kTileStride * 4, "the partial tile aliases the planes");
   static constexpr int kBars = kRaw + kStages * kStage;
   static constexpr int kSlot = kBars + 8 * (6 + 2 * kStages);
-  static constexpr int kBytes = kSlot + 8 + 1024;  // slack to align to 1024
+  static constexpr int kBytes = kSlot + 16 + 1024;  // slack to align to 1024
   // Registers a thread of the three kinds of warpgroups; 128 * (2 * sum + 4 * split + mma) is the 896 * 72 of the launch.
   static constexpr int kSumRegs = 152, kSplitRegs = 40, kMmaRegs = 40;
   static_assert(128 * (2 * kSumRegs + 4 * kSplitRegs + kMmaRegs) <= kThreads * 72, "more registers than the launch has");
@@ -117,19 +118,6 @@ __device__ __forceinline__ void Split2(uint64_t xy, uint32_t& h, uint32_t& m, ui
   part(xy, l);
 }
 
-// One output with plain FMAs; a NaN stays one.
-__device__ __noinline__ float PlainDot(const float* x, const float* w, int k)
-{
-  float v = 0.f;
-  for (int i = 0; i < k && v == v; i += 4) {
-    const float4 a = __ldcg(reinterpret_cast<const float4*>(x + i)), b = __ldcg(reinterpret_cast<const float4*>(w + i));
-    v = fmaf(a.x, b.x, v);
-    v = fmaf(a.y, b.y, v);
-    v = fmaf(a.z, b.z, v);
-    v = fmaf(a.w, b.w, v);
-  }
-  return v;
-}
 __device__ __forceinline__ bool Doubtful(float v) { return !(fabsf(v) < INFINITY); }
 
 __device__ __forceinline__ const float* XRow(const tlaloc_b200_dense_problem& p, const Tile& t, int m)
@@ -146,22 +134,73 @@ __device__ __forceinline__ void Put(const tlaloc_b200_dense_problem& p, size_t a
   else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
 }
 
-// CH sums (times 2^48) of column n (a warp's lanes hold 32 consecutive columns), rows m, m + step, ... below end: epilogue and store.
-template <int CH>
-__device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const Tile& t, int n, int m, int step, int end, float* v)
+// Eight sums again with plain FMAs in k order (the plain kernel's bits): rows 0 .. last of x, ld apart, with a column of w a lane, by the whole warp.
+// Bound by the way of its words (the columns' are scattered); two steps' loads are in flight.  The rest of the CTA waits meanwhile, so it counts its
+// progress at `beat` (MbarWaitAlive).
+struct Sums {
+  float v[8];
+};
+__device__ __noinline__ Sums PlainSums(const float* x, size_t ld, int last, const float* w, int K, volatile uint32_t* beat)
 {
-  const size_t out = p.row_offsets != nullptr ? 0 : p.batch_y * t.b;
+  Sums s = {};
+#pragma unroll 2
+  for (int k = 0; k < K; k += 4) {
+    const float4 b = *reinterpret_cast<const float4*>(w + k);
+    float4 a[8];
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int r = m + c * step;
-    v[c] = n < p.n && r < end && Doubtful(v[c]) ? PlainDot(XRow(p, t, r), WRow(p, t, n), p.k) : v[c] * kDown;
+    for (int c = 0; c < 8; ++c) a[c] = *reinterpret_cast<const float4*>(x + min(c, last) * ld + k);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) s.v[c] = fmaf(a[c].w, b.w, fmaf(a[c].z, b.z, fmaf(a[c].y, b.y, fmaf(a[c].x, b.x, s.v[c]))));
+    if ((k & 511) == 0 && (threadIdx.x & 31) == 0) atomicAdd(const_cast<uint32_t*>(beat), 1u);
   }
+  return s;
+}
+
+// MbarWait that goes on while `words[1]` counts: sums that are computed again may take longer than the limit.
+__device__ __forceinline__ bool MbarWaitOn(uint32_t bar, uint32_t parity, volatile uint32_t* words)
+{
+  for (;;) {
+    const uint32_t seen = words[1];
+    if (MbarPoll(bar, parity, words)) return true;
+    if (words[0] != 0u || words[1] == seen) break;
+  }
+  words[0] = 1u;
+  return false;
+}
+__device__ __forceinline__ bool MbarWaitAlive(uint32_t bar, uint32_t parity, volatile uint32_t* words)
+{
+  return MbarPoll(bar, parity, words) || MbarWaitOn(bar, parity, words);
+}
+__device__ __forceinline__ bool MbarWaitAliveWarp(uint32_t bar, uint32_t parity, int lane, volatile uint32_t* words)
+{
+  int ok = 1;
+  if (lane == 0) ok = MbarWaitAlive(bar, parity, words) ? 1 : 0;
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// A tile is finished in two passes: what is sure is stored at once, the rest is computed again when the sums in registers are gone and only
+// bits say which; doing both at once cost registers on the way of every tile (203 rows, n 18944, k 2048: 118 us, 109 so).
+// Which of a lane's eight sums (times 2^48) have to be computed again, as bits; of a gated pair both have.
+__device__ __forceinline__ uint32_t DoubtfulBits(const tlaloc_b200_dense_problem& p, int n, int m, int step, int end, const float* v)
+{
+  uint32_t bits = 0;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) bits |= m + c * step < end && Doubtful(v[c]) ? 1u << c : 0u;
+  if (n >= p.n) bits = 0;
+  return IsGated(p.act) ? bits | __shfl_xor_sync(0xffffffffu, bits, kGateBlock) : bits;
+}
+
+// Eight finished sums of column n (a warp's lanes hold 32 consecutive columns), rows m, m + step, ... below end: epilogue and store of those whose bit is set.
+__device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const Tile& t, int n, int m, int step, int end, const float* v, uint32_t bits)
+{
+  constexpr int kU = 8;
+  const size_t out = p.row_offsets != nullptr ? 0 : p.batch_y * t.b;
   if (IsGated(p.act)) {  // gate and other factor are sixteen lanes apart
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
+    for (int c = 0; c < kU; ++c) {
       const int r = m + c * step;
       const float other = __shfl_xor_sync(0xffffffffu, v[c], kGateBlock);
-      if (n < p.n && r < end && (n & kGateBlock) == 0) {
+      if (n < p.n && r < end && (n & kGateBlock) == 0 && (bits >> c & 1u) != 0) {
         Put(p, out + static_cast<size_t>(r) * p.ld_y + (n >> 5) * kGateBlock + (n & 15), GatedValue(p.act, v[c], other));
       }
     }
@@ -169,17 +208,34 @@ __device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const
   }
   if (n >= p.n) return;
   const float bias = p.bias != nullptr ? __ldg(p.bias + n) : 0.f;
-  float res[CH];
+  float res[kU];
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
+  for (int c = 0; c < kU; ++c) {
     const int r = m + c * step;
     res[c] = p.residual != nullptr && r < end ? p.residual[static_cast<size_t>(r) * p.ld_res + n] : 0.f;
   }
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
+  for (int c = 0; c < kU; ++c) {
     const int r = m + c * step;
-    if (r < end) Put(p, out + static_cast<size_t>(r) * p.ld_y + n, DenseActivation(p.act, v[c] + bias) + res[c]);
+    if (r < end && (bits >> c & 1u) != 0) Put(p, out + static_cast<size_t>(r) * p.ld_y + n, DenseActivation(p.act, v[c] + bias) + res[c]);
   }
+}
+
+// The same for sums still times 2^48; leaves the bits of those that are not stored.
+__device__ __forceinline__ uint32_t FinishSure(const tlaloc_b200_dense_problem& p, const Tile& t, int n, int m, int step, int end, float* v)
+{
+  const uint32_t doubt = DoubtfulBits(p, n, m, step, end, v);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] *= kDown;
+  Finish(p, t, n, m, step, end, v, ~doubt);
+  return doubt;
+}
+__device__ __forceinline__ void FinishDoubtful(const tlaloc_b200_dense_problem& p, const Tile& t, int n, int m, int step, int end, uint32_t bits,
+                                               volatile uint32_t* beat)
+{
+  if (!__any_sync(0xffffffffu, bits != 0)) return;
+  const Sums s = PlainSums(XRow(p, t, m), static_cast<size_t>(step) * p.ld_x, (end - 1 - m) / step, WRow(p, t, min(n, p.n - 1)), p.k, beat);
+  Finish(p, t, n, m, step, end, s.v, bits);
 }
 
 __device__ __forceinline__ void ClusterSync()
@@ -232,9 +288,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t full = base + L::kBars, done = full + 16, empty = done + 16;  // planes written; a chunk's MMAs through; its accumulator added
   const uint32_t landed = empty + 16, freed = landed + 8 * S;                                      // a stage's boxes are there; split
   volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(smem + L::kSlot);
-  volatile uint32_t* abort_word = slot + 1;
+  volatile uint32_t* words = slot + 1;  // abort word; progress of sums computed again
   if (tid == 0) {
-    *abort_word = 0u;
+    words[0] = words[1] = 0u;
     for (int i = 0; i < 2; ++i) {
       MbarInit(full + 8 * i, kSplitWarps);
       MbarInit(done + 8 * i, 1);
@@ -294,8 +350,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int nb = Chunks(a, t, first);
         for (int c = 0; c < nb; ++c, ++it) {
           const int b = it & 1;
-          if (it >= 2) ok = MbarWait(empty + 8 * b, ((it >> 1) - 1) & 1, abort_word) && ok;
-          ok = MbarWait(full + 8 * b, (it >> 1) & 1, abort_word) && ok;
+          if (it >= 2) ok = MbarWaitAlive(empty + 8 * b, ((it >> 1) - 1) & 1, words) && ok;
+          ok = MbarWaitAlive(full + 8 * b, (it >> 1) & 1, words) && ok;
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           const uint32_t acc = tmem + b * L::kAcc;
           constexpr uint32_t P = L::kPlane >> 4;
@@ -349,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           round = ahead == S ? 1 : 0;
         }
         for (; c < nb; ++c) {
-          if (round > 0) ok = MbarWait(freed + 8 * s, (round - 1) & 1, abort_word) && ok;
+          if (round > 0) ok = MbarWaitAlive(freed + 8 * s, (round - 1) & 1, words) && ok;
           load_w(c, s);
           load_x(c, s);
           if (++s == S) {
@@ -386,8 +442,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       int first;
       const int nb = Chunks(a, t, first);
       for (int c = 0; c < nb; ++c, ++it) {
-        ok = MbarWaitWarp(landed + 8 * s, phase, lane, abort_word) && ok;
-        if (it >= 2) ok = MbarWaitWarp(done + 8 * (it & 1), ((it >> 1) - 1) & 1, lane, abort_word) && ok;
+        ok = MbarWaitAliveWarp(landed + 8 * s, phase, lane, words) && ok;
+        if (it >= 2) ok = MbarWaitAliveWarp(done + 8 * (it & 1), ((it >> 1) - 1) & 1, lane, words) && ok;
         const uint32_t from = from0 + s * L::kStage, to = to0 ^ ((it & 1) << 6);
 #pragma unroll
         for (int i = 0; i < (kBN + BT) / 8; i += kSplitWarps) {
@@ -437,7 +493,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[q][e] = 0.f;
       for (int c = 0; c < nb; ++c, ++it) {
-        ok = MbarWaitWarp(done + 8 * (it & 1), (it >> 1) & 1, lane, abort_word) && ok;
+        ok = MbarWaitAliveWarp(done + 8 * (it & 1), (it >> 1) & 1, lane, words) && ok;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t from = tmem + (static_cast<uint32_t>(quad * 32) << 16) + (it & 1) * L::kAcc + col0;
 #pragma unroll
@@ -459,9 +515,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) MbarArrive(empty + 8 * (it & 1));
       }
       if (a.ks <= 1) {
+        const int n = t.n0 + quad * 32 + lane, m = t.m0 + col0;
+        uint32_t doubt[(L::kUnits + 3) / 4] = {};
 #pragma unroll
         for (int q = 0; q < L::kUnits; ++q)
-          if (q < units) Finish<8>(p, t, t.n0 + quad * 32 + lane, t.m0 + col0 + q * 8, 1, t.M, acc[q]);
+          if (q < units) doubt[q >> 2] |= FinishSure(p, t, n, m + q * 8, 1, t.M, acc[q]) << 8 * (q & 3);
+#pragma unroll
+        for (int i = 0; i < (L::kUnits + 3) / 4; ++i)
+          for (int q = 0; q < 4 && __any_sync(0xffffffffu, doubt[i] != 0); ++q, doubt[i] >>= 8) {
+            FinishDoubtful(p, t, n, m + (i * 4 + q) * 8, 1, t.M, doubt[i] & 255u, words + 1);
+          }
       } else {
         float* tile = reinterpret_cast<float*>(smem);  // over the planes: every MMA of this CTA's one tile is through
 #pragma unroll
@@ -492,7 +555,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int e = 0; e < kU; ++e) v[e] += w[e];
         }
-        Finish<kU>(p, t, t.n0 + nl, t.m0 + c0, step, t.m0 + rows, v);
+        const uint32_t doubt = FinishSure(p, t, t.n0 + nl, t.m0 + c0, step, t.m0 + rows, v);
+        FinishDoubtful(p, t, t.n0 + nl, t.m0 + c0, step, t.m0 + rows, doubt, words + 1);
       }
       ClusterSync();  // no CTA leaves while a peer may still read its tile
     }

@@ -26,9 +26,9 @@ __device__ __forceinline__ void MbarInit(uint32_t bar, uint32_t count)
 }
 // Waits for the phase with the given parity.  Bounded twice over: a wait gives up after kTcWaitNs of wall time, and the
 // first wait of a CTA that gives up raises the CTA's abort word in shared memory, which every other wait polls, so a
-// pipeline that has stopped costs one time limit and not one per block.  Returns false when it gave up.
+// pipeline that has stopped costs one time limit and not one per block.  Returns false when it gave up (MbarPoll: without raising the word).
 constexpr unsigned long long kTcWaitNs = 200ull * 1000ull * 1000ull;  // 0.2 s: a block takes under a microsecond
-__device__ __forceinline__ bool MbarWait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word)
+__device__ __forceinline__ bool MbarPoll(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word)
 {
   unsigned long long t0 = 0;
   for (uint32_t i = 0; i < kTcSpinLimit; ++i) {
@@ -49,6 +49,11 @@ __device__ __forceinline__ bool MbarWait(uint32_t bar, uint32_t parity, volatile
       else if (now - t0 > kTcWaitNs) break;
     }
   }
+  return false;
+}
+__device__ __forceinline__ bool MbarWait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_word)
+{
+  if (MbarPoll(bar, parity, abort_word)) return true;
   *abort_word = 1u;
   return false;
 }
