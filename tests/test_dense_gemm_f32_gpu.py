@@ -140,6 +140,27 @@ def test_tiles_of_infinities_before_finite_ones(m, n, k, act):
         assert bool(((y[:, 148 * 128:].double() - want).abs() <= bound(x, w[148 * 128:])).all())
 
 
+@pytest.mark.parametrize("batch_x,batch_w", [(0, None), (None, 0), (None, 4), (4, None), (0, 0), (100 * 64, 0)])
+def test_batches_that_share_or_overlap(batch_x, batch_w):
+    """Strides between batch entries that a tensor map may not have: the same rows or weights for all of them, or each four values further on."""
+    b, m, n, k = 5, 40, 96, 64
+    x, w, y = rand(b * 100 * k), rand(b * n * k, seed=1), torch.empty((b, m, n), device=DEV)
+    p = ops().dense(x[:b * m * k].view(b, m, k), w.view(b, n, k), y)
+    p.batch_x = p.batch_x if batch_x is None else batch_x
+    p.batch_w = p.batch_w if batch_w is None else batch_w
+    ops().dense_gemm(p)
+    xs, ws = x.as_strided((b, m, k), (p.batch_x, k, 1)), w.as_strided((b, n, k), (p.batch_w, k, 1))
+    assert bool(((y.double() - xs.double() @ ws.double().transpose(1, 2)).abs() <= bound(xs, ws)).all())
+
+
+def test_a_row_stride_beyond_tensor_maps():
+    x, w, y = rand(1, 64), rand(96, 64, seed=1), torch.empty((1, 96), device=DEV)
+    p = ops().dense(x, w, y)
+    p.ld_x = 1 << 38  # of one row: never used
+    ops().dense_gemm(p)
+    assert bool(((y.double() - x.double() @ w.double().T).abs() <= bound(x, w)).all())
+
+
 @pytest.mark.parametrize("sizes", [[0, 3, 40, 0, 70, 1], [5] * 64, [300, 0]])
 @pytest.mark.parametrize("act", [0, 2])
 def test_groups(sizes, act):

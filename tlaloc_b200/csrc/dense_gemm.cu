@@ -123,8 +123,8 @@ extern "C" int tlaloc_b200_dense_gemm(const tlaloc_b200_dense_problem* problems,
   bool split = dtype == TLALOC_B200_F32 && !OrderFaithful();
   for (int i = 0; i < count; ++i) split = split && DenseGemmF32Applies(problems[i], m);
   if (split) {
-    e = LaunchDenseGemmF32(problems, count, m, (flags & TLALOC_B200_GEMM_WEIGHTS_CONST) != 0, st);
-    launches = 1;
+    e = LaunchDenseGemmF32(problems, count, m, (flags & TLALOC_B200_GEMM_WEIGHTS_CONST) != 0, st, &split);
+    launches = split ? 1 : 0;
   }
   for (int i = 0; i < count && e == cudaSuccess && !tc && !split; ++i) {
     e = dtype == TLALOC_B200_F32 ? LaunchTiled<float>(problems[i], m, st) : LaunchTiled<__nv_bfloat16>(problems[i], m, st);

@@ -684,11 +684,13 @@ bool DenseGemmF32Applies(const tlaloc_b200_dense_problem& p, int m)
 {
   const long long rows = p.rows > 0 ? p.rows : m;
   return p.k % 4 == 0 && p.ld_x % 4 == 0 && Aligned16(p.x) && Aligned16(p.w) && (p.batch == 1 || (p.batch_x % 4 == 0 && p.batch_w % 4 == 0)) &&
+         (p.batch == 1 || ((p.row_offsets != nullptr || p.batch_x >= p.k) && p.batch_w >= p.k)) && TensorMapEncoder() != nullptr &&
          (rows / 16 + p.batch + 1) * ((p.n + kBN - 1) / kBN) * (p.row_offsets != nullptr ? 1 : p.batch) < (1ll << 30);
 }
 
-cudaError_t LaunchDenseGemmF32(const tlaloc_b200_dense_problem* problems, int count, int m, bool weights_const, cudaStream_t st)
+cudaError_t LaunchDenseGemmF32(const tlaloc_b200_dense_problem* problems, int count, int m, bool weights_const, cudaStream_t st, bool* taken)
 {
+  *taken = true;
   cudaError_t e = PrepareDenseF32();
   if (e != cudaSuccess) return e;
   // Rows of a tile: what the problem has in equal parts of up to 208, or what a group has on average (one that has more takes several tiles).
@@ -710,7 +712,8 @@ cudaError_t LaunchDenseGemmF32(const tlaloc_b200_dense_problem* problems, int co
     int swap_w = 0;
     if (!EncodeMatrix(&maps[2 * i], s.w, s.k, s.n, s.batch, s.k, s.batch_w, kBN, &swap_w) || swap_w ||
         !EncodeMatrix(&maps[2 * i + 1], s.x, s.k, a.M[i], s.row_offsets != nullptr ? 1 : s.batch, s.ld_x, s.batch_x, a.bt, &a.swap_x[i])) {
-      return cudaErrorInvalidValue;
+      *taken = false;  // strides that no tensor map has (2^40 bytes and more)
+      return cudaSuccess;
     }
     a.tiles_m[i] = (a.M[i] + a.bt - 1) / a.bt;
     a.tiles_n[i] = (s.n + kBN - 1) / kBN;
