@@ -331,9 +331,11 @@ typedef struct tlaloc_b200_dense_problem {
 
 /*
  * `count` (1 or 2) projections of the same m rows (or of `rows` of their own) in one launch where a tensor-core kernel takes them, else one launch
- * each.  dtype: F32 or BF16, the type of x and w of every problem; y is F32 or BF16 per problem.  F32 products are exact
- * to the last place of f32 (on the tensor cores: each operand as three bf16 parts, the sums no further from 64 bits than f32 FMAs in k order).  flags: TLALOC_B200_GEMM_WEIGHTS_CONST.  Two problems of one call must not depend on
- * each other's results.
+ * each.  dtype: F32 or BF16, the type of x and w of every problem; y is F32 or BF16 per problem.  F32 operands count
+ * with all their bits, subnormal ones too: with f32 FMAs in k order, or (k from 32, dense_gemm_f32.cu) as three bf16 parts on the tensor cores, whose sums
+ * came out closer to 64 bits than those FMAs for normal and for one-signed operands at every k measured (32 to 10304, 2-norm); a sum that one
+ * product outweighs may be off by two units of its last place there.  flags: TLALOC_B200_GEMM_WEIGHTS_CONST.  Two problems of one call must not
+ * depend on each other's results.
  */
 int tlaloc_b200_dense_gemm(const tlaloc_b200_dense_problem* problems, int32_t count, int32_t dtype, int32_t m, int32_t flags,
                            void* stream);

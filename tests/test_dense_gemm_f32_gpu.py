@@ -71,6 +71,18 @@ def test_no_further_from_f64_than_plain_sums(m, k):
     assert float((y - want).norm()) <= float((in_order(x, w) - want).norm())
 
 
+@pytest.mark.parametrize("m", [4, 200])
+@pytest.mark.parametrize("k", [4, 16, 28, 32, 36, 64, 128, 512])
+@pytest.mark.parametrize("signs", ["both", "one", "near one"])
+def test_no_further_from_f64_at_few_k(m, k, signs):
+    x, w = rand(m, k), rand(512, k, seed=1)
+    if signs != "both":
+        x, w = (torch.sigmoid(a) if signs == "one" else 1 + 1e-3 * torch.sigmoid(a) for a in (x, w))
+    y, want = torch.empty((m, 512), device=DEV), x.double() @ w.double().T
+    ops().dense_gemm(ops().dense(x, w, y))
+    assert float((y - want).norm()) <= float((in_order(x, w) - want).norm())
+
+
 # k 2048: slices of k; n 19000: none
 @pytest.mark.parametrize("m,n,k", [(9, 200, 2048), (200, 200, 2048), (9, 19000, 96), (200, 19000, 96)])
 @pytest.mark.parametrize("large", [1.0, 1e10, 1e20, 1e30, 1e38])

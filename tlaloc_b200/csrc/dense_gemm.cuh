@@ -34,9 +34,8 @@ __device__ __forceinline__ float DenseEpilogue(const tlaloc_b200_dense_problem& 
 // The tensor-core kernel (dense_gemm_tc.cu): bf16 x and w whose addresses, row and batch strides are multiples of 16 bytes.
 bool DenseGemmTcApplies(const tlaloc_b200_dense_problem& p);
 cudaError_t LaunchDenseGemmTc(const tlaloc_b200_dense_problem* problems, int count, int m, bool weights_const, cudaStream_t st);
-// The tensor-core kernel of f32 x and w (dense_gemm_f32.cu): k, row and batch strides multiples of four, 16-byte addresses, batch
-// entries that neither share nor overlap their rows' words.  *taken: false, and nothing
-// launched, where no tensor map has the operands' strides.
+// The tensor-core kernel of f32 x and w (dense_gemm_f32.cu): k from 32, k, row and batch strides multiples of four, 16-byte addresses, batch
+// entries that neither share nor overlap their rows' words.  *taken: false, and nothing launched, where no tensor map has the operands' strides.
 bool DenseGemmF32Applies(const tlaloc_b200_dense_problem& p, int m);
 cudaError_t LaunchDenseGemmF32(const tlaloc_b200_dense_problem* problems, int count, int m, bool weights_const, cudaStream_t st, bool* taken);
 

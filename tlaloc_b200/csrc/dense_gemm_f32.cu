@@ -3,8 +3,12 @@
 //
 // Accuracy.  Products of parts are exact; what is left out (middle x low, low x low) is below 2^-26 of a product and of either sign.  An
 // accumulator in TMEM holds one chunk of 32 k only, its small products first and its large ones last; the chunks are summed in registers with
-// rounding to nearest.  So a sum of k products has k / 32 rounded additions where the plain kernel (dense_gemm.cu) has k, and its error
-// against 64 bits (2-norm, relative) is the smaller one at every k: k = 128: 0.7e-7 and the plain kernel's 2.0e-7; 2048: 1.2e-7, 8.1e-7; 10304: 1.6e-7, 1.8e-6.
+// rounding to nearest.  So a sum of k products has k / 32 rounded additions where the plain kernel (dense_gemm.cu) has k; but inside a chunk the
+// tensor core cuts what it adds.  Error against 64 bits (2-norm over 200 x 512 sums, relative, 1e-7) and the plain kernel's:
+//   k          4            16           32           128          2048         10304
+//   normal     0.46  0.40   0.48  0.73   0.57  1.02   0.71  2.04   0.97  8.04   1.43  18.1
+//   1 .. 1.001 0.69  0.43   0.69  0.63   0.69  0.81   0.78  1.51   0.82  5.91   0.84  15.7
+// hence the plain kernel below k = 32.  A sum that one product outweighs is cut where the plain kernel rounds: 1.4e-7 and 0.3e-7 at worst (k = 32).
 // bf16 ends where f32 does (2^-149 is f32's last place there, 2^-126 bf16's smallest normal number), so the parts of small operands would lose
 // their low bits: operands are split after a multiplication by 2^24, which leaves every nonzero part normal, and a finished sum is
 // multiplied by 2^-48.  What gets too large by that (an operand of 2^104, a sum of 2^80 and more), an infinity or a NaN makes a part infinite
@@ -683,7 +687,7 @@ cudaError_t Launch(const CUtensorMap* maps, const F32Args& a, int ctas, cudaStre
 bool DenseGemmF32Applies(const tlaloc_b200_dense_problem& p, int m)
 {
   const long long rows = p.rows > 0 ? p.rows : m;
-  return p.k % 4 == 0 && p.ld_x % 4 == 0 && Aligned16(p.x) && Aligned16(p.w) && (p.batch == 1 || (p.batch_x % 4 == 0 && p.batch_w % 4 == 0)) &&
+  return p.k >= kBK && p.k % 4 == 0 && p.ld_x % 4 == 0 && Aligned16(p.x) && Aligned16(p.w) && (p.batch == 1 || (p.batch_x % 4 == 0 && p.batch_w % 4 == 0)) &&
          (p.batch == 1 || ((p.row_offsets != nullptr || p.batch_x >= p.k) && p.batch_w >= p.k)) && TensorMapEncoder() != nullptr &&
          (rows / 16 + p.batch + 1) * ((p.n + kBN - 1) / kBN) * (p.row_offsets != nullptr ? 1 : p.batch) < (1ll << 30);
 }
