@@ -163,3 +163,22 @@ def test_batch_of_40_with_swiglu_in_the_projection_epilogue_matches_the_oracle()
             swaps += 1
     print(f"near-tie swaps: {swaps} of {64 * B}")
     assert swaps <= 0.015 * 64 * B  # observed: 13 of 2560
+
+
+def test_rows_asked_for_in_every_form():
+    """`run`'s rows as anything that indexes a tensor: lists, arrays, tensors on either side, a single one, rows of rows."""
+    from tlaloc_b200 import paging
+
+    *_, dec, tables, prompts, _, _, _ = _setup(torch.bfloat16, True)
+    seqs = [paging.Sequence(pages=[int(p) for p in t]) for t in tables]
+    step = paging.stage_ragged([(s, p[:1]) for s, p in zip(seqs, prompts)], max_blocks=tables.shape[1], block_size=16)
+    every = dec.run(step, range(4)).clone()
+    assert torch.equal(every, dec.logits)
+    for want in ([2, 0], [-1], [], np.array([3, 3]), torch.tensor([1, 2]), torch.tensor([1, -2], device="cuda:0"), [[0, 1], [2, 3]], 2,
+                 torch.tensor(1, device="cuda:0"), [0, 1, 2, 3, 3, 3]):
+        rows = torch.as_tensor(want, dtype=torch.long)
+        got = dec.run(step, want)
+        assert got.shape == (*rows.shape, every.shape[1]) and torch.equal(got, every[rows.to(every.device)])
+    for want in ([4], [[0, 1], [2, -5]]):
+        with pytest.raises(IndexError):
+            dec.run(step, want)

@@ -91,11 +91,14 @@ class StepModel:
             ops.unpack_i32(self._packed[:total], [dst for dst, _ in pairs])
 
     def _wanted(self, want, rows: int):
-        """Indices as a list takes them (negative ones from the end), as int32; None where they do not fit `want_rows`."""
-        want = np.asarray(want, np.int64).reshape(-1)
+        """Indices as a list takes them (negative ones from the end), as int32; None where they are not a list on the host that fits `want_rows`."""
+        want = torch.as_tensor(want, dtype=torch.long)
+        if want.device.type != "cpu":
+            return None
+        shape, want = want.shape, want.reshape(-1).numpy()
         if want.size and (want.min() < -rows or want.max() >= rows):
             raise IndexError(f"rows {want.tolist()} of {rows}")
-        return np.where(want < 0, want + rows, want).astype(np.int32) if want.size <= self.max_sequences else None
+        return np.where(want < 0, want + rows, want).astype(np.int32) if len(shape) == 1 and want.size <= self.max_sequences else None
 
     def capture(self, rows: int | None = None) -> None:
         """Capture the step over `rows` rows into a CUDA graph (after one eager warm-up step on a side stream)."""
