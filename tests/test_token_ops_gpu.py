@@ -78,3 +78,23 @@ def test_inputs_of_steps_in_flight_do_not_mix():
         assert all(np.array_equal(g.cpu().numpy(), w) for g, w in zip(got, want))
     with pytest.raises(RuntimeError):
         m.set_inputs(sent[0][0][:7], None, None, None, None)
+
+
+@pytest.mark.parametrize("as_array", [False, True])
+def test_page_locked_inputs_are_read_in_stream_order(as_array):
+    """A copy from the device into the inputs is still on its way when they are handed over."""
+    from tlaloc_b200.step_model import StepModel
+
+    m = StepModel(50, 50, 8, 30, 16, 100, DEV)
+    pinned = [torch.zeros(s, dtype=torch.int32).pin_memory() for s in ((50,), (50,), (50, 30), (50,), (50,))]
+    coming = [torch.randint(0, 99, tuple(p.shape), dtype=torch.int32, device=DEV) for p in pinned]
+    a = torch.randn((8192, 8192), device=DEV)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        a = a @ a * 1e-4
+    for p, c in zip(pinned, coming):
+        p.copy_(c, non_blocking=True)
+    m.set_inputs(*([p.numpy() for p in pinned] if as_array else pinned))
+    torch.cuda.synchronize()
+    for got, want in zip((m.token_ids, m.positions, m.block_tables, m.seq_lens, m.slot_mapping), coming):
+        assert torch.equal(got, want)

@@ -47,7 +47,8 @@ class StepModel:
         raise NotImplementedError
 
     def set_inputs(self, token_ids, positions, block_tables, seq_lens, slot_mapping) -> None:
-        """Host (NumPy or pinned torch) step inputs -> the device buffers the graph reads."""
+        """Host (NumPy or torch) step inputs -> the device buffers the graph reads.  Page-locked inputs are read in stream order, so a copy into
+        them may still be on its way, and they stay as they are until the stream has read them; others are read before this returns."""
         self._put_all([(self.token_ids, token_ids), (self.positions, positions), (self.block_tables, block_tables),
                        (self.seq_lens, seq_lens), (self.slot_mapping, slot_mapping)])
 
@@ -59,14 +60,24 @@ class StepModel:
             src = torch.from_numpy(np.ascontiguousarray(src, dtype=np.int32))
         dst.copy_(src.reshape(dst.shape), non_blocking=True)
 
+    @staticmethod
+    def _in_stream_order(src) -> bool:
+        """True for an input that is not to be read now: on the device, or in page-locked memory (a view of it as an array too)."""
+        if isinstance(src, torch.Tensor):
+            return src.is_cuda or src.is_pinned()
+        base = src
+        while isinstance(base, np.ndarray):
+            base = base.base
+        return base is not None and src.dtype == np.int32 and src.flags.c_contiguous and torch.from_numpy(src).is_pinned()
+
     def _put_all(self, pairs) -> None:
         """Host sources into device buffers [(buffer, source or None)], all with one copy: the buffers are contiguous."""
         pairs = [(dst, src) for dst, src in pairs if src is not None]
-        if self.device.type != "cuda" or torch.cuda.is_current_stream_capturing() or any(isinstance(src, torch.Tensor) and src.is_cuda for _, src in pairs):
+        if self.device.type != "cuda" or torch.cuda.is_current_stream_capturing() or any(self._in_stream_order(src) for _, src in pairs):
             for dst, src in pairs:
                 self._put(dst, src)
             return
-        host = [src.numpy() if isinstance(src, torch.Tensor) else np.asarray(src) for _, src in pairs]
+        host = [src.numpy() if isinstance(src, torch.Tensor) else src for _, src in pairs]
         for (dst, _), src in zip(pairs, host):
             if src.size != dst.numel():
                 raise RuntimeError(f"an input of shape {src.shape} does not fit {tuple(dst.shape)}")
