@@ -98,3 +98,12 @@ def test_page_locked_inputs_are_read_in_stream_order(as_array):
     torch.cuda.synchronize()
     for got, want in zip((m.token_ids, m.positions, m.block_tables, m.seq_lens, m.slot_mapping), coming):
         assert torch.equal(got, want)
+
+
+def test_the_first_step_locks_no_pages():
+    from tlaloc_b200.step_model import StepModel
+
+    m = StepModel(50, 50, 8, 30, 16, 100, DEV)
+    before = torch.cuda.host_memory_stats()["num_host_alloc"]
+    m.set_inputs(*(np.zeros(s, np.int32) for s in ((50,), (50,), (50, 30), (50,), (50,))))
+    assert torch.cuda.host_memory_stats()["num_host_alloc"] == before

@@ -36,10 +36,13 @@ class StepModel:
         self.seq_lens = torch.ones((rows,), **i32)
         self.slot_mapping = torch.full((rows,), PADDING_SLOT, **i32)
         self.want_rows = torch.zeros((tables,), **i32)  # rows whose logits are asked for
-        # a step's inputs on their way: two pinned copies in turn (one is filled while the other travels) and where they arrive
-        self._pinned: list[torch.Tensor] = []
-        self._sent: list[torch.cuda.Event] = []
-        self._packed: torch.Tensor | None = None
+        # a step's inputs on their way: two pinned copies in turn (one is filled while the other travels) and where they arrive.  Page-locking takes
+        # milliseconds, ten times a small step: here, not at the first one
+        if self.device.type == "cuda":
+            most = 6 * rows + self.block_tables.numel() + tables
+            self._pinned = torch.empty((2, most), dtype=torch.int32, pin_memory=True)
+            self._sent = [torch.cuda.Event() for _ in range(2)]
+            self._packed = torch.empty((most,), **i32)
         self._turn = 0
         self._graphs: dict[int, torch.cuda.CUDAGraph] = {}
 
@@ -84,11 +87,6 @@ class StepModel:
         total = sum(src.size for src in host)
         if total == 0:
             return
-        if self._packed is None:
-            most = 6 * self.rows + self.block_tables.numel() + self.max_sequences
-            self._pinned = [torch.empty((most,), dtype=torch.int32, pin_memory=True) for _ in range(2)]
-            self._sent = [torch.cuda.Event() for _ in range(2)]
-            self._packed = torch.empty((most,), dtype=torch.int32, device=self.device)
         turn = self._turn
         self._turn ^= 1
         self._sent[turn].synchronize()  # the copy before last has left
