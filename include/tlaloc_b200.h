@@ -378,7 +378,8 @@ int tlaloc_b200_rope_interleaved(const void* in, int64_t in_ld_token, int64_t in
  * over the positions j of the row's sequence with seq_lens[t] - window <= j < seq_lens[t] (window 0: all j < seq_lens[t]).
  * query [T, H, kv_rank + rot_dim], out [T, H, kv_rank], pool rows pool_ld elements apart, all of `dtype`; block_tables i32
  * [num_tables, max_blocks] of pages of block_size rows; row_tables i32 [T] names each row's table (NULL: row t uses table t).
- * scratch: tlaloc_b200_latent_attention_scratch_bytes; scores, weights and sums are f32.
+ * scratch: tlaloc_b200_latent_attention_scratch_bytes; scores, weights and sums are f32.  max_live: the most positions that any row
+ * sees, by which rows are cut into slices (0: what window and table allow).
  */
 size_t tlaloc_b200_latent_attention_scratch_bytes(int32_t num_tokens, int32_t num_heads, int32_t kv_rank, int32_t rot_dim,
                                                   int32_t max_live);

@@ -178,6 +178,29 @@ def test_absorbed_attention_over_pages(dtype, heads, kv_rank, rot_dim, window, b
     assert float((one[0].double() - results[0][7].double()).abs().max()) <= tol(dtype)
 
 
+@pytest.mark.parametrize("heads,kv_rank,rot_dim", SHAPES)
+@pytest.mark.parametrize("window", [0, 500])
+@pytest.mark.parametrize("max_live", [0, 1000, 400, 200, 1])
+def test_absorbed_attention_in_f32_over_slices_of_unequal_rows(heads, kv_rank, rot_dim, window, max_live):
+    """Rows of no position to a thousand and a portion beside them, cut into slices for rows of `max_live` positions, shorter than some."""
+    from tlaloc_b200 import ops
+
+    row = kv_rank + rot_dim
+    lens = [1, 15, 17, 160, 1000, 999]
+    seqs = [randn(n, row, seed=n, dtype=torch.float32) for n in lens]
+    pool, table = paged(seqs, 16, row, torch.float32)
+    which = torch.tensor([0, 1, 2, 3, 4, 5, 4] + [5] * 9, dtype=torch.int32, device=DEV)
+    ends = torch.tensor(lens + [0] + list(range(600, 609)), dtype=torch.int32, device=DEV)
+    q = randn(len(which), heads, row, seed=9, dtype=torch.float32)
+    out = torch.full((len(which) + 1, heads, kv_rank), 7.0, device=DEV)
+    ops.latent_attention(q, pool, table, ends, out[:-1], kv_rank=kv_rank, scale=1.7 * row ** -0.5, window=window, row_tables=which,
+                         scratch=torch.full((1 << 22,), float("nan"), device=DEV), max_live=max_live)
+    for t, hi in enumerate(ends.tolist()):
+        want = attend(q[t], seqs[int(which[t])], kv_rank, 1.7 * row ** -0.5, max(0, hi - window) if window else 0, hi) if hi else 0
+        assert float((out[t].double() - want).abs().max()) <= tol(torch.float32, 2.5), (t, hi)
+    assert bool((out[-1] == 7).all())
+
+
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("window", [40, 64, 129, 700])
 def test_absorbed_attention_needle_at_the_window_edge(dtype, window):

@@ -159,8 +159,9 @@ __global__ void __launch_bounds__(kF32Threads, 1) LatentAttentionF32(LatentParam
   const int slice = blockIdx.x, h0 = blockIdx.y * kF32Heads + quad * 4, t = blockIdx.z;
   const int words = p.row >> 2, vwords = p.kv_rank >> 2;
   const int2 live = LiveRange(p, t);
-  const int tile0 = live.x / kF32Tile + slice * sp.slice_tiles;
-  const int n = min((live.y + kF32Tile - 1) / kF32Tile, tile0 + sp.slice_tiles) - tile0;
+  // The last slice goes to the row's end, wherever that is: a row may see more than the launch was cut for.
+  const int tile0 = live.x / kF32Tile + slice * sp.slice_tiles, end = (live.y + kF32Tile - 1) / kF32Tile;
+  const int n = (slice + 1 < sp.slices ? min(end, tile0 + sp.slice_tiles) : end) - tile0;
   if (n <= 0 && sp.records != nullptr) return;  // an empty slice writes nothing
   const int* table = TableOf(p, t);
   const float* pool = static_cast<const float*>(p.pool);
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(128) LatentCombineF32(LatentParams p, F32Slice
   const int h = blockIdx.x, t = blockIdx.y;
   const int2 live = LiveRange(p, t);
   const int tiles = live.y > live.x ? (live.y + kF32Tile - 1) / kF32Tile - live.x / kF32Tile : 0;
-  const int n = (tiles + sp.slice_tiles - 1) / sp.slice_tiles;
+  const int n = min((tiles + sp.slice_tiles - 1) / sp.slice_tiles, sp.slices);
   const float* rec = sp.records + (static_cast<size_t>(t) * p.H + h) * (p.kv_rank + 2);
   const size_t step = static_cast<size_t>(p.T) * p.H * (p.kv_rank + 2);
   float top = -INFINITY, sum = 0.f;
