@@ -201,6 +201,30 @@ def test_absorbed_attention_in_f32_over_slices_of_unequal_rows(heads, kv_rank, r
     assert bool((out[-1] == 7).all())
 
 
+@pytest.mark.parametrize("heads,kv_rank,rot_dim", [(16, 512, 64), (5, 36, 8), (20, 256, 4)])
+@pytest.mark.parametrize("rows", [1, 3, 40])
+def test_absorbed_attention_in_f32_with_the_scratch_asked_for(heads, kv_rank, rot_dim, rows):
+    """The size reported is enough for the slices that any size would give, and nothing behind it is written; channels in multiples of four alone too."""
+    from tlaloc_b200 import ops
+
+    row = kv_rank + rot_dim
+    seqs = [randn(n, row, seed=n, dtype=torch.float32) for n in (700, 1600)]
+    pool, table = paged(seqs, 16, row, torch.float32)
+    which, ends = torch.arange(rows, device=DEV).int() % 2, torch.tensor([700, 1600] * rows, dtype=torch.int32, device=DEV)[:rows]
+    q = randn(rows, heads, row, seed=9, dtype=torch.float32)
+    size = ops.latent_attention_scratch_bytes(rows, heads, kv_rank, rot_dim, 1600) // 4
+    assert size >= 2 * rows * heads * (kv_rank + 2)
+    out = [torch.empty((rows, heads, kv_rank), device=DEV) for _ in range(2)]
+    for o, n in zip(out, (size, 1 << 24)):
+        scratch = torch.full((n + 4096,), 7.0, device=DEV)
+        ops.latent_attention(q, pool, table, ends, o, kv_rank=kv_rank, scale=row ** -0.5, row_tables=which, scratch=scratch[:n], max_live=1600)
+        assert bool((scratch[n:] == 7).all())
+    assert torch.equal(*out)
+    for t in range(rows):
+        want = attend(q[t], seqs[t % 2], kv_rank, row ** -0.5, 0, int(ends[t]))
+        assert float((out[0][t].double() - want).abs().max()) <= tol(torch.float32)
+
+
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("window", [40, 64, 129, 700])
 def test_absorbed_attention_needle_at_the_window_edge(dtype, window):

@@ -351,22 +351,23 @@ __global__ void __launch_bounds__(128) LatentCombineF32(LatentParams p, F32Slice
   }
 }
 
+bool F32Sizes(int kv_rank, int row) { return kv_rank % 4 == 0 && row % 4 == 0 && kv_rank <= 512 && row <= 640; }
 bool F32Applies(const LatentParams& p)
 {
-  return p.kv_rank % 4 == 0 && p.row % 4 == 0 && p.kv_rank <= 512 && p.row <= 640 && p.pool_ld % 4 == 0 && Aligned16(p.query) && Aligned16(p.pool) &&
-         Aligned16(p.out) && p.T <= 65535;
+  return F32Sizes(p.kv_rank, p.row) && p.pool_ld % 4 == 0 && Aligned16(p.query) && Aligned16(p.pool) && Aligned16(p.out) && p.T <= 65535;
 }
+size_t F32Record(int rows, int heads, int kv_rank) { return static_cast<size_t>(rows) * heads * (kv_rank + 2) * sizeof(float); }
 constexpr int F32Smem(int nw) { return kF32Stages * kF32Tile * nw * 32 * 16; }
 
 // Slices of the positions: waves of CTAs (one an SM) times the tiles of the longest, and what a slice's start and its record cost (in tiles).
-F32Slices ChooseF32Slices(const LatentParams& p, int max_live, void* scratch, size_t scratch_bytes)
+F32Slices ChooseF32Slices(int rows, int heads, int kv_rank, int max_live, size_t scratch_bytes)
 {
   const int tiles = (max_live + kF32Tile - 1) / kF32Tile + 1, slots = 148;
-  const long long ctas = static_cast<long long>(p.T) * ((p.H + kF32Heads - 1) / kF32Heads);
-  const size_t record = static_cast<size_t>(p.T) * p.H * (p.kv_rank + 2) * sizeof(float);
+  const long long ctas = static_cast<long long>(rows) * ((heads + kF32Heads - 1) / kF32Heads);
+  const size_t record = F32Record(rows, heads, kv_rank);
   F32Slices best = {nullptr, 1, 0x3fffffff};
   double best_cost = 1e30;
-  for (int s = 1; s <= std::min(tiles, 64) && (s == 1 || (scratch != nullptr && Aligned16(scratch) && record * s <= scratch_bytes)); ++s) {
+  for (int s = 1; s <= std::min(tiles, 64) && (s == 1 || record * s <= scratch_bytes); ++s) {
     const int per = (tiles + s - 1) / s;
     const double waves = static_cast<double>((ctas * s + slots - 1) / slots);
     const double cost = waves * (per + 3.0) + (s > 1 ? 3.0 + 0.1 * s * static_cast<double>(ctas) / slots : 0.0);
@@ -376,7 +377,6 @@ F32Slices ChooseF32Slices(const LatentParams& p, int max_live, void* scratch, si
       best.slice_tiles = s > 1 ? per : 0x3fffffff;
     }
   }
-  if (best.slices > 1) best.records = static_cast<float*>(scratch);
   return best;
 }
 
@@ -912,13 +912,14 @@ using namespace tlaloc_b200;
 extern "C" size_t tlaloc_b200_latent_attention_scratch_bytes(int32_t num_tokens, int32_t num_heads, int32_t kv_rank, int32_t rot_dim,
                                                              int32_t max_live)
 {
-  if (num_tokens < 1 || num_heads < 1 || max_live < 1 || !MmaApplies(num_heads, kv_rank, rot_dim)) return 0;
-  // fewer rows may take more slices: the largest need over the row counts up to num_tokens
+  if (num_tokens < 1 || num_heads < 1 || kv_rank < 1 || rot_dim < 0 || max_live < 1) return 0;
+  const bool bf16 = MmaApplies(num_heads, kv_rank, rot_dim), f32 = F32Sizes(kv_rank, kv_rank + rot_dim);
+  // fewer rows may take more slices: the largest need over the row counts up to num_tokens, and over the two types
   size_t most = 0;
   for (int rows = 1;; rows = std::min(2 * rows, num_tokens)) {
-    int tiles = 0;
-    const int s = ChooseLatentSlices(rows, num_heads, kv_rank, max_live, &tiles);
-    if (s > 1) most = std::max(most, static_cast<size_t>(s) * std::min(2 * rows, num_tokens) * num_heads * (kv_rank + 2) * sizeof(float));
+    int tiles = 0, s = bf16 ? ChooseLatentSlices(rows, num_heads, kv_rank, max_live, &tiles) : 1;
+    if (f32) s = std::max(s, ChooseF32Slices(rows, num_heads, kv_rank, max_live, SIZE_MAX).slices);
+    if (s > 1) most = std::max(most, s * F32Record(std::min(2 * rows, num_tokens), num_heads, kv_rank));
     if (rows == num_tokens) break;
   }
   return most;
@@ -990,7 +991,9 @@ extern "C" int tlaloc_b200_latent_attention(const void* query, const void* pool,
   if (dtype == TLALOC_B200_F32 && !OrderFaithful() && F32Applies(p)) {
     cudaError_t e = PrepareLatentAttention();
     if (e != cudaSuccess) return CudaFail("LATENT_ATTENTION set-up", e);
-    const F32Slices sp = ChooseF32Slices(p, MaxLive(max_live, window, static_cast<int64_t>(max_blocks) * block_size), scratch, scratch_bytes);
+    F32Slices sp = ChooseF32Slices(num_tokens, num_heads, kv_rank, MaxLive(max_live, window, static_cast<int64_t>(max_blocks) * block_size),
+                                   scratch != nullptr && Aligned16(scratch) ? scratch_bytes : 0);
+    sp.records = sp.slices > 1 ? static_cast<float*>(scratch) : nullptr;
     const dim3 grid(sp.slices, (num_heads + kF32Heads - 1) / kF32Heads, num_tokens);
     e = kv_rank <= 256 && p.row <= 384 ? LaunchChained(LatentAttentionF32<3, 2>, grid, kF32Threads, F32Smem(3), st, p, sp)
                                        : LaunchChained(LatentAttentionF32<5, 4>, grid, kF32Threads, F32Smem(5), st, p, sp);
