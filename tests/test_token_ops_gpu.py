@@ -15,6 +15,13 @@ def ops():
     return o
 
 
+@pytest.mark.parametrize("offset", [0, 1])
+def test_embedding_rows_longer_than_a_grid(offset):
+    dim = 65535 * 512 + 516
+    table = torch.arange(2 * dim + offset, dtype=torch.int32, device=DEV).float()[offset:].view(2, dim)
+    assert torch.equal(ops().embedding(table, torch.tensor([1], dtype=torch.int32, device=DEV)), table[1:])
+
+
 # one CTA a row up to 8191 columns, then clusters of 2, 4 and 8; multiples of four take 16-byte loads
 @pytest.mark.parametrize("n", [1, 3, 4, 2047, 8191, 8192, 8195, 16384, 32767, 32768, 40004, 128256])
 @pytest.mark.parametrize("rows", [1, 7])

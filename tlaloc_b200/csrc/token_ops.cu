@@ -2,6 +2,8 @@
 // model of the framework begins and ends a step with.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace tlaloc_b200 {
@@ -10,28 +12,29 @@ namespace {
 namespace cg = cooperative_groups;
 constexpr int kEmbedThreads = 128, kArgmaxThreads = 512, kArgmaxCluster = 8;
 
-// A row of the table widened to f32, sixteen bytes of it per thread: blockIdx.y counts stretches of the row.  A single CTA walking a row
+// A row of the table widened to f32, sixteen bytes of it per thread: blockIdx.y counts stretches of the row (as many as a grid has, then again).  A single CTA walking a row
 // element by element was a chain of dim / 256 dependent trips (128 rows of 8192: 16.7 us; this form 3.8 us, 5.2 MB of traffic).
 template <typename TT, bool VEC>
 __global__ void __launch_bounds__(kEmbedThreads) EmbeddingKernel(const TT* table, const int* ids, float* out, int vocab, int dim)
 {
   constexpr int kPer = 16 / static_cast<int>(sizeof(TT));
   GridDependencySync();
-  const int p = blockIdx.x, d0 = (blockIdx.y * kEmbedThreads + threadIdx.x) * kPer;
-  if (d0 >= dim) return;
+  const int p = blockIdx.x;
   int v = __ldg(ids + p);
   v = v < 0 ? 0 : (v >= vocab ? vocab - 1 : v);
-  const TT* src = table + static_cast<size_t>(v) * dim + d0;
-  float* dst = out + static_cast<size_t>(p) * dim + d0;
-  if (VEC) {
-    const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(src));  // L2: an f32 table may be rows that the kernel before has written
-    const TT* e = reinterpret_cast<const TT*>(&raw);
+  for (long long d0 = (static_cast<long long>(blockIdx.y) * kEmbedThreads + threadIdx.x) * kPer; d0 < dim; d0 += gridDim.y * kEmbedThreads * kPer) {
+    const TT* src = table + static_cast<size_t>(v) * dim + d0;
+    float* dst = out + static_cast<size_t>(p) * dim + d0;
+    if (VEC) {
+      const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(src));  // L2: an f32 table may be rows that the kernel before has written
+      const TT* e = reinterpret_cast<const TT*>(&raw);
 #pragma unroll
-    for (int i = 0; i < kPer; i += 4) {
-      *reinterpret_cast<float4*>(dst + i) = make_float4(ToF32(e[i]), ToF32(e[i + 1]), ToF32(e[i + 2]), ToF32(e[i + 3]));
+      for (int i = 0; i < kPer; i += 4) {
+        *reinterpret_cast<float4*>(dst + i) = make_float4(ToF32(e[i]), ToF32(e[i + 1]), ToF32(e[i + 2]), ToF32(e[i + 3]));
+      }
+    } else {
+      for (int i = 0; i < kPer && d0 + i < dim; ++i) dst[i] = ToF32(src[i]);
     }
-  } else {
-    for (int i = 0; i < kPer && d0 + i < dim; ++i) dst[i] = ToF32(src[i]);
   }
 }
 
@@ -140,7 +143,7 @@ template <typename TT>
 cudaError_t LaunchEmbedding(const void* table, const int32_t* ids, float* out, int positions, int vocab, int dim, cudaStream_t st)
 {
   constexpr int kPer = 16 / static_cast<int>(sizeof(TT));
-  const dim3 grid(positions, (dim + kEmbedThreads * kPer - 1) / (kEmbedThreads * kPer));
+  const dim3 grid(positions, std::min(65535, (dim - 1) / (kEmbedThreads * kPer) + 1));
   const TT* t = static_cast<const TT*>(table);
   return dim % kPer == 0 && Aligned16(table) && Aligned16(out) ? LaunchChained(EmbeddingKernel<TT, true>, grid, kEmbedThreads, 0, st, t, ids, out, vocab, dim)
                                                              : LaunchChained(EmbeddingKernel<TT, false>, grid, kEmbedThreads, 0, st, t, ids, out, vocab, dim);
