@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // ---- host -----------------------------------------------------------------------------------------------------------
 
-int g_slots[kMaxDevices][9];  // resident CTAs when launched as clusters of ks
+int g_slots[kMaxDevices][9];  // resident CTAs when launched as clusters of ks: measured for one layout, every one of which fills an SM's shared memory
 
 cudaError_t PrepareDenseF32()
 {
