@@ -1,0 +1,27 @@
+"""The row-vector int8 projection over every number of slices of k: one to eight CTAs of a cluster share a column tile, some of them without rows of their own."""
+import numpy as np
+import pytest
+import torch
+
+from tlaloc_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+# (k, n): shapes whose tiles of 128 columns fill the SMs with 1, 2, 3, 4, 5, 6, 7 and 8 slices; ragged ends of k and n
+SHAPES = [(128, 28672), (264, 37888), (512, 28656), (520, 14208), (640, 14336), (776, 9472), (904, 8064), (1032, 7088), (16, 16), (2048, 144)]
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 16])
+@pytest.mark.parametrize("k,n", SHAPES)
+def test_every_slice_count(k, n, rows):
+    """Whole activations: every sum stays below 2^24 (2048 x 8 x 128 = 2^21), so f32 sums in any order are exact."""
+    rng = np.random.default_rng(k + n + rows)
+    x = rng.integers(-8, 9, size=(rows, k)).astype(np.float32)
+    codes = rng.integers(-128, 128, size=(k, n), dtype=np.int8)
+    residual = rng.integers(-100, 101, size=(rows, n)).astype(np.float32)
+    scales = (0.25 * 2.0 ** rng.integers(0, 3, size=n)).astype(np.float32)
+    t = lambda a: torch.from_numpy(a).cuda()
+    want = torch.from_numpy((x.astype(np.float64) @ codes.astype(np.float64)) * scales + residual).float()
+    for const in (False, True):
+        got = ops.int8_gemm(t(x).bfloat16(), t(codes), t(scales), residual=t(residual), weights_const=const)
+        assert torch.equal(got.cpu(), want)

@@ -15,6 +15,9 @@
 //                    summed through distributed shared memory in rank order: no global scratch, no second kernel,
 //                    and a result that does not depend on timing.  The per-column scale (and an optional residual)
 //                    is applied to the finished sum, as the graph multiplies after the dot.
+//                    Bound at one row by the issue of the conversion (ncu, 4096 x 28672: ALU pipe 57 %, issue slots 50 % busy, 3.3 warps a scheduler)
+//                    and by the SMs that idle at its ends (22 % of the time).  4096 x 28672 with a norm in front: 34.3 us with two slices and a division
+//                    per stage for the ring's place, 31.0 with three slices, 30.1 with places and sources that move on by themselves.
 //   GemmExactKernel  the interpreter's MATMUL order (DxirInterpreter.kt:739-765): f32, k ascending, separate
 //                    multiply and add, zero activations skipped.  Bit-identical to the CPU oracle; slow.
 #include <cooperative_groups.h>
@@ -137,63 +140,57 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
   const uint32_t xdst = kGvWBytes + xm * (kGvStageK * 2) + ((xpiece ^ ((xm >> 1) & 3)) << 4);
   const __nv_bfloat16* x_lane = p.x + static_cast<size_t>(xm) * p.K + kb + warp * kGvStageK + xpiece * 8;
 
-  // A stage's copies in two parts: the weights, which with weights_const depend on no earlier kernel, and the activations.
-  auto issue_w = [&](int it) {
-    const int k0 = kb + (warp + kGvWarps * it) * kGvStageK;
-    const uint32_t dst = my_pipe_addr + (it % kGvStages) * L::kStageBytes;
-    const int8_t* src = w_lane + it * w_stage;
-    if (k0 + kGvStageK <= ke) {  // the whole stage is inside K
+  // A stage's copies in two parts: the weights, which with weights_const depend on no earlier kernel, and the activations.  Both go through the
+  // slice from front to back; the ring's place and the sources move on by themselves, without a division or a product per stage.
+  int w_k0 = kb + warp * kGvStageK, x_k0 = w_k0;
+  uint32_t w_place = my_pipe_addr, x_place = my_pipe_addr;
+  const uint32_t ring_end = my_pipe_addr + L::kWarpBytes;
+  auto issue_w = [&]() {
+    if (w_k0 + kGvStageK <= ke) {  // the whole stage is inside K
       const int bytes = col_ok ? 16 : 0;
 #pragma unroll
       for (int i = 0; i < 8; i += 2) {
-        CpAsync16(dst + wdst_even + i * (4 * kGvCols), src + i * w_row4, bytes);
-        CpAsync16(dst + wdst_odd + i * (4 * kGvCols), src + (i + 1) * w_row4, bytes);
+        CpAsync16(w_place + wdst_even + i * (4 * kGvCols), w_lane + i * w_row4, bytes);
+        CpAsync16(w_place + wdst_odd + i * (4 * kGvCols), w_lane + (i + 1) * w_row4, bytes);
       }
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const bool valid = col_ok && k0 + l3 + 4 * i < ke;
-        CpAsync16(dst + ((i & 1) ? wdst_odd - 4 * kGvCols : wdst_even) + i * (4 * kGvCols), valid ? src + i * w_row4 : p.w, valid ? 16 : 0);
+        const bool valid = col_ok && w_k0 + l3 + 4 * i < ke;
+        CpAsync16(w_place + ((i & 1) ? wdst_odd - 4 * kGvCols : wdst_even) + i * (4 * kGvCols), valid ? w_lane + i * w_row4 : p.w, valid ? 16 : 0);
       }
     }
+    w_k0 += kGvWarps * kGvStageK;
+    w_lane += w_stage;
+    w_place = w_place + L::kStageBytes == ring_end ? my_pipe_addr : w_place + L::kStageBytes;
   };
-  auto issue_x = [&](int it) {
-    const int k0 = kb + (warp + kGvWarps * it) * kGvStageK;
-    const uint32_t dst = my_pipe_addr + (it % kGvStages) * L::kStageBytes;
-    if (k0 + kGvStageK <= ke) {
+  auto issue_x = [&]() {
 #pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const bool valid = xm + 8 * i < p.M;
-        CpAsync16(dst + xdst + i * (8 * kGvStageK * 2), x_lane + (valid ? static_cast<size_t>(8 * i) * p.K + it * (kGvWarps * kGvStageK) : 0),
-                  valid ? 16 : 0);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const bool valid = xm + 8 * i < p.M && k0 + xpiece * 8 < ke;
-        CpAsync16(dst + xdst + i * (8 * kGvStageK * 2),
-                  valid ? x_lane + static_cast<size_t>(8 * i) * p.K + it * (kGvWarps * kGvStageK) : p.x, valid ? 16 : 0);
-      }
+    for (int i = 0; i < NT; ++i) {
+      const bool valid = xm + 8 * i < p.M && x_k0 + xpiece * 8 < ke;
+      CpAsync16(x_place + xdst + i * (8 * kGvStageK * 2), valid ? x_lane + static_cast<size_t>(8 * i) * p.K : p.x, valid ? 16 : 0);
     }
-  };
-  auto issue = [&](int it) {
-    issue_w(it);
-    issue_x(it);
+    x_k0 += kGvWarps * kGvStageK;
+    x_lane += kGvWarps * kGvStageK;
+    x_place = x_place + L::kStageBytes == ring_end ? my_pipe_addr : x_place + L::kStageBytes;
   };
 
   if (p.weights_const) {
     // The weights of the first stages are on their way while the previous kernel drains; the first commit group then
     // holds all of them together with the first stage's activations.
     for (int it = 0; it < kGvStages - 1; ++it)
-      if (it < my_n) issue_w(it);
+      if (it < my_n) issue_w();
     GridDependencySync();
     for (int it = 0; it < kGvStages - 1; ++it) {
-      if (it < my_n) issue_x(it);
+      if (it < my_n) issue_x();
       CpAsyncCommit();
     }
   } else {
     for (int it = 0; it < kGvStages - 1; ++it) {
-      if (it < my_n) issue(it);
+      if (it < my_n) {
+        issue_w();
+        issue_x();
+      }
       CpAsyncCommit();
     }
   }
@@ -212,12 +209,15 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
   const uint32_t xread0 = kGvWBytes + xr * (kGvStageK * 2) + ((xp0 ^ xsw) << 4);
   const uint32_t xread1 = kGvWBytes + xr * (kGvStageK * 2) + (((xp0 + 2) ^ xsw) << 4);
 
+  uint32_t st_addr = my_pipe_addr;
   for (int it = 0; it < my_n; ++it) {
-    if (it + kGvStages - 1 < my_n) issue(it + kGvStages - 1);
+    if (it + kGvStages - 1 < my_n) {
+      issue_w();
+      issue_x();
+    }
     CpAsyncCommit();
     CpAsyncWait<kGvStages - 1>();
     __syncwarp();
-    const uint32_t st_addr = my_pipe_addr + (it % kGvStages) * L::kStageBytes;
 #pragma unroll
     for (int h = 0; h < kGvStageK / 16; ++h) {
       // x^T as B fragments: b0b1 = x[row gid][16h + 2tig, +1], b2b3 = x[row gid][16h + 8 + 2tig, +1].
@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
       }
     }
     __syncwarp();  // the stage is free for the copy the next iteration issues
+    st_addr = st_addr + L::kStageBytes == ring_end ? my_pipe_addr : st_addr + L::kStageBytes;
   }
   CpAsyncWait<0>();
   __syncthreads();  // every warp is done with the pipeline space
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
     }
   }
   __syncthreads();
-  for (int e = tid; e < L::kRows * kGvCols; e += kGvThreads) {
+  for (int e = tid; e < p.M * kGvCols; e += kGvThreads) {
     const int m = e / kGvCols, c = e - m * kGvCols;
     float v = 0.f;
 #pragma unroll
@@ -281,14 +282,15 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
   // The K slices of this column tile are the ranks of one cluster: rank r finishes every ks-th row.
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank(), nranks = cluster.num_blocks();
+  const int col = col0 + tid;
+  const float scale = p.scales != nullptr && col < p.N ? __ldg(p.scales + col) : 1.f;  // on its way while the ranks meet
   cluster.sync();
   YT* y = static_cast<YT*>(p.y);
   for (int m = rank; m < p.M; m += nranks) {
-    const int col = col0 + tid;
     if (col < p.N) {
       float v = 0.f;
       for (unsigned q = 0; q < nranks; ++q) v += cluster.map_shared_rank(tile, q)[m * kGvRedStride + tid];
-      if (p.scales != nullptr) v *= __ldg(p.scales + col);
+      if (p.scales != nullptr) v *= scale;
       if (p.residual != nullptr) v += __ldg(p.residual + static_cast<size_t>(m) * p.N + col);
       y[static_cast<size_t>(m) * p.N + col] = FromF32<YT>(v);
     }
@@ -404,8 +406,10 @@ cudaError_t LaunchGemv(const GemmParams& p, cudaStream_t stream)
   return cudaLaunchKernelEx(&cfg, Int8GemvKernel<NT, YT>, p);
 }
 
-// K slices for a shape (1, 2, 4 or 8: the portable cluster sizes): the count that wastes the least of the last
-// wave of CTAs over the 148 SMs (four CTAs each), among those that leave every warp at least four stages.
+// K slices for a shape, one to eight (the portable cluster sizes), each of at least one stage a warp.  What counts is how evenly the CTAs fall on the 148 SMs
+// and that there are about three an SM, so that loads in flight cover the way to HBM; more slices than that have to be worth a seventh.  Columns that are cut
+// evenly over all SMs instead (112 or 96 a CTA) lose more to rows of codes that start within a 128-byte line than the last wave costs.
+// Microseconds at one row with a norm in front, slices 2 / 3 / 4 of 4096 x 28672: 30.8 / 28.3 / 29.7; 4 / 5 / 6 of 5120 x 14336: 21.1 / 19.4 / 21.1.
 // $TLALOC_B200_GEMV_KS overrides.
 int ChooseSlices(int k, int n)
 {
@@ -413,18 +417,17 @@ int ChooseSlices(int k, int n)
     const char* e = std::getenv("TLALOC_B200_GEMV_KS");
     return e != nullptr ? std::atoi(e) : 0;
   }();
-  if (forced == 1 || forced == 2 || forced == 4 || forced == 8) return forced;
+  if (forced >= 1 && forced <= 8) return forced;
+  constexpr int kSms = 148, kWanted = 3 * kSms;
   const int tiles = (n + kGvCols - 1) / kGvCols;
-  const int slots = 148 * 4;
   int best = 1;
-  double best_eff = -1.0;
-  for (int ks = 1; ks <= 8; ks *= 2) {
-    if (ks > 1 && k / ks < kGvStageK * kGvWarps * 4) break;
-    const int items = tiles * ks;
-    const int waves = (items + slots - 1) / slots;
-    const double eff = static_cast<double>(items) / (static_cast<double>(waves) * slots);
-    if (eff > best_eff + 0.02) {
-      best_eff = eff;
+  double best_score = 0.0;
+  for (int ks = 1; ks <= 8; ++ks) {
+    if (ks > 1 && k / ks < kGvStageK * kGvWarps) break;
+    const int items = tiles * ks, share = (items + kSms - 1) / kSms;
+    const double score = static_cast<double>(items) / (share * kSms) * std::min(1.0, static_cast<double>(items) / kWanted);
+    if (score > best_score * 1.15) {
+      best_score = score;
       best = ks;
     }
   }
