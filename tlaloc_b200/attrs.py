@@ -7,6 +7,7 @@ refusing by name what the reference refuses.  Operates on anything with ``.shape
 """
 from __future__ import annotations
 
+import functools
 import math
 from dataclasses import dataclass
 
@@ -49,6 +50,7 @@ class PagedAttentionShape:
         return self.max_blocks_per_seq * self.block_size
 
 
+@functools.lru_cache(maxsize=64)
 def _is_integral(dtype) -> bool:
     return str(dtype).replace("torch.", "") in ("int32", "int64")
 
@@ -56,7 +58,7 @@ def _is_integral(dtype) -> bool:
 def parse_paged_attention(query, key_cache, value_cache, block_tables, seq_lens, *, scale, sliding_window=None,
                           keep=None, return_lse=False, layer="tlaloc_b200", **other_attrs) -> PagedAttentionShape:
     """Validate the operands and attrs of one PAGED_ATTENTION and return the derived shape story."""
-    q, k, v, t, l = (tuple(x.shape) for x in (query, key_cache, value_cache, block_tables, seq_lens))
+    q, k, v, t, l = tuple(query.shape), tuple(key_cache.shape), tuple(value_cache.shape), tuple(block_tables.shape), tuple(seq_lens.shape)
     if len(q) != 3:
         raise ValueError(f"{layer}: PAGED_ATTENTION query must be rank-3 [numSeqs, numHeads, headDim], got {list(q)}")
     if len(k) != 4:
@@ -117,5 +119,9 @@ def parse_paged_attention(query, key_cache, value_cache, block_tables, seq_lens,
         if kt[1] < 1 or ctx % kt[1] != 0:
             raise ValueError(f"{layer}: PAGED_ATTENTION keep has {kt[1]} chunks, which do not divide the {ctx} positions")
         keep_chunk = ctx // kt[1]
-    return PagedAttentionShape(num_seqs, num_heads, head_dim, num_blocks, block_size, num_kv_heads, max_blocks,
-                               float(scale), window, num_tables, keep_chunk, bool(return_lse))
+    # every field is checked by now; the frozen class's own constructor sets them one by one, 3 us of a 25 us call
+    out = object.__new__(PagedAttentionShape)
+    out.__dict__.update(num_seqs=num_seqs, num_heads=num_heads, head_dim=head_dim, num_blocks=num_blocks, block_size=block_size,
+                        num_kv_heads=num_kv_heads, max_blocks_per_seq=max_blocks, scale=float(scale), sliding_window=window,
+                        num_tables=num_tables, keep_chunk=keep_chunk, return_lse=bool(return_lse))
+    return out

@@ -344,7 +344,13 @@ class MixedDecoder(RaggedModel):
 
     @staticmethod
     def _view(flat: torch.Tensor, *shape) -> torch.Tensor:
-        return flat[:math.prod(shape)].view(*shape)
+        strides, n = [1] * len(shape), 1
+        for i in range(len(shape) - 1, -1, -1):
+            strides[i] = n
+            n *= shape[i]
+        if n > flat.numel():
+            raise ValueError(f"a view of {shape} on {flat.numel()} values")
+        return flat.as_strided(shape, strides)  # one call of torch's for two
 
     def _attention(self, i: int, n: int, spans, proj: torch.Tensor, out: torch.Tensor) -> None:
         m, lw, pool, (cos, sin) = self.cfg.layers[i].mixer, self.layers[i], self.pools[i], self._rot[i]

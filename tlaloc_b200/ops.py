@@ -13,6 +13,7 @@ import torch
 from . import _native as N
 from .attrs import PagedAttentionShape, parse_paged_attention
 
+_current_raw_stream = torch._C._cuda_getCurrentRawStream
 _DT = {torch.float32: N.F32, torch.bfloat16: N.BF16, torch.int8: N.S8, torch.int32: N.S32, torch.float8_e4m3fn: N.F8E4M3FN}
 
 
@@ -36,7 +37,7 @@ def _out(name: str, t, shape, dtypes, like: torch.Tensor) -> None:
         return
     if not isinstance(dtypes, (tuple, list)):
         dtypes = (dtypes,)
-    if (not t.is_cuda or not t.is_contiguous() or t.device != like.device or t.dtype not in dtypes
+    if (not t.is_cuda or not t.is_contiguous() or t.get_device() != like.get_device() or t.dtype not in dtypes
             or (shape is not None and tuple(t.shape) != tuple(shape))):
         want = "x".join(str(d) for d in shape) if shape is not None else "any shape"
         raise ValueError(f"{name} must be a contiguous {'/'.join(str(d) for d in dtypes)} tensor [{want}] on {like.device}, "
@@ -48,8 +49,9 @@ def _ptr(t):
 
 
 def _stream(t: torch.Tensor) -> int:
-    """The current stream of the tensor's own device (not of whichever device happens to be current)."""
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The current stream of the tensor's own device (not of whichever device happens to be current).  The handle alone: making a Stream
+    object of it takes 4 us, more than a launch."""
+    return _current_raw_stream(t.get_device())
 
 
 def init() -> None:
@@ -79,14 +81,17 @@ def paged_attention(query, key_cache, value_cache, block_tables, seq_lens, *, sc
     _dev(query, key_cache, value_cache, block_tables, seq_lens, keep)
     if block_tables.dtype != torch.int32 or seq_lens.dtype != torch.int32 or (keep is not None and keep.dtype != torch.int32):
         raise TypeError("PAGED_ATTENTION: the kernels read blockTables, seqLens and keep as int32")
-    if out is None:
+    given = out is not None
+    if not given:
         out = torch.empty_like(query)
+    if given or out.dtype not in (torch.float32, torch.bfloat16):
+        _out("PAGED_ATTENTION out", out, (p.num_seqs, p.num_heads, p.head_dim), (torch.float32, torch.bfloat16), query)
     if scratch is None:
         scratch = paged_attention_scratch(p, query.device)
-    _out("PAGED_ATTENTION out", out, (p.num_seqs, p.num_heads, p.head_dim), (torch.float32, torch.bfloat16), query)
-    if scratch.dim() != 4 or scratch.shape[0] < 1:
-        raise ValueError("PAGED_ATTENTION scratch must be f32 [S, R, H, D + 2] with S >= 1")
-    _out("PAGED_ATTENTION scratch", scratch, (scratch.shape[0], p.num_seqs, p.num_heads, p.head_dim + 2), torch.float32, query)
+    else:
+        if scratch.dim() != 4 or scratch.shape[0] < 1:
+            raise ValueError("PAGED_ATTENTION scratch must be f32 [S, R, H, D + 2] with S >= 1")
+        _out("PAGED_ATTENTION scratch", scratch, (scratch.shape[0], p.num_seqs, p.num_heads, p.head_dim + 2), torch.float32, query)
     lse = torch.empty((p.num_seqs, p.num_heads), dtype=torch.float32, device=query.device) if return_lse else None
     N.check(N.lib().tlaloc_b200_paged_attention(
         _ptr(query), _dt(query), _ptr(key_cache), _ptr(value_cache), _dt(key_cache), _ptr(block_tables),
@@ -267,22 +272,23 @@ def dense(x, w, out, *, bias=None, residual=None, act=N.ACT_NONE) -> N.DenseProb
     """One projection out = act(x @ w.T + bias) + residual for `dense_gemm`.  x [M, K], w [N, K], out [M, N]; or a batch
     of them (the heads of a layer): x [B, M, K], w [B, N, K], out [B, M, N].  x, out and residual may be strided views whose
     last dimension is dense; w is contiguous.  A gated act (see interleave_gate) leaves out [M, N / 2]."""
-    batched = w.dim() == 3
-    for name, t in (("x", x), ("out", out)) + ((("residual", residual),) if residual is not None else ()):
-        if not t.is_cuda or t.stride(-1) != 1 or t.dim() != w.dim():
-            raise ValueError(f"DENSE_PROJ {name}: a CUDA tensor of rank {w.dim()} with a dense last dimension is needed")
+    ws, xs, os = w.shape, x.shape, out.shape
+    rank = len(ws)
+    batched = rank == 3
+    b, n, k = ws if batched else (1, *ws)
+    m, x_ld, out_ld = xs[-2], x.stride(), out.stride()
+    for name, t, ld in (("x", x, x_ld), ("out", out, out_ld)) + ((("residual", residual, residual.stride()),) if residual is not None else ()):
+        if not t.is_cuda or ld[-1] != 1 or len(ld) != rank:
+            raise ValueError(f"DENSE_PROJ {name}: a CUDA tensor of rank {rank} with a dense last dimension is needed")
     _dev(w, bias)
-    b, n, k = w.shape if batched else (1, *w.shape)
-    m = x.shape[-2]
-    if x.shape[-1] != k or tuple(out.shape[-2:]) != (m, n // 2 if act in GATED else n) or (batched and (x.shape[0] != b or out.shape[0] != b)) or x.dtype != w.dtype:
+    if xs[-1] != k or os[-2] != m or os[-1] != (n // 2 if act in GATED else n) or (batched and (xs[0] != b or os[0] != b)) or x.dtype != w.dtype:
         raise ValueError(f"DENSE_PROJ: x {tuple(x.shape)} {x.dtype}, w {tuple(w.shape)} {w.dtype}, out {tuple(out.shape)} do not fit")
     if (bias is not None and (bias.dtype != torch.float32 or tuple(bias.shape) != (n,))) or (
             residual is not None and (residual.dtype != torch.float32 or tuple(residual.shape) != (m, n))):
         raise ValueError(f"DENSE_PROJ: bias is f32 [{n}], residual f32 [{m}, {n}]")
-    p = N.DenseProblem(x=_ptr(x), w=_ptr(w), bias=_ptr(bias), residual=_ptr(residual), y=_ptr(out), ld_x=x.stride(-2),
-                       ld_res=residual.stride(-2) if residual is not None else 0, ld_y=out.stride(-2),
-                       batch_x=x.stride(0) if batched else 0, batch_w=n * k, batch_y=out.stride(0) if batched else 0,
-                       k=k, n=n, batch=b, act=act, y_dtype=_dt(out))
+    # in the order of the structure's fields: keywords take as long as everything else here
+    p = N.DenseProblem(x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), x_ld[-2], residual.stride(-2) if residual is not None else 0,
+                       out_ld[-2], x_ld[0] if batched else 0, n * k, out_ld[0] if batched else 0, k, n, b, act, _dt(out))
     p.rows, p.like = m, x
     return p
 
@@ -299,8 +305,8 @@ def grouped_dense(x, w, out, row_offsets, *, act=N.ACT_NONE) -> N.DenseProblem:
     if (x.shape[1] != k or tuple(out.shape) != (m, n // 2 if act in GATED else n) or x.dtype != w.dtype or row_offsets.dtype != torch.int32
             or row_offsets.shape[0] != b + 1):
         raise ValueError(f"GROUPED_PROJ: x {tuple(x.shape)} {x.dtype}, w {tuple(w.shape)} {w.dtype}, out {tuple(out.shape)} do not fit")
-    p = N.DenseProblem(x=_ptr(x), w=_ptr(w), y=_ptr(out), ld_x=x.stride(0), ld_y=out.stride(0), batch_w=n * k, k=k, n=n, batch=b, act=act,
-                       y_dtype=_dt(out), row_offsets=_ptr(row_offsets))
+    p = N.DenseProblem(x.data_ptr(), w.data_ptr(), None, None, out.data_ptr(), x.stride(0), 0, out.stride(0), 0, n * k, 0, k, n, b, act, _dt(out), 0,
+                       row_offsets.data_ptr())
     p.rows, p.like = m, x
     return p
 
@@ -320,10 +326,13 @@ def interleave_gate(gate, up):
 def dense_gemm(*problems, weights_const=False) -> None:
     """Runs one or two `dense` problems of the same type (a `grouped_dense` one last)."""
     like, m = problems[0].like, problems[0].rows
-    if any(p.like.dtype != like.dtype for p in problems):
-        raise ValueError("DENSE_PROJ: the problems of one call have the same type")
-    N.check(N.lib().tlaloc_b200_dense_gemm((N.DenseProblem * len(problems))(*problems), len(problems), _dt(like), m,
-                                           N.GEMM_WEIGHTS_CONST if weights_const else 0, _stream(like)))
+    if len(problems) == 1:
+        packed = ctypes.byref(problems[0])
+    else:
+        if any(p.like.dtype != like.dtype for p in problems):
+            raise ValueError("DENSE_PROJ: the problems of one call have the same type")
+        packed = (N.DenseProblem * len(problems))(*problems)
+    N.check(N.lib().tlaloc_b200_dense_gemm(packed, len(problems), _dt(like), m, N.GEMM_WEIGHTS_CONST if weights_const else 0, _stream(like)))
 
 
 def rmsnorm_pair(x, gain_a, out_a, eps, gain_b=None, out_b=None) -> None:
