@@ -1,13 +1,18 @@
 // Retention: linear attention with a fixed decay per head (include/tlaloc_b200.h).  The state is f32 throughout.
-//   RetentionStepKernel   one token per row, fused: rotation, state update, output, its norm and gate.  A CTA has one head of one
-//                         row and streams its state through registers once: the kernel is bound by those bytes.
+//   RetentionStepKernel   one token per row, fused: rotation, state update, output, its norm and gate.  A cluster has one head of one
+//                         row, a CTA some of its value columns, whose state it streams through registers once: the kernel is bound by those
+//                         bytes where there are CTAs enough to keep them coming.
 //   RetentionScanKernel   a portion token by token with the state in registers, 32 value columns a CTA: any size and type.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tlaloc_b200 {
 namespace {
 
-constexpr int kThreads = 256, kAhead = 8;
+constexpr int kThreads = 256, kAhead = 8, kMostRanks = 8, kWantedCtas = 148 * 3 / 2;
 
 __device__ __forceinline__ float WarpSum(float v)
 {
@@ -16,23 +21,40 @@ __device__ __forceinline__ float WarpSum(float v)
   return v;
 }
 
-// Thread (r, c): state rows r, r + R, ... and the four columns from 4 c.
-template <typename T>
+// Thread (r, c): state rows r, r + R, ... and the four columns from 4 c of the CTA's.  The ranks of a cluster share the columns of a head
+// (whole fours) and meet only for the sum of squares of its norm.  DEEP: the
+// next kAhead rows of a thread are loaded under these; with 96 registers a CTA finds two places on an SM instead of three.
+template <typename T, bool DEEP>
 __global__ void __launch_bounds__(kThreads) RetentionStepKernel(const float* in, int64_t ld, const int* positions, const float* cos_t, const float* sin_t,
                                                                 const float* decay, const int* row_states, float* state, T* out, int64_t out_ld, int heads,
                                                                 int dim, int vdim, int rot_dims, int num_slots, int max_pos, float k_scale, float eps)
 {
   GridDependencySync();
   extern __shared__ float smem[];
-  __shared__ float red[8];
-  const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x;
-  const int vp = (vdim + 3) & ~3, cols = vp >> 2, R = min(kThreads / cols, dim), c = tid % cols, r = tid / cols;
+  __shared__ float red[8], s_ranks[kMostRanks];
+  const int h = blockIdx.x, rank = blockIdx.y, ranks = gridDim.y, t = blockIdx.z, tid = threadIdx.x;
+  const int vp = (vdim + 3) & ~3, share = ((vp >> 2) + ranks - 1) / ranks, c0 = 4 * rank * share;  // this CTA's columns: [c0, c0 + wide), live ones [c0, c0 + mine)
+  const int cols = min(share, (vp >> 2) - rank * share), wide = 4 * cols, mine = min(wide, vdim - c0);
+  const int R = min(kThreads / cols, dim), c = tid % cols, r = tid / cols;
   const int dp = (dim + 3) & ~3;
-  float *qs = smem, *ks = smem + dp, *part = smem + 2 * dp;  // part [R][vp], 16-byte aligned
+  float *qs = smem, *ks = smem + dp, *part = smem + 2 * dp;  // part [R][wide], 16-byte aligned
   const float* row = in + t * ld;
-  const float *q = row + h * dim, *k = row + (heads + h) * dim, *v = row + 2 * heads * dim + h * vdim, *g = v + heads * vdim;
+  const float *q = row + h * dim, *k = row + (heads + h) * dim, *v = row + 2 * heads * dim + h * vdim + c0, *g = v + heads * vdim;
   const int pos = min(max(__ldg(positions + t), 0), max_pos - 1), half = rot_dims >> 1;
-  const bool fresh = pos == 0;
+  const bool fresh = pos == 0, live = r < R;
+  const int slot = min(max(__ldg(row_states + t), 0), num_slots - 1);
+  float* s = state + (static_cast<size_t>(slot) * heads + h) * dim * vp + c0 + 4 * c;
+  // The state's first rows are on their way while the query and the key are rotated.
+  auto load = [&](float4 (&x)[kAhead], int i0) {
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e) {
+      const int i = i0 + e * R;
+      x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live && i < dim && !fresh) x[e] = *reinterpret_cast<const float4*>(s + static_cast<size_t>(i) * vp);
+    }
+  };
+  float4 x[kAhead];
+  load(x, r);
   for (int i = tid; i < dim; i += kThreads) {
     float a = q[i], b = k[i];
     if (i < rot_dims) {
@@ -46,38 +68,33 @@ __global__ void __launch_bounds__(kThreads) RetentionStepKernel(const float* in,
     ks[i] = b * k_scale;
   }
   float4 vv = make_float4(0.f, 0.f, 0.f, 0.f);
-  const bool live = r < R;
   if (live) {
     vv.x = v[4 * c];
-    if (4 * c + 1 < vdim) vv.y = v[4 * c + 1];
-    if (4 * c + 2 < vdim) vv.z = v[4 * c + 2];
-    if (4 * c + 3 < vdim) vv.w = v[4 * c + 3];
+    if (4 * c + 1 < mine) vv.y = v[4 * c + 1];
+    if (4 * c + 2 < mine) vv.z = v[4 * c + 2];
+    if (4 * c + 3 < mine) vv.w = v[4 * c + 3];
   }
-  const int slot = min(max(__ldg(row_states + t), 0), num_slots - 1);
   const float d = __ldg(decay + h);
-  float* s = state + (static_cast<size_t>(slot) * heads + h) * dim * vp + 4 * c;
   __syncthreads();
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   if (live) {
     for (int i0 = r; i0 < dim; i0 += R * kAhead) {
-      float4 x[kAhead];
+      float4 next[kAhead];
+      if constexpr (DEEP) load(next, i0 + R * kAhead);
+      else if (i0 != r) load(x, i0);
 #pragma unroll
       for (int e = 0; e < kAhead; ++e) {
         const int i = i0 + e * R;
-        x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < dim && !fresh) x[e] = *reinterpret_cast<const float4*>(s + static_cast<size_t>(i) * vp);
-      }
-#pragma unroll
-      for (int e = 0; e < kAhead; ++e) {
-        const int i = i0 + e * R;
-        if (i >= dim) break;
-        const float kk = ks[i], qq = qs[i];
-        x[e] = make_float4(fmaf(d, x[e].x, kk * vv.x), fmaf(d, x[e].y, kk * vv.y), fmaf(d, x[e].z, kk * vv.z), fmaf(d, x[e].w, kk * vv.w));
-        *reinterpret_cast<float4*>(s + static_cast<size_t>(i) * vp) = x[e];
-        o = make_float4(fmaf(qq, x[e].x, o.x), fmaf(qq, x[e].y, o.y), fmaf(qq, x[e].z, o.z), fmaf(qq, x[e].w, o.w));
+        if (i < dim) {
+          const float kk = ks[i], qq = qs[i];
+          x[e] = make_float4(fmaf(d, x[e].x, kk * vv.x), fmaf(d, x[e].y, kk * vv.y), fmaf(d, x[e].z, kk * vv.z), fmaf(d, x[e].w, kk * vv.w));
+          *reinterpret_cast<float4*>(s + static_cast<size_t>(i) * vp) = x[e];
+          o = make_float4(fmaf(qq, x[e].x, o.x), fmaf(qq, x[e].y, o.y), fmaf(qq, x[e].z, o.z), fmaf(qq, x[e].w, o.w));
+        }
+        if constexpr (DEEP) x[e] = next[e];
       }
     }
-    *reinterpret_cast<float4*>(part + r * vp + 4 * c) = o;
+    *reinterpret_cast<float4*>(part + r * wide + 4 * c) = o;
   }
   __syncthreads();
   float sum[4], ss = 0.f;  // vdim <= 1024: up to four columns a thread
@@ -85,8 +102,8 @@ __global__ void __launch_bounds__(kThreads) RetentionStepKernel(const float* in,
   for (int e = 0; e < 4; ++e) {
     const int j = tid + e * kThreads;
     sum[e] = 0.f;
-    if (j < vdim) {
-      for (int i = 0; i < R; ++i) sum[e] += part[i * vp + j];
+    if (j < mine) {
+      for (int i = 0; i < R; ++i) sum[e] += part[i * wide + j];
     }
     ss = fmaf(sum[e], sum[e], ss);
   }
@@ -96,11 +113,19 @@ __global__ void __launch_bounds__(kThreads) RetentionStepKernel(const float* in,
   ss = 0.f;
 #pragma unroll
   for (int w = 0; w < 8; ++w) ss += red[w];
+  if (ranks > 1) {  // every rank's sum to every rank, added in rank order
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();  // all of them run: their shared memory may be written
+    if (tid < ranks) cluster.map_shared_rank(s_ranks, tid)[rank] = ss;
+    cluster.sync();
+    ss = 0.f;
+    for (int i = 0; i < ranks; ++i) ss += s_ranks[i];
+  }
   const float inv = 1.f / sqrtf(ss / static_cast<float>(vdim) + eps);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int j = tid + e * kThreads;
-    if (j < vdim) out[t * out_ld + h * vdim + j] = FromF32<T>(sum[e] * inv * (g[j] / (1.f + expf(-g[j]))));
+    if (j < mine) out[t * out_ld + h * vdim + c0 + j] = FromF32<T>(sum[e] * inv * (g[j] / (1.f + expf(-g[j]))));
   }
 }
 
@@ -203,13 +228,29 @@ extern "C" int tlaloc_b200_retention_step(const float* in, int64_t ld, const int
   if (dim > 512 || vdim > 1024) return Fail(kUnsupported, "%s: dim up to 512, vdim up to 1024", op);
   if (rows == 0) return kOk;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int vp = (vdim + 3) / 4 * 4, lanes = kThreads / (vp / 4);
-  const size_t smem = sizeof(float) * (2 * ((dim + 3) / 4 * 4) + static_cast<size_t>(lanes < dim ? lanes : dim) * vp);
-  const dim3 grid(heads, rows);
+  const int vp = (vdim + 3) / 4 * 4;
+  // Ranks: where heads and rows alone leave SMs idle, as long as each has at least 32 columns (a whole 128-byte line of a state row) and 32 KB of state;
+  // a CTA's beginning and the cluster's meeting cost about as much as that.  Microseconds with one rank and split, head x dim x vdim of rows:
+  // 8 x 256 x 512 of 15 31.0 -> 25.6 (two ranks) and 35 (eight), of 1 21.4 -> 6.6; 16 x 128 x 256 of 1 7.8 -> 5.2; 20 x 64 x 128 of 3 4.1 -> 4.9 (not split).
+  const size_t bytes = sizeof(float) * dim * vp;
+  int ranks = 1;
+  while (ranks < kMostRanks && static_cast<long long>(heads) * rows * ranks < kWantedCtas && vp / (2 * ranks) >= 32 && bytes / (2 * ranks) >= 32 * 1024) ranks *= 2;
+  const int cols = (vp / 4 + ranks - 1) / ranks;
+  const bool deep = dim > kThreads / cols * kAhead && static_cast<long long>(heads) * rows * ranks <= 2 * 148;  // two places an SM are enough
+  const size_t smem = sizeof(float) * (2 * ((dim + 3) / 4 * 4) + 4 * static_cast<size_t>(kThreads));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(heads, ranks, rows);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attrs[2];
+  cfg.numAttrs = ChainAttributes(attrs, ranks);
+  cfg.attrs = attrs;
   cudaError_t e;
 #define TLALOC_LAUNCH(T)                                                                                                                         \
-  e = LaunchChained(RetentionStepKernel<T>, grid, kThreads, smem, st, in, ld, positions, cos_table, sin_table, decay, row_states, state,          \
-                    static_cast<T*>(out), out_ld, heads, dim, vdim, rot_dims, num_slots, max_pos, k_scale, eps)
+  e = cudaLaunchKernelEx(&cfg, deep ? RetentionStepKernel<T, true> : RetentionStepKernel<T, false>, in, ld, positions, cos_table, sin_table, decay, row_states, state, static_cast<T*>(out),   \
+                         out_ld, static_cast<int>(heads), static_cast<int>(dim), static_cast<int>(vdim), static_cast<int>(rot_dims),              \
+                         static_cast<int>(num_slots), static_cast<int>(max_pos), k_scale, eps)
   if (dtype == TLALOC_B200_F32) TLALOC_LAUNCH(float);
   else TLALOC_LAUNCH(__nv_bfloat16);
 #undef TLALOC_LAUNCH
