@@ -85,16 +85,18 @@ template <>
 __device__ __forceinline__ float AsBf16Value<float>(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 // One CTA per row: the row's largest magnitude, the power-of-two step s, then q = x / s (exact: a power of two) rounded
-// to the nearest integer and split as q = 256 hi + lo.
-template <typename XT>
-__global__ void __launch_bounds__(256) QuantizeRowsI8Kernel(const XT* __restrict__ x, int8_t* __restrict__ hi,
-                                                            int8_t* __restrict__ lo, float* __restrict__ row_scale, int K)
+// to the nearest integer and split as q = 256 hi + lo.  A row is bound by latency (128 rows of 28672 are 7 MB of L2 traffic), so up to WORDS
+// 16-byte words a thread are read once, all in flight together, and kept (128 rows of 8192 and of 28672 after one another in a step: 13.6 us by two passes of dependent loads, 6.2 so);
+// WORDS 0: rows that are longer or not whole aligned words, read twice.
+constexpr int kQuantThreads = 512;
+template <typename XT, int WORDS>
+__global__ void __launch_bounds__(kQuantThreads) QuantizeRowsI8Kernel(const XT* x, int8_t* __restrict__ hi, int8_t* __restrict__ lo,
+                                                                      float* __restrict__ row_scale, int K)
 {
   GridDependencySync();
   const int m = blockIdx.x, tid = threadIdx.x;
   const XT* row = x + static_cast<size_t>(m) * K;
   constexpr int kVec = 16 / sizeof(XT);  // elements per 16-byte load
-  const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0 && K % kVec == 0;
   float amax = 0.f;
   bool bad = false;
   auto see = [&](float v) {
@@ -102,18 +104,25 @@ __global__ void __launch_bounds__(256) QuantizeRowsI8Kernel(const XT* __restrict
     bad = bad || !(a <= 3.4e38f);
     amax = fmaxf(amax, a);
   };
-  if (vec) {
-    for (int i = tid * kVec; i < K; i += 256 * kVec) {
-      const uint4 u = *reinterpret_cast<const uint4*>(row + i);
-      const XT* e = reinterpret_cast<const XT*>(&u);
+  uint4 u[WORDS > 0 ? WORDS : 1];
+  if constexpr (WORDS > 0) {
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+      const int i = (tid + w * kQuantThreads) * kVec;
+      u[w] = i < K ? *reinterpret_cast<const uint4*>(row + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+      const XT* e = reinterpret_cast<const XT*>(&u[w]);
 #pragma unroll
       for (int j = 0; j < kVec; ++j) see(AsBf16Value<XT>(e[j]));
     }
   } else {
-    for (int i = tid; i < K; i += 256) see(AsBf16Value<XT>(row[i]));
+    for (int i = tid; i < K; i += kQuantThreads) see(AsBf16Value<XT>(row[i]));
   }
-  __shared__ float s_max[8];
-  __shared__ int s_bad[8];
+  constexpr int kWarps = kQuantThreads / 32;
+  __shared__ float s_max[kWarps];
+  __shared__ int s_bad[kWarps];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   const int any_bad = __any_sync(0xffffffffu, bad);
@@ -125,7 +134,7 @@ __global__ void __launch_bounds__(256) QuantizeRowsI8Kernel(const XT* __restrict
   amax = s_max[0];
   int row_bad = s_bad[0];
 #pragma unroll
-  for (int w = 1; w < 8; ++w) {
+  for (int w = 1; w < kWarps; ++w) {
     amax = fmaxf(amax, s_max[w]);
     row_bad |= s_bad[w];
   }
@@ -134,29 +143,32 @@ __global__ void __launch_bounds__(256) QuantizeRowsI8Kernel(const XT* __restrict
   if (tid == 0) row_scale[m] = step;
   int8_t* hrow = hi + static_cast<size_t>(m) * K;
   int8_t* lrow = lo + static_cast<size_t>(m) * K;
-  auto split = [&](float v, int8_t& h, int8_t& l) {
-    int hq, lq;
-    I8Split(v, inv, hq, lq);
-    h = static_cast<int8_t>(hq);
-    l = static_cast<int8_t>(lq);
-  };
-  if (vec) {
-    for (int i = tid * kVec; i < K; i += 256 * kVec) {
-      const uint4 u = *reinterpret_cast<const uint4*>(row + i);
-      const XT* el = reinterpret_cast<const XT*>(&u);
-      alignas(8) int8_t h[kVec], l[kVec];
+  if constexpr (WORDS > 0) {
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) split(AsBf16Value<XT>(el[j]), h[j], l[j]);
+    for (int w = 0; w < WORDS; ++w) {
+      const int i = (tid + w * kQuantThreads) * kVec;
+      if (i >= K) break;
+      const XT* e = reinterpret_cast<const XT*>(&u[w]);
+      uint32_t h[kVec / 4], l[kVec / 4];
+#pragma unroll
+      for (int j = 0; j < kVec; j += 4) {
+        I8Split4(AsBf16Value<XT>(e[j]), AsBf16Value<XT>(e[j + 1]), AsBf16Value<XT>(e[j + 2]), AsBf16Value<XT>(e[j + 3]), inv, h[j / 4], l[j / 4]);
+      }
       if constexpr (kVec == 8) {
-        *reinterpret_cast<uint2*>(hrow + i) = *reinterpret_cast<const uint2*>(h);
-        *reinterpret_cast<uint2*>(lrow + i) = *reinterpret_cast<const uint2*>(l);
+        *reinterpret_cast<uint2*>(hrow + i) = make_uint2(h[0], h[1]);
+        *reinterpret_cast<uint2*>(lrow + i) = make_uint2(l[0], l[1]);
       } else {
-        *reinterpret_cast<uint32_t*>(hrow + i) = *reinterpret_cast<const uint32_t*>(h);
-        *reinterpret_cast<uint32_t*>(lrow + i) = *reinterpret_cast<const uint32_t*>(l);
+        *reinterpret_cast<uint32_t*>(hrow + i) = h[0];
+        *reinterpret_cast<uint32_t*>(lrow + i) = l[0];
       }
     }
   } else {
-    for (int i = tid; i < K; i += 256) split(AsBf16Value<XT>(row[i]), hrow[i], lrow[i]);
+    for (int i = tid; i < K; i += kQuantThreads) {
+      int hq, lq;
+      I8Split(AsBf16Value<XT>(row[i]), inv, hq, lq);
+      hrow[i] = static_cast<int8_t>(hq);
+      lrow[i] = static_cast<int8_t>(lq);
+    }
   }
 }
 
@@ -567,7 +579,7 @@ cudaError_t LaunchInt8GemmI8(const void* x, int x_dtype, const int8_t* codes, co
   p.ks = ChooseI8Slices(k, n);
   const int nb = (k + kI8BK - 1) / kI8BK;
   p.Kc = (nb + p.ks - 1) / p.ks * kI8BK;
-  p.weights_const = weights_const ? 1 : 0;
+  p.weights_const = weights_const || !have_planes ? 1 : 0;  // the quantizer is past its own dependency wait by now and writes no weights
   p.swiglu = swiglu ? 1 : 0;
   e = y_dtype == TLALOC_B200_F32 ? LaunchI8Rows<float>(mw, mh, ml, p, st) : LaunchI8Rows<__nv_bfloat16>(mw, mh, ml, p, st);
   if (e != cudaSuccess) return e;
@@ -575,15 +587,24 @@ cudaError_t LaunchInt8GemmI8(const void* x, int x_dtype, const int8_t* codes, co
   return cudaSuccess;
 }
 
+template <typename XT>
+cudaError_t LaunchQuantize(const XT* x, int8_t* planes, int m, int k, cudaStream_t st)
+{
+  int8_t *hi = planes, *lo = hi + static_cast<size_t>(m) * k;
+  float* row_scale = reinterpret_cast<float*>(lo + static_cast<size_t>(m) * k);
+  constexpr int kVec = 16 / sizeof(XT);
+  const int words = (k + kQuantThreads * kVec - 1) / (kQuantThreads * kVec);
+  auto kernel = k % kVec != 0 || !Aligned16(x) || words > 8 ? QuantizeRowsI8Kernel<XT, 0>
+                : words <= 2                                ? QuantizeRowsI8Kernel<XT, 2>
+                : words <= 4                                ? QuantizeRowsI8Kernel<XT, 4>
+                                                            : QuantizeRowsI8Kernel<XT, 8>;
+  return LaunchChained(kernel, static_cast<unsigned>(m), kQuantThreads, 0, st, x, hi, lo, row_scale, k);
+}
+
 cudaError_t LaunchQuantizeRowsI8(const void* x, int x_dtype, void* planes, int m, int k, cudaStream_t st)
 {
-  int8_t* hi = static_cast<int8_t*>(planes);
-  int8_t* lo = hi + static_cast<size_t>(m) * k;
-  float* row_scale = reinterpret_cast<float*>(lo + static_cast<size_t>(m) * k);
-  return x_dtype == TLALOC_B200_F32
-             ? LaunchChained(QuantizeRowsI8Kernel<float>, static_cast<unsigned>(m), 256, 0, st, static_cast<const float*>(x), hi, lo, row_scale, k)
-             : LaunchChained(QuantizeRowsI8Kernel<__nv_bfloat16>, static_cast<unsigned>(m), 256, 0, st,
-                             static_cast<const __nv_bfloat16*>(x), hi, lo, row_scale, k);
+  int8_t* p = static_cast<int8_t*>(planes);
+  return x_dtype == TLALOC_B200_F32 ? LaunchQuantize(static_cast<const float*>(x), p, m, k, st) : LaunchQuantize(static_cast<const __nv_bfloat16*>(x), p, m, k, st);
 }
 
 int ReadI8Status()
