@@ -63,8 +63,10 @@ struct Branch {
   int top;
 };
 
-// One CTA per row.  VEC: up to 8192 values, a multiple of 4, 16-byte aligned, kept in registers; else the row is read several times.
-template <typename T, bool VEC>
+// One CTA per row.  NI > 0: up to 1024 NI values, a multiple of 4, 16-byte aligned, kept in registers, NI words a thread; 0: any row, read several times.
+// The kernel is bound by the loads in flight, so a thread asks for no registers its row does not need: 2048 rows of 2560 values with eight words a thread
+// (64 registers, 28 warps an SM) took 13.7 us, with three 9.9.
+template <typename T, int NI>
 __global__ void __launch_bounds__(256) ResidualNormKernel(Branch b, float* x, const float* gain_post, const float* gain_next, T* out, int n, float eps)
 {
   GridDependencySync();
@@ -73,12 +75,12 @@ __global__ void __launch_bounds__(256) ResidualNormKernel(Branch b, float* x, co
   const T* parts = static_cast<const T*>(b.parts);
   const float shared = b.gate != nullptr ? Sigmoid(b.gate[row * b.gate_ld]) : 1.f;
   const size_t at = static_cast<size_t>(row) * n;
-  if constexpr (VEC) {
+  if constexpr (NI > 0) {
     const int n4 = n >> 2;
-    float4 v[8];
+    float4 v[NI];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NI; ++i) {
       const int j = threadIdx.x + i * 256;
       v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (j < n4) {
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(256) ResidualNormKernel(Branch b, float* x, co
     const float inv = InvRms(CtaSum(ss, red), n, eps);
     ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NI; ++i) {
       const int j = threadIdx.x + i * 256;
       if (j < n4) {
         const float4 g = Load4(gain_post + 4 * j), r = Load4(x + at + 4 * j);
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(256) ResidualNormKernel(Branch b, float* x, co
     if (out == nullptr) return;
     const float inv2 = InvRms(CtaSum(ss, red), n, eps);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NI; ++i) {
       const int j = threadIdx.x + i * 256;
       if (j < n4) {
         const float4 g = Load4(gain_next + 4 * j);
@@ -145,67 +147,73 @@ struct RotateArgs {
   int count;
 };
 
-// One CTA per token, W elements a thread at a time (W 4: sizes, offsets and the halves of the rotation are multiples of 4).
+// A thread's way through the units of a part: unit i of head h, then 256 further, without a division each.
+struct Units {
+  int h, u, dh, du, per;
+  __device__ __forceinline__ Units(int per_head, int start) : h(start / per_head), u(start % per_head), dh(256 / per_head), du(256 % per_head), per(per_head) {}
+  __device__ __forceinline__ void Next()
+  {
+    h += dh;
+    u += du;
+    if (u >= per) {
+      u -= per;
+      ++h;
+    }
+  }
+};
+
+// A CTA per token and part.  W 4 (sizes, offsets and the halves of the rotation are multiples of 4): the two fours of a rotation at a time, each read once,
+// and the rest by fours; W 1: element by element.  2048 tokens of 5120 values (42 MB read, 21 written): 12.9 us with a division and the partner
+// read again per four, 10.1 so.
 template <typename T, int W>
 __global__ void __launch_bounds__(256) RotateRowsKernel(const float* in, int64_t ld, const __grid_constant__ RotateArgs a, const int* positions,
                                                         const float* cos_t, const float* sin_t, const int* slots, int rot_dims, int num_slots, int max_pos)
 {
   GridDependencySync();
+  const tlaloc_b200_rotate_part& s = a.part[blockIdx.y];
   const int t = blockIdx.x, half = rot_dims >> 1;
-  const float* row = in + static_cast<size_t>(t) * ld;
-  const int pos = min(max(__ldg(positions + t), 0), max_pos - 1);
-  const float *c_row = cos_t + static_cast<size_t>(pos) * half, *s_row = sin_t + static_cast<size_t>(pos) * half;
-  const int slot = slots != nullptr ? __ldg(slots + t) : 0;
-  for (int p = 0; p < a.count; ++p) {
-    const tlaloc_b200_rotate_part& s = a.part[p];
-    if (s.by_slot && (slot < 0 || slot >= num_slots)) continue;
-    T* dst = static_cast<T*>(s.out) + static_cast<size_t>(s.by_slot ? slot : t) * s.out_ld;
-    const int per = s.padded / W, total = s.heads * per;
-    for (int i = threadIdx.x; i < total; i += 256) {
-      const int h = i / per, c = (i - h * per) * W;
-      const float* src = row + s.first + h * s.dim;
-      float v[W];
-#pragma unroll
-      for (int e = 0; e < W; ++e) v[e] = 0.f;
-      if (c < s.dim) {
-        if constexpr (W == 4) {
-          const float4 u = Load4(src + c);
-          v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
-        } else {
-          v[0] = src[c];
-        }
-        if (s.rotate && c < rot_dims) {
-          const bool upper = c >= half;
-          const int f = upper ? c - half : c;
-          float o[W], cs[W], sn[W];
-          if constexpr (W == 4) {
-            const float4 u = Load4(src + (upper ? f : c + half)), cc = Load4(c_row + f), ss = Load4(s_row + f);
-            o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w;
-            cs[0] = cc.x; cs[1] = cc.y; cs[2] = cc.z; cs[3] = cc.w;
-            sn[0] = ss.x; sn[1] = ss.y; sn[2] = ss.z; sn[3] = ss.w;
-          } else {
-            o[0] = src[upper ? f : c + half];
-            cs[0] = c_row[f];
-            sn[0] = s_row[f];
-          }
-#pragma unroll
-          for (int e = 0; e < W; ++e) v[e] = upper ? v[e] * cs[e] + o[e] * sn[e] : v[e] * cs[e] - o[e] * sn[e];
-        }
-      }
-      T* d = dst + h * s.out_head_ld + c;
+  const int slot = s.by_slot ? __ldg(slots + t) : t;
+  if (s.by_slot && (slot < 0 || slot >= num_slots)) return;
+  const float* src = in + static_cast<size_t>(t) * ld + s.first;
+  T* dst = static_cast<T*>(s.out) + static_cast<size_t>(slot) * s.out_ld;
+  const int turned = s.rotate ? rot_dims : 0;
+  if (turned > 0) {
+    const int pos = min(max(__ldg(positions + t), 0), max_pos - 1);
+    const float *c_row = cos_t + static_cast<size_t>(pos) * half, *s_row = sin_t + static_cast<size_t>(pos) * half;
+    for (Units i(half / W, threadIdx.x); i.h < s.heads; i.Next()) {
+      const float* lo = src + i.h * s.dim + i.u * W;
+      T* d = dst + i.h * s.out_head_ld + i.u * W;
       if constexpr (W == 4) {
-        Store4(d, make_float4(v[0] * s.scale, v[1] * s.scale, v[2] * s.scale, v[3] * s.scale));
+        const float4 x = Load4(lo), y = Load4(lo + half), c = Load4(c_row + i.u * W), n = Load4(s_row + i.u * W);
+        Store4(d, make_float4((x.x * c.x - y.x * n.x) * s.scale, (x.y * c.y - y.y * n.y) * s.scale, (x.z * c.z - y.z * n.z) * s.scale, (x.w * c.w - y.w * n.w) * s.scale));
+        Store4(d + half, make_float4((y.x * c.x + x.x * n.x) * s.scale, (y.y * c.y + x.y * n.y) * s.scale, (y.z * c.z + x.z * n.z) * s.scale,
+                                     (y.w * c.w + x.w * n.w) * s.scale));
       } else {
-        *d = FromF32<T>(v[0] * s.scale);
+        const float x = lo[0], y = lo[half], c = c_row[i.u], n = s_row[i.u];
+        d[0] = FromF32<T>((x * c - y * n) * s.scale);
+        d[half] = FromF32<T>((y * c + x * n) * s.scale);
+      }
+    }
+  }
+  if (turned < s.padded) {
+    for (Units i((s.padded - turned) / W, threadIdx.x); i.h < s.heads; i.Next()) {
+      const int c = turned + i.u * W;
+      const float* from = src + i.h * s.dim + c;
+      T* d = dst + i.h * s.out_head_ld + c;
+      if constexpr (W == 4) {
+        const float4 x = c < s.dim ? Load4(from) : make_float4(0.f, 0.f, 0.f, 0.f);
+        Store4(d, make_float4(x.x * s.scale, x.y * s.scale, x.z * s.scale, x.w * s.scale));
+      } else {
+        d[0] = FromF32<T>((c < s.dim ? from[0] : 0.f) * s.scale);
       }
     }
   }
 }
 
 // One warp per (token, head): the two maps' outputs out of the slices' records ({maximum (log2), sum, acc[in_ld]}; slices > 0) or as
-// they are (slices 0); their difference, its norm, the head's gate.  PAIRS: even sizes up to 512 values, two a lane at a time, kept in
-// registers; else the values are computed twice.
-template <typename T, bool PAIRS>
+// they are (slices 0); their difference, its norm, the head's gate.  NI > 0: even sizes up to 64 NI values, two a lane at a time, kept in
+// registers; 0: any size, the values are computed twice.
+template <typename T, int NI>
 __global__ void __launch_bounds__(128) MapDifferenceKernel(const float* in, int slices, const float* gate, int64_t gate_ld, T* out, int64_t out_ld, int rows,
                                                            int heads, int vdim, int in_ld, float lambda, float keep, float eps)
 {
@@ -233,11 +241,11 @@ __global__ void __launch_bounds__(128) MapDifferenceKernel(const float* in, int 
   }
   const float g = keep * (gate != nullptr ? Sigmoid(gate[t * gate_ld + h]) : 1.f);
   T* dst = out + t * out_ld + static_cast<size_t>(h) * vdim;
-  if constexpr (PAIRS) {
+  if constexpr (NI > 0) {
     const int pairs = vdim >> 1;
-    float2 v[8];
+    float2 v[NI];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = make_float2(0.f, 0.f);
+    for (int i = 0; i < NI; ++i) v[i] = make_float2(0.f, 0.f);
     for (int s = 0; s < max(slices, 1); ++s) {
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
@@ -248,23 +256,23 @@ __global__ void __launch_bounds__(128) MapDifferenceKernel(const float* in, int 
           f *= exp2f(r[0] - top[p]);
           r += 2;
         }
-        float2 x[8];
+        float2 x[NI];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < NI; ++i) {
           if (lane + 32 * i < pairs) x[i] = *reinterpret_cast<const float2*>(r + 2 * (lane + 32 * i));
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < NI; ++i) {
           if (lane + 32 * i < pairs) v[i] = make_float2(fmaf(f, x[i].x, v[i].x), fmaf(f, x[i].y, v[i].y));
         }
       }
     }
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, ss));
+    for (int i = 0; i < NI; ++i) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, ss));
     const float f = InvRms(WarpSum(ss), vdim, eps) * g;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NI; ++i) {
       if (lane + 32 * i < pairs) StorePair(dst + 2 * (lane + 32 * i), v[i].x * f, v[i].y * f);
     }
   } else {
@@ -290,8 +298,9 @@ __global__ void __launch_bounds__(128) MapDifferenceKernel(const float* in, int 
   }
 }
 
-// One warp per (token, head): a recurrence's output over its root mean square, times silu of the gate.  PAIRS as above.
-template <typename T, bool PAIRS>
+// One warp per (token, head): a recurrence's output over its root mean square, times silu of the gate.  NI as above.  Bound by the instructions issued: 40960 rows of
+// 128 with eight pairs of values a lane, most of them past the row's end, took 13.7 us, with two 11.9.
+template <typename T, int NI>
 __global__ void __launch_bounds__(128) HeadNormGateKernel(const float* in, const float* gate, int64_t gate_ld, T* out, int64_t out_ld, int rows, int heads,
                                                           int vdim, float eps)
 {
@@ -303,11 +312,11 @@ __global__ void __launch_bounds__(128) HeadNormGateKernel(const float* in, const
   const float* g = gate + t * gate_ld + static_cast<size_t>(h) * vdim;
   T* dst = out + t * out_ld + static_cast<size_t>(h) * vdim;
   float ss = 0.f;
-  if constexpr (PAIRS) {
+  if constexpr (NI > 0) {
     const int pairs = vdim >> 1;
-    float2 v[8], z[8];
+    float2 v[NI], z[NI];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NI; ++i) {
       v[i] = z[i] = make_float2(0.f, 0.f);
       if (lane + 32 * i < pairs) {
         v[i] = *reinterpret_cast<const float2*>(a + 2 * (lane + 32 * i));
@@ -315,10 +324,10 @@ __global__ void __launch_bounds__(128) HeadNormGateKernel(const float* in, const
       }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, ss));
+    for (int i = 0; i < NI; ++i) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, ss));
     const float inv = InvRms(WarpSum(ss), vdim, eps);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NI; ++i) {
       if (lane + 32 * i < pairs) StorePair(dst + 2 * (lane + 32 * i), v[i].x * inv * Silu(z[i].x), v[i].y * inv * Silu(z[i].y));
     }
   } else {
@@ -348,14 +357,19 @@ extern "C" int tlaloc_b200_residual_norm(const float* y, const float* gate, int6
   const Branch b = {y, gate, gate_ld, parts, part_rows, part_weights, top};
   const bool vec = n % 4 == 0 && n <= 8192 && Aligned16(y) && Aligned16(parts) && Aligned16(x) && Aligned16(gain_post) && Aligned16(gain_next) && Aligned16(out);
   cudaError_t e;
-#define TLALOC_LAUNCH(T, VEC) e = LaunchChained(ResidualNormKernel<T, VEC>, rows, 256, 0, st, b, x, gain_post, gain_next, static_cast<T*>(out), n, eps)
+#define TLALOC_LAUNCH(T, NI) e = LaunchChained(ResidualNormKernel<T, NI>, rows, 256, 0, st, b, x, gain_post, gain_next, static_cast<T*>(out), n, eps)
+#define TLALOC_LAUNCH_NI(T)                     \
+  if (!vec) TLALOC_LAUNCH(T, 0);                \
+  else if (n <= 2 * 1024) TLALOC_LAUNCH(T, 2);  \
+  else if (n <= 3 * 1024) TLALOC_LAUNCH(T, 3);  \
+  else if (n <= 4 * 1024) TLALOC_LAUNCH(T, 4);  \
+  else TLALOC_LAUNCH(T, 8)
   if (dtype == TLALOC_B200_F32) {
-    if (vec) TLALOC_LAUNCH(float, true);
-    else TLALOC_LAUNCH(float, false);
+    TLALOC_LAUNCH_NI(float);
   } else {
-    if (vec) TLALOC_LAUNCH(__nv_bfloat16, true);
-    else TLALOC_LAUNCH(__nv_bfloat16, false);
+    TLALOC_LAUNCH_NI(__nv_bfloat16);
   }
+#undef TLALOC_LAUNCH_NI
 #undef TLALOC_LAUNCH
   if (e != cudaSuccess) return CudaFail("RESIDUAL_NORM launch", e);
   CountLaunches(1);
@@ -390,7 +404,7 @@ extern "C" int tlaloc_b200_rotate_rows(const float* in, int64_t ld, const tlaloc
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e;
 #define TLALOC_LAUNCH(T, W) \
-  e = LaunchChained(RotateRowsKernel<T, W>, num_tokens, 256, 0, st, in, ld, a, positions, cos_table, sin_table, slot_mapping, rot_dims, num_slots, max_pos)
+  e = LaunchChained(RotateRowsKernel<T, W>, dim3(num_tokens, count), 256, 0, st, in, ld, a, positions, cos_table, sin_table, slot_mapping, rot_dims, num_slots, max_pos)
   if (dtype == TLALOC_B200_F32) {
     if (vec) TLALOC_LAUNCH(float, 4);
     else TLALOC_LAUNCH(float, 1);
@@ -403,6 +417,14 @@ extern "C" int tlaloc_b200_rotate_rows(const float* in, int64_t ld, const tlaloc
   CountLaunches(1);
   return kOk;
 }
+
+// By the pairs of values a lane has of a row of vdim (pairs: even and aligned, up to 512).
+#define TLALOC_LAUNCH_PAIRS(T)                \
+  if (!pairs) TLALOC_LAUNCH(T, 0);            \
+  else if (vdim <= 64) TLALOC_LAUNCH(T, 1);   \
+  else if (vdim <= 128) TLALOC_LAUNCH(T, 2);  \
+  else if (vdim <= 256) TLALOC_LAUNCH(T, 4);  \
+  else TLALOC_LAUNCH(T, 8)
 
 extern "C" int tlaloc_b200_map_difference(const float* in, int32_t slices, const float* gate, int64_t gate_ld, void* out, int64_t out_ld, int32_t dtype,
                                           int32_t rows, int32_t heads, int32_t vdim, int32_t in_ld, float lambda, float keep, float eps, void* stream)
@@ -417,14 +439,12 @@ extern "C" int tlaloc_b200_map_difference(const float* in, int32_t slices, const
   cudaError_t e;
   const bool pairs = vdim % 2 == 0 && in_ld % 2 == 0 && vdim <= 512 && out_ld % 2 == 0 && reinterpret_cast<uintptr_t>(in) % 8 == 0 &&
                      reinterpret_cast<uintptr_t>(out) % 8 == 0;
-#define TLALOC_LAUNCH(T, PAIRS) \
-  e = LaunchChained(MapDifferenceKernel<T, PAIRS>, blocks, 128, 0, st, in, slices, gate, gate_ld, static_cast<T*>(out), out_ld, rows, heads, vdim, in_ld, lambda, keep, eps)
+#define TLALOC_LAUNCH(T, NI) \
+  e = LaunchChained(MapDifferenceKernel<T, NI>, blocks, 128, 0, st, in, slices, gate, gate_ld, static_cast<T*>(out), out_ld, rows, heads, vdim, in_ld, lambda, keep, eps)
   if (dtype == TLALOC_B200_F32) {
-    if (pairs) TLALOC_LAUNCH(float, true);
-    else TLALOC_LAUNCH(float, false);
+    TLALOC_LAUNCH_PAIRS(float);
   } else {
-    if (pairs) TLALOC_LAUNCH(__nv_bfloat16, true);
-    else TLALOC_LAUNCH(__nv_bfloat16, false);
+    TLALOC_LAUNCH_PAIRS(__nv_bfloat16);
   }
 #undef TLALOC_LAUNCH
   if (e != cudaSuccess) return CudaFail("MAP_DIFFERENCE launch", e);
@@ -445,14 +465,12 @@ extern "C" int tlaloc_b200_head_norm_gate(const float* in, const float* gate, in
   cudaError_t e;
   const bool pairs = vdim % 2 == 0 && vdim <= 512 && out_ld % 2 == 0 && gate_ld % 2 == 0 && reinterpret_cast<uintptr_t>(in) % 8 == 0 &&
                      reinterpret_cast<uintptr_t>(gate) % 8 == 0 && reinterpret_cast<uintptr_t>(out) % 8 == 0;
-#define TLALOC_LAUNCH(T, PAIRS) \
-  e = LaunchChained(HeadNormGateKernel<T, PAIRS>, blocks, 128, 0, st, in, gate, gate_ld, static_cast<T*>(out), out_ld, rows, heads, vdim, eps)
+#define TLALOC_LAUNCH(T, NI) \
+  e = LaunchChained(HeadNormGateKernel<T, NI>, blocks, 128, 0, st, in, gate, gate_ld, static_cast<T*>(out), out_ld, rows, heads, vdim, eps)
   if (dtype == TLALOC_B200_F32) {
-    if (pairs) TLALOC_LAUNCH(float, true);
-    else TLALOC_LAUNCH(float, false);
+    TLALOC_LAUNCH_PAIRS(float);
   } else {
-    if (pairs) TLALOC_LAUNCH(__nv_bfloat16, true);
-    else TLALOC_LAUNCH(__nv_bfloat16, false);
+    TLALOC_LAUNCH_PAIRS(__nv_bfloat16);
   }
 #undef TLALOC_LAUNCH
   if (e != cudaSuccess) return CudaFail("HEAD_NORM_GATE launch", e);
