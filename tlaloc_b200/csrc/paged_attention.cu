@@ -1491,15 +1491,19 @@ cudaError_t LaunchGeneric(const PaParams& p, cudaStream_t stream)
   return LaunchChained(PaSliceGeneric<QT, KVT>, dim3(p.S, p.Hkv, p.Tb), kGenThreads, smem, stream, p);
 }
 
-// Positions per slice of the tensor-core kernel when the scratch allows it; $TLALOC_B200_PA_SLICE overrides.
+// Positions per slice of the tensor-core kernels when the scratch allows it, for `pairs` (table, KV head) pairs that see up to `seen` positions each;
+// $TLALOC_B200_PA_SLICE overrides.
 // A CTA pays about 3 us of latency before its first position (lengths and table entries, then the first K/V rows)
 // and again to merge its warps and write its records, so slices should be as long as the grid can afford: 1024
 // positions, doubled (up to 4096) while the launch would still have some 2000 CTAs at the longest context, i.e. a
-// few waves of the 444 resident ones at typical lengths.  Measured on the 70B step (1024 (table, KV head) pairs,
+// few waves of the 444 resident ones at typical lengths, and halved (down to 256) while it would not fill one wave.  Measured on the 70B step (1024 pairs,
 // contexts up to 16K): 0.718 -> 0.670 -> 0.661 ms per layer at 1024 / 2048 / 4096; 512 pairs: 382 / 374 / 372 us; 256
-// pairs: 203 / 200 / 222 us; 128 pairs (one KV head per rank): 117 / 128 us, and 256 pairs at contexts up to 8K also
-// keep 1024.
-int PreferredSlice(int ctx, long long pairs)
+// pairs: 203 / 200 / 222 us; 500 pairs of 64 channels 190 / 188 / 216; 128 pairs (one KV head per rank): 117 / 128 us.
+// e4m3fn rows are half as long and their CTAs (592 resident) wait less for memory than for their conversions, so an uneven last wave costs more: 320 pairs
+// at up to 16K 94 / 124 / 150 us, 500 pairs 139 / 158 / 199, 1024 pairs 435 / 408 / 422.
+// Few pairs, lengths spread up to the context, at 256 / 512 / 1024 us: 8 pairs of 16000 e4m3fn 9.4 / 11.9 / 17.2; 64 pairs of 2000 bf16 16.7 / 16.7 / 20.0, of 4000
+// 24.7 / 21.2 / 22.9, of 4000 e4m3fn 19.4 / 22.7 / 21.7; 256 pairs of 1000 e4m3fn 15.8 / 13.7 / 15.9.
+int PreferredSlice(int seen, long long pairs, bool f8)
 {
   static const int forced = [] {
     const char* e = std::getenv("TLALOC_B200_PA_SLICE");
@@ -1508,7 +1512,9 @@ int PreferredSlice(int ctx, long long pairs)
   }();
   if (forced > 0) return forced;
   int slice = 1024;
-  while (slice < 4096 && pairs * ((ctx + 2 * slice - 1) / (2 * slice)) >= 2000) slice *= 2;
+  auto ctas = [&](int length) { return pairs * ((seen + length - 1) / length); };
+  while (slice < 4096 && ctas(2 * slice) >= (f8 ? 5000 : 2048)) slice *= 2;
+  while (slice > 256 && ctas(slice) < (f8 ? 592 : 444)) slice /= 2;
   return slice;
 }
 
@@ -1674,7 +1680,8 @@ extern "C" int tlaloc_b200_paged_attention(const void* query, int32_t q_dtype, c
   const bool mma = (kv_dtype == TLALOC_B200_BF16 || (f8 && !f8_generic)) && (head_dim == 64 || head_dim == 128) && p.NQ <= kMmaQ &&
                    keep == nullptr && (f8 ? block_size >= 16 : block_size >= 8) && Aligned16(key_cache) && Aligned16(value_cache);
   // Slice length: the preferred one (tensor-core kernel) or 256, stretched until `splits` slices cover the context.
-  int slice = mma ? PreferredSlice(ctx, static_cast<long long>(num_tables) * num_kv_heads) : 256;
+  const int seen = sliding_window > 0 ? std::min(sliding_window, ctx) : ctx;
+  int slice = mma ? PreferredSlice(seen, static_cast<long long>(num_tables) * num_kv_heads, f8) : 256;
   if (static_cast<int64_t>(slice) * splits < ctx) slice = (ctx + splits - 1) / splits;
   if (mma) slice = std::min((slice + 15) / 16 * 16, 8192);
   if (static_cast<int64_t>(slice) * splits < ctx) {
