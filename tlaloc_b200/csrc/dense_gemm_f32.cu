@@ -16,13 +16,16 @@
 //
 // D[n, m] = sum_k W[n, k] X[m, k]: 128 weight rows are the MMA's M, a tile of up to 208 activation rows its N.
 //   producer lane boxes of 32 k of both operands by TMA (f32, 128-byte swizzle), two to eight stages ahead
-//   sixteen warps split a chunk of 32 k into the three planes (128-byte swizzle; a buffer is one half of the planes' rows)
+//   sixteen warps split a chunk of 32 k into the three planes: the weights' go to TMEM (a lane a row; an MMA of 208 columns takes 114 cycles with A there, 148
+//                 with A in shared memory, whose bandwidth the splits' stores need as well), the activations' to shared memory (128-byte swizzle; a
+//                 buffer is one half of the planes' rows)
 //   MMA lane      the six products of a chunk, into one of two accumulators
 //   eight warps   add the finished accumulator to sums in registers (104 a thread at 208 rows, hence the register split), and write the tile
 //   persistent    a CTA walks tiles;   K slices   the slices of a tile are a cluster and sum their partial tiles in rank order
-// Bound at 208 rows by the split and the six products, which run side by side (each alone takes about 100 us of the 109 us of 203 rows, n 18944, k 2048),
-// at few rows by the way of a chunk through the three kinds of warps (0.85 us each).  203 rows, n 2048, k 10304: 85 us, 1414 us with plain FMAs; one
-// row, n 32768, k 2048: 113 us, 443 us.  Every mbarrier wait is bounded.  Sums computed again: 203 rows, n 18944, k 2048 with one row of NaN 0.26 ms, all
+// Bound at 208 rows by the split and the six products, which run side by side (203 rows, n 18944, k 2048: 106 us with the weights' planes in shared memory too, where
+// each of the two alone took about 100; 92 us now, the split first: its warps wait for one another's latencies, with 40 registers there is one group of words at a time),
+// at few rows by the way of a chunk through the three kinds of warps (0.8 us each).  203 rows, n 2048, k 10304: 77 us, 1414 us with plain FMAs; one
+// row, n 32768, k 2048: 106 us, 443 us.  Every mbarrier wait is bounded.  Sums computed again: 203 rows, n 18944, k 2048 with one row of NaN 0.26 ms, all
 // infinite 2.2 ms (DenseGemmTiled 0.85 ms); n 2048, k 10304: 0.80, 2.3 (1.4) ms.
 #include <cuda.h>
 
@@ -37,24 +40,34 @@ using namespace tc;
 
 constexpr int kBN = 128, kBK = 32, kSumWarps = 8, kSplitWarps = 16, kMmaWarp = kSumWarps + kSplitWarps, kProducerWarp = kMmaWarp + 1;
 constexpr int kThreads = (kMmaWarp + 4) * 32;
+constexpr int kOutUnits = 4;
 
 // BT: most activation rows of a tile.
 template <int BT>
 struct Layout {
-  static constexpr int kPlane = (kBN + BT) * 128;  // 64 k a row: two buffers of 32
+  static constexpr int kPlane = BT * 128;  // of the activations, 64 k a row: two buffers of 32
   static constexpr int kRaw = 3 * kPlane;
   static constexpr int kStage = (kBN + BT) * 128;
   static constexpr int kStages = BT == 208 ? 2 : BT == 128 ? 3 : BT == 64 ? 6 : 8;
-  static constexpr int kTileStride = kBN + 4;  // a slice's partial tile [BT][kTileStride] f32, aliases the planes
-  static_assert(kRaw >= BT * kTileStride * 4, "the partial tile aliases the planes");
-  static constexpr int kBars = kRaw + kStages * kStage;
+  static constexpr int kTileStride = kBN + 4;  // a slice's partial tile [BT][kTileStride] f32, aliases the planes and the ring
+  static constexpr int kOut = kRaw + kStages * kStage;  // what each sum warp has finished of its tile, kOutUnits of its units at a time
+  static_assert(kOut >= BT * kTileStride * 4, "the partial tile aliases the planes and the ring");
+  static constexpr int kBars = kOut + kSumWarps * kOutUnits * 8 * 32 * 4;
   static constexpr int kSlot = kBars + 8 * (6 + 2 * kStages);
   static constexpr int kBytes = kSlot + 16 + 1024;  // slack to align to 1024
   // Registers a thread of the three kinds of warpgroups; 128 * (2 * sum + 4 * split + mma) is the 896 * 72 of the launch.
   static constexpr int kSumRegs = 152, kSplitRegs = 40, kMmaRegs = 40;
   static_assert(128 * (2 * kSumRegs + 4 * kSplitRegs + kMmaRegs) <= kThreads * 72, "more registers than the launch has");
   static constexpr int kUnits = BT / 16;           // groups of eight activation rows a thread sums
-  static constexpr int kAcc = BT <= 32 ? 32 : BT <= 64 ? 64 : BT <= 128 ? 128 : 256;  // TMEM columns of an accumulator
+  // TMEM: two accumulators kAcc columns apart, and the weights' three planes of a chunk, sixteen columns each, twice.
+  static constexpr int kAcc = BT == 208 ? 224 : BT;
+  static constexpr uint32_t kCols = BT >= 128 ? 512 : 256;
+  __device__ static constexpr uint32_t PlaneColumn(int buffer, int plane)
+  {
+    const int i = buffer * 3 + plane;
+    if (BT == 208) return i < 5 ? 432 + 16 * i : 208;  // the last one between the accumulators
+    return 2 * kAcc + 16 * i;
+  }
 };
 
 struct F32Args {
@@ -211,17 +224,40 @@ __device__ __forceinline__ void Finish(const tlaloc_b200_dense_problem& p, const
     return;
   }
   if (n >= p.n) return;
+  // What is the same for all eight is asked once, ahead of them: few warps are left here, and a chain of questions for each value was most of a short tile's
+  // time.
+  const int64_t y_step = step * p.ld_y;
+  const size_t at = out + static_cast<size_t>(m) * p.ld_y + n;
+  float o[kU];
   const float bias = p.bias != nullptr ? __ldg(p.bias + n) : 0.f;
-  float res[kU];
 #pragma unroll
   for (int c = 0; c < kU; ++c) {
-    const int r = m + c * step;
-    res[c] = p.residual != nullptr && r < end ? p.residual[static_cast<size_t>(r) * p.ld_res + n] : 0.f;
+    o[c] = v[c] + bias;
+    if (m + c * step >= end) bits &= ~(1u << c);
   }
+  if (p.act != TLALOC_B200_ACT_NONE) {
 #pragma unroll
-  for (int c = 0; c < kU; ++c) {
-    const int r = m + c * step;
-    if (r < end && (bits >> c & 1u) != 0) Put(p, out + static_cast<size_t>(r) * p.ld_y + n, DenseActivation(p.act, v[c] + bias) + res[c]);
+    for (int c = 0; c < kU; ++c) o[c] = DenseActivation(p.act, o[c]);
+  }
+  if (p.residual != nullptr) {
+    const float* from = p.residual + static_cast<size_t>(m) * p.ld_res + n;
+    const int64_t r_step = step * p.ld_res;
+    float res[kU];
+#pragma unroll
+    for (int c = 0; c < kU; ++c) res[c] = (bits >> c & 1u) != 0 ? from[c * r_step] : 0.f;
+#pragma unroll
+    for (int c = 0; c < kU; ++c) o[c] += res[c];
+  }
+  if (p.y_dtype == TLALOC_B200_F32) {
+    float* y = static_cast<float*>(p.y) + at;
+#pragma unroll
+    for (int c = 0; c < kU; ++c)
+      if ((bits >> c & 1u) != 0) y[c * y_step] = o[c];
+  } else {
+    __nv_bfloat16* y = static_cast<__nv_bfloat16*>(p.y) + at;
+#pragma unroll
+    for (int c = 0; c < kU; ++c)
+      if ((bits >> c & 1u) != 0) y[c * y_step] = __float2bfloat16_rn(o[c]);
   }
 }
 
@@ -254,6 +290,11 @@ __device__ __forceinline__ void TcLd8(uint32_t taddr, uint32_t* r)
                : "r"(taddr));
 }
 
+__device__ __forceinline__ void TcSt4(uint32_t taddr, const uint32_t (&r)[4])
+{
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0, %1, %2, %3};\n" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(taddr) : "memory");
+}
+
 // The chunks of a tile that a CTA sums: all of them, or the slice of its cluster rank.
 __device__ __forceinline__ int Chunks(const F32Args& a, const Tile& t, int& first)
 {
@@ -283,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 {
   using L = Layout<BT>;
   constexpr int S = L::kStages;
-  constexpr uint32_t kCols = 2 * L::kAcc;
+  constexpr uint32_t kCols = L::kCols;
   extern __shared__ unsigned char smem_raw[];
   __shared__ int s_start[kMaxGroups + 1];
   const uint32_t base = (SmemAddr(smem_raw) + 1023u) & ~1023u;  // the swizzle is a function of address bits 4..9
@@ -347,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == kMmaWarp && ElectOne()) {
       // f32 accumulator, bf16 A and B, both K-major, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(a.bt >> 3) << 17) | (8u << 24);
-      const uint64_t wd = SmemDesc(base, 16, 1024), xd = SmemDesc(base + kBN * 128, 16, 1024);
+      const uint64_t xd = SmemDesc(base, 16, 1024);
       for (int id = blockIdx.x; id < tiles; id += gridDim.x) {
         const Tile t = TileAt(a, id, s_start);
         int first;
@@ -359,20 +400,21 @@ __global__ void __launch_bounds__(kThreads, 1)
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           const uint32_t acc = tmem + b * L::kAcc;
           constexpr uint32_t P = L::kPlane >> 4;
-          const uint64_t w = wd + 4 * b, x = xd + 4 * b;
+          const uint64_t x = xd + 4 * b;
+          const uint32_t high = tmem + L::PlaneColumn(b, 0), middle = tmem + L::PlaneColumn(b, 1), low = tmem + L::PlaneColumn(b, 2);
           // planes high, middle, low: small products first
-          TcMmaBf16(acc, w, x + 2 * P, idesc, 0u);
-          TcMmaBf16(acc, w + 2, x + 2 * P + 2, idesc, 1u);
-          TcMmaBf16(acc, w + 2 * P, x, idesc, 1u);
-          TcMmaBf16(acc, w + 2 * P + 2, x + 2, idesc, 1u);
-          TcMmaBf16(acc, w + P, x + P, idesc, 1u);
-          TcMmaBf16(acc, w + P + 2, x + P + 2, idesc, 1u);
-          TcMmaBf16(acc, w, x + P, idesc, 1u);
-          TcMmaBf16(acc, w + 2, x + P + 2, idesc, 1u);
-          TcMmaBf16(acc, w + P, x, idesc, 1u);
-          TcMmaBf16(acc, w + P + 2, x + 2, idesc, 1u);
-          TcMmaBf16(acc, w, x, idesc, 1u);
-          TcMmaBf16(acc, w + 2, x + 2, idesc, 1u);
+          TcMmaTmemA(acc, high, x + 2 * P, idesc, 0u);
+          TcMmaTmemA(acc, high + 8, x + 2 * P + 2, idesc, 1u);
+          TcMmaTmemA(acc, low, x, idesc, 1u);
+          TcMmaTmemA(acc, low + 8, x + 2, idesc, 1u);
+          TcMmaTmemA(acc, middle, x + P, idesc, 1u);
+          TcMmaTmemA(acc, middle + 8, x + P + 2, idesc, 1u);
+          TcMmaTmemA(acc, high, x + P, idesc, 1u);
+          TcMmaTmemA(acc, high + 8, x + P + 2, idesc, 1u);
+          TcMmaTmemA(acc, middle, x, idesc, 1u);
+          TcMmaTmemA(acc, middle + 8, x + 2, idesc, 1u);
+          TcMmaTmemA(acc, high, x, idesc, 1u);
+          TcMmaTmemA(acc, high + 8, x + 2, idesc, 1u);
           TcCommit(done + 8 * b);
         }
       }
@@ -435,11 +477,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp >= kSumWarps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(L::kSplitRegs));
-    // A lane's eight k are two 16-byte words of a row of the stage and one of each plane's; four lanes a row, and the two rows of a phase of
+    // Weights: a thread has a row of the warp's TMEM lanes and eight k, two 16-byte words of a row of the stage (the eight lanes of a phase have them in
+    // different places by the swizzle) and four columns of each plane.
+    // Activations: a lane's eight k are two words of a row of the stage and one of each plane's; four lanes a row, and the two rows of a phase of
     // eight lanes differ by 5 in their swizzle, so that neither the loads (words 0 2 4 6 of a row) nor the stores (words 0 - 3, or 4 - 7) collide.
-    const int sw = warp - kSumWarps, u = lane & 3, low = (lane >> 3) ^ ((lane & 4) != 0 ? 5 : 0);
-    const uint32_t from0 = base + L::kRaw + low * 128 + (((2 * u) ^ low) << 4), to0 = base + low * 128 + ((u ^ low) << 4);
-    const int groups = (kBN + a.bt) >> 3;  // of eight rows
+    const int sw = warp - kSumWarps, u = lane & 3, low = (lane >> 3) ^ ((lane & 4) != 0 ? 5 : 0), w_row = (warp & 3) * 32 + lane, w_k = sw >> 2;
+    const uint32_t w_from = base + L::kRaw + w_row * 128 + (((2 * w_k) ^ (w_row & 7)) << 4);
+    const uint32_t w_to = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 4 * w_k;
+    const uint32_t from0 = base + L::kRaw + kBN * 128 + low * 128 + (((2 * u) ^ low) << 4), to0 = base + low * 128 + ((u ^ low) << 4);
+    const int groups = a.bt >> 3;  // of eight rows of activations
     int s = 0, phase = 0;
     for (int id = blockIdx.x; id < tiles; id += gridDim.x) {
       const Tile t = TileAt(a, id, s_start);
@@ -448,17 +494,27 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int c = 0; c < nb; ++c, ++it) {
         ok = MbarWaitAliveWarp(landed + 8 * s, phase, lane, words) && ok;
         if (it >= 2) ok = MbarWaitAliveWarp(done + 8 * (it & 1), ((it >> 1) - 1) & 1, lane, words) && ok;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t from = from0 + s * L::kStage, to = to0 ^ ((it & 1) << 6);
-#pragma unroll
-        for (int i = 0; i < (kBN + BT) / 8; i += kSplitWarps) {
-          const int g = i + sw;
-          if (g >= groups) break;
+        auto split = [](uint32_t at, uint32_t (&part)[3][4]) {
           uint64_t v[4];
-          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[0]), "=l"(v[1]) : "r"(from + g * 1024));
-          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[2]), "=l"(v[3]) : "r"((from + g * 1024) ^ 16));
-          uint32_t part[3][4];
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[0]), "=l"(v[1]) : "r"(at));
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[2]), "=l"(v[3]) : "r"(at ^ 16));
 #pragma unroll
           for (int e = 0; e < 4; ++e) Split2(v[e], part[0][e], part[1][e], part[2][e]);
+        };
+        {
+          uint32_t part[3][4];
+          split(w_from + s * L::kStage, part);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) TcSt4(w_to + ((it & 1) != 0 ? L::PlaneColumn(1, q) : L::PlaneColumn(0, q)), part[q]);
+        }
+#pragma unroll
+        for (int i = 0; i < BT / 8; i += kSplitWarps) {
+          const int g = i + sw;
+          if (g >= groups) break;
+          uint32_t part[3][4];
+          split(from + g * 1024, part);
 #pragma unroll
           for (int q = 0; q < 3; ++q) {
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(to + g * 1024 + q * L::kPlane), "r"(part[q][0]), "r"(part[q][1]),
@@ -466,6 +522,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                          : "memory");
           }
         }
+        asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncwarp();
         if (lane == 0) {
@@ -519,18 +577,46 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) MbarArrive(empty + 8 * (it & 1));
       }
       if (a.ks <= 1) {
+        // Through shared memory, a few units at a time, so that there is one copy of the epilogue's code: unrolled over the registers it was 470 KB, all
+        // of which a tile fetched once (203 rows, n 128, k 32: 26.1 us, 22.2 so, 14.4 with the epilogue's questions asked once for eight values).
         const int n = t.n0 + quad * 32 + lane, m = t.m0 + col0;
-        uint32_t doubt[(L::kUnits + 3) / 4] = {};
+        constexpr int kRounds = (L::kUnits + kOutUnits - 1) / kOutUnits;
+        float* place = reinterpret_cast<float*>(smem + L::kOut) + warp * (kOutUnits * 8 * 32) + lane;
+        uint32_t doubt[kRounds] = {};
+#pragma unroll 1
+        for (int i = 0; i < kRounds; ++i) {
+          __syncwarp();
 #pragma unroll
-        for (int q = 0; q < L::kUnits; ++q)
-          if (q < units) doubt[q >> 2] |= FinishSure(p, t, n, m + q * 8, 1, t.M, acc[q]) << 8 * (q & 3);
+          for (int q = 0; q < L::kUnits; ++q) {
+            if (q / kOutUnits == i) {
 #pragma unroll
-        for (int i = 0; i < (L::kUnits + 3) / 4; ++i)
-          for (int q = 0; q < 4 && __any_sync(0xffffffffu, doubt[i] != 0); ++q, doubt[i] >>= 8) {
-            FinishDoubtful(p, t, n, m + (i * 4 + q) * 8, 1, t.M, doubt[i] & 255u, words + 1);
+              for (int e = 0; e < 8; ++e) place[((q % kOutUnits) * 8 + e) * 32] = acc[q][e];
+            }
           }
+          __syncwarp();
+          uint32_t bits = 0;
+#pragma unroll 1
+          for (int q = i * kOutUnits; q < min(units, (i + 1) * kOutUnits); ++q) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = place[((q % kOutUnits) * 8 + e) * 32];
+            bits |= FinishSure(p, t, n, m + q * 8, 1, t.M, v) << 8 * (q % kOutUnits);
+          }
+#pragma unroll
+          for (int j = 0; j < kRounds; ++j) doubt[j] = j == i ? bits : doubt[j];
+        }
+#pragma unroll 1
+        for (int i = 0; i < kRounds; ++i) {
+          uint32_t bits = 0;
+#pragma unroll
+          for (int j = 0; j < kRounds; ++j) bits = j == i ? doubt[j] : bits;
+#pragma unroll 1
+          for (int q = 0; q < kOutUnits && __any_sync(0xffffffffu, bits != 0); ++q, bits >>= 8) {
+            FinishDoubtful(p, t, n, m + (i * kOutUnits + q) * 8, 1, t.M, bits & 255u, words + 1);
+          }
+        }
       } else {
-        float* tile = reinterpret_cast<float*>(smem);  // over the planes: every MMA of this CTA's one tile is through
+        float* tile = reinterpret_cast<float*>(smem);  // over the planes and the ring: every chunk of this CTA's one tile has been split, every MMA is through
 #pragma unroll
         for (int q = 0; q < L::kUnits; ++q) {
           if (q < units) {
