@@ -219,6 +219,34 @@ __device__ __forceinline__ void I8Split4(float a, float b, float c, float d, flo
 }
 __device__ __forceinline__ float Bf16Value(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
+// Sums over the ranks of a cluster, in rank order: U words of every rank's shared memory, `step` words apart from the place of this CTA's `mine`, the first
+// `count` of them there.  All loads are in flight before the first add: one way to the peers, not one for each of the (up to eight) ranks.
+template <int U>
+__device__ __forceinline__ void SumRanks(const float* mine, int ranks, int step, int count, float (&v)[U])
+{
+  const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(mine));
+  float w[8][U];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (q < ranks) {
+      uint32_t peer;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(peer) : "r"(at), "r"(q));
+#pragma unroll
+      for (int e = 0; e < U; ++e) {
+        w[q][e] = 0.f;
+        if (e < count) asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(w[q][e]) : "r"(peer + e * step * 4));
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < U; ++e) {
+    v[e] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < ranks) v[e] += w[q][e];
+  }
+}
+
 inline bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace tlaloc_b200

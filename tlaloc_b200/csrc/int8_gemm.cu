@@ -286,13 +286,22 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
   const float scale = p.scales != nullptr && col < p.N ? __ldg(p.scales + col) : 1.f;  // on its way while the ranks meet
   cluster.sync();
   YT* y = static_cast<YT*>(p.y);
-  for (int m = rank; m < p.M; m += nranks) {
-    if (col < p.N) {
-      float v = 0.f;
-      for (unsigned q = 0; q < nranks; ++q) v += cluster.map_shared_rank(tile, q)[m * kGvRedStride + tid];
-      if (p.scales != nullptr) v *= scale;
-      if (p.residual != nullptr) v += __ldg(p.residual + static_cast<size_t>(m) * p.N + col);
-      y[static_cast<size_t>(m) * p.N + col] = FromF32<YT>(v);
+  constexpr int kU = NT == 1 ? 1 : 2;  // rows at a time: with eight ranks a CTA has one of eight rows, two of sixteen
+  for (int m0 = rank; m0 < p.M && col < p.N; m0 += kU * nranks) {
+    float v[kU], residual[kU];
+#pragma unroll
+    for (int e = 0; e < kU; ++e) {
+      const int m = m0 + e * static_cast<int>(nranks);
+      residual[e] = p.residual != nullptr && m < p.M ? __ldg(p.residual + static_cast<size_t>(m) * p.N + col) : 0.f;
+    }
+    SumRanks(tile + m0 * kGvRedStride + tid, nranks, nranks * kGvRedStride, (p.M - m0 + nranks - 1) / nranks, v);
+#pragma unroll
+    for (int e = 0; e < kU; ++e) {
+      const int m = m0 + e * static_cast<int>(nranks);
+      if (m >= p.M) break;
+      if (p.scales != nullptr) v[e] *= scale;
+      if (p.residual != nullptr) v[e] += residual[e];
+      y[static_cast<size_t>(m) * p.N + col] = FromF32<YT>(v[e]);
     }
   }
   cluster.sync();  // no CTA leaves while a peer may still read its tile
