@@ -7,7 +7,7 @@
 //                    128 output columns and one slice of K; each of its four warps is an independent cp.async
 //                    pipeline over its own 32-row stages (a 32 x 128 int8 weight tile plus the matching 32-wide
 //                    strip of the bf16 activations, XOR-swizzled in shared memory), so there is no CTA-wide barrier
-//                    in the loop and four CTAs fit an SM.  The MMA runs transposed: the 16 output columns a lane
+//                    in the loop and six CTAs fit an SM.  The MMA runs transposed: the 16 output columns a lane
 //                    pair-set owns are the M dimension and the (<= 8 per n-tile) activation rows the N dimension, so
 //                    one 16-row step costs 8 mma.sync m16n8k16 per n-tile.  The int8 codes become exact bf16 pairs in
 //                    registers (one byte-permute, two logic ops and one packed bf16 add per pair); products are
@@ -17,7 +17,8 @@
 //                    is applied to the finished sum, as the graph multiplies after the dot.
 //                    Bound at one row by the issue of the conversion (ncu, 4096 x 28672: ALU pipe 57 %, issue slots 50 % busy, 3.3 warps a scheduler)
 //                    and by the SMs that idle at its ends (22 % of the time).  4096 x 28672 with a norm in front: 34.3 us with two slices and a division
-//                    per stage for the ring's place, 31.0 with three slices, 30.1 with places and sources that move on by themselves.
+//                    per stage for the ring's place, 31.0 with three slices, 30.1 with places and sources that move on by themselves, 29.0 with the ranks' sums in flight together,
+//                    27.1 with two stages a warp and six CTAs an SM in place of three and four.
 //   GemmExactKernel  the interpreter's MATMUL order (DxirInterpreter.kt:739-765): f32, k ascending, separate
 //                    multiply and add, zero activations skipped.  Bit-identical to the CPU oracle; slow.
 #include <cooperative_groups.h>
@@ -45,7 +46,6 @@ constexpr int kGvThreads = 128;
 constexpr int kGvWarps = 4;
 constexpr int kGvCols = 128;
 constexpr int kGvStageK = 32;  // k rows per pipeline stage
-constexpr int kGvStages = 3;
 constexpr int kGvWBytes = kGvStageK * kGvCols;  // the stage's weight tile
 constexpr int kGvRedStride = kGvCols + 4;
 
@@ -95,12 +95,14 @@ __device__ __forceinline__ uint32_t CodesToBf16x2(uint32_t w_lo_k, uint32_t w_hi
   return r;
 }
 
-template <int NT>
+// NT: n-tiles of eight activation rows.  S: stages of a warp.  Two are 37 KB a CTA, six an SM: where CTAs are many, more warps to hide the conversion behind are
+// worth more than a third stage (4096 x 28672 29.0 -> 27.1 us, 6144 10.5 -> 9.9); with one CTA an SM the loads in flight are (9 rows, 8192 x 1024 10.1, 10.3).
+template <int NT, int S>
 struct GvLayout {
   static constexpr int kRows = NT * 8;                     // activation rows a launch covers
   static constexpr int kXBytes = kRows * kGvStageK * 2;    // the stage's activation strip, [rows][32] bf16
   static constexpr int kStageBytes = kGvWBytes + kXBytes;
-  static constexpr int kWarpBytes = kGvStages * kStageBytes;
+  static constexpr int kWarpBytes = S * kStageBytes;
   static constexpr int kPipeBytes = kGvWarps * kWarpBytes;
   // After the loop the same space holds the four warps' partial tiles and the CTA's summed tile.
   static constexpr int kTileBytes = kRows * kGvRedStride * 4;
@@ -108,11 +110,11 @@ struct GvLayout {
   static constexpr int kBytes = kPipeBytes > kRedBytes ? kPipeBytes : kRedBytes;
 };
 
-template <int NT, typename YT>
+template <int NT, int S, typename YT>
 __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
 {
   if (!p.weights_const) GridDependencySync();
-  using L = GvLayout<NT>;
+  using L = GvLayout<NT, S>;
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
@@ -178,15 +180,15 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
   if (p.weights_const) {
     // The weights of the first stages are on their way while the previous kernel drains; the first commit group then
     // holds all of them together with the first stage's activations.
-    for (int it = 0; it < kGvStages - 1; ++it)
+    for (int it = 0; it < S - 1; ++it)
       if (it < my_n) issue_w();
     GridDependencySync();
-    for (int it = 0; it < kGvStages - 1; ++it) {
+    for (int it = 0; it < S - 1; ++it) {
       if (it < my_n) issue_x();
       CpAsyncCommit();
     }
   } else {
-    for (int it = 0; it < kGvStages - 1; ++it) {
+    for (int it = 0; it < S - 1; ++it) {
       if (it < my_n) {
         issue_w();
         issue_x();
@@ -211,12 +213,12 @@ __global__ void __launch_bounds__(kGvThreads) Int8GemvKernel(GemmParams p)
 
   uint32_t st_addr = my_pipe_addr;
   for (int it = 0; it < my_n; ++it) {
-    if (it + kGvStages - 1 < my_n) {
+    if (it + S - 1 < my_n) {
       issue_w();
       issue_x();
     }
     CpAsyncCommit();
-    CpAsyncWait<kGvStages - 1>();
+    CpAsyncWait<S - 1>();
     __syncwarp();
 #pragma unroll
     for (int h = 0; h < kGvStageK / 16; ++h) {
@@ -398,27 +400,37 @@ __global__ void __launch_bounds__(256) GemmSwigluExactKernel(const XT* x, const 
 template <int NT, typename YT>
 cudaError_t PrepareGemv()
 {
-  return cudaFuncSetAttribute(Int8GemvKernel<NT, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GvLayout<NT>::kBytes);
+  const cudaError_t e = cudaFuncSetAttribute(Int8GemvKernel<NT, 2, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GvLayout<NT, 2>::kBytes);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(Int8GemvKernel<NT, 3, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GvLayout<NT, 3>::kBytes);
 }
 
-template <int NT, typename YT>
-cudaError_t LaunchGemv(const GemmParams& p, cudaStream_t stream)
+template <int NT, int S, typename YT>
+cudaError_t LaunchGemvStages(const GemmParams& p, cudaStream_t stream)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((p.N + kGvCols - 1) / kGvCols, p.ks, 1);
   cfg.blockDim = dim3(kGvThreads, 1, 1);
-  cfg.dynamicSmemBytes = GvLayout<NT>::kBytes;
+  cfg.dynamicSmemBytes = GvLayout<NT, S>::kBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   cfg.numAttrs = ChainAttributes(attr, p.ks);
   cfg.attrs = attr;
-  return cudaLaunchKernelEx(&cfg, Int8GemvKernel<NT, YT>, p);
+  return cudaLaunchKernelEx(&cfg, Int8GemvKernel<NT, S, YT>, p);
+}
+constexpr int kSms = 148;
+template <int NT, typename YT>
+cudaError_t LaunchGemv(const GemmParams& p, cudaStream_t stream)
+{
+  const int ctas = (p.N + kGvCols - 1) / kGvCols * p.ks;
+  return ctas <= kSms ? LaunchGemvStages<NT, 3, YT>(p, stream) : LaunchGemvStages<NT, 2, YT>(p, stream);
 }
 
-// K slices for a shape, one to eight (the portable cluster sizes), each of at least one stage a warp.  What counts is how evenly the CTAs fall on the 148 SMs
-// and that there are about three an SM, so that loads in flight cover the way to HBM; more slices than that have to be worth a seventh.  Columns that are cut
+// K slices for a shape, one to eight (the portable cluster sizes; not seven, which came out slower than six and eight wherever measured), each of at least one stage a warp.  What counts is how evenly the CTAs fall on the 148 SMs
+// and that there are about three an SM, so that loads in flight cover the way to HBM, and how much of the longest slice the average one has; more slices
+// than that have to be worth a seventh.  Columns that are cut
 // evenly over all SMs instead (112 or 96 a CTA) lose more to rows of codes that start within a 128-byte line than the last wave costs.
-// Microseconds at one row with a norm in front, slices 2 / 3 / 4 of 4096 x 28672: 30.8 / 28.3 / 29.7; 4 / 5 / 6 of 5120 x 14336: 21.1 / 19.4 / 21.1.
+// Microseconds at one row with a norm in front, slices 2 / 3 / 4 of 4096 x 28672: 30.1 / 27.4 / 30.5; 4 / 5 / 6 of 5120 x 14336: 21.2 / 19.0 / 20.0;
+// 4 / 6 / 8 of 14336 x 4096: 20.9 / 19.8 / 16.5.
 // $TLALOC_B200_GEMV_KS overrides.
 int ChooseSlices(int k, int n)
 {
@@ -427,15 +439,17 @@ int ChooseSlices(int k, int n)
     return e != nullptr ? std::atoi(e) : 0;
   }();
   if (forced >= 1 && forced <= 8) return forced;
-  constexpr int kSms = 148, kWanted = 3 * kSms;
+  constexpr int kWanted = 3 * kSms;
   const int tiles = (n + kGvCols - 1) / kGvCols;
   int best = 1;
   double best_score = 0.0;
   for (int ks = 1; ks <= 8; ++ks) {
     if (ks > 1 && k / ks < kGvStageK * kGvWarps) break;
+    if (ks == 7) continue;
     const int items = tiles * ks, share = (items + kSms - 1) / kSms;
-    const double score = static_cast<double>(items) / (share * kSms) * std::min(1.0, static_cast<double>(items) / kWanted);
-    if (score > best_score * 1.15) {
+    const int unit = kGvStageK * kGvWarps, slice = ((k + ks - 1) / ks + unit - 1) / unit * unit;
+    const double score = static_cast<double>(items) / (share * kSms) * std::min(1.0, static_cast<double>(items) / kWanted) * k / (static_cast<double>(ks) * slice);
+    if (score > best_score * (tiles * best < kWanted ? 1.08 : 1.15)) {
       best_score = score;
       best = ks;
     }
