@@ -7,7 +7,10 @@
 //   GroupedAttentionMma      bf16, pages of a multiple of 16.  A CTA has one value head, up to 16 of its query heads (8 of two maps each) and one
 //                            slice, so every cached byte of the slice is read once for all of them.  Four warps, each with groups and a
 //                            ring of its own: one lane looks up the page and requests the group's boxes (64 channels x 16 rows, 128-byte
-//                            swizzle) by TMA; no CTA-wide barrier in the loop.  Query heads are the rows of mma.m16n8k16; with two maps the
+//                            swizzle) by TMA; no CTA-wide barrier in the loop.  A warp's chain of products and exponentials is what a step takes, so two
+//                            CTAs an SM are worth more than the deeper rings of one; where a group is too large for that (HALVES), its keys and values
+//                            travel on their own, and the keys' place is free again once the scores are there.  64 rows of 4 value heads, two maps of
+//                            128, values of 256 channels, up to 4160 positions: 161 us with one CTA an SM and three groups a warp, 139 with two CTAs and three halves.  Query heads are the rows of mma.m16n8k16; with two maps the
 //                            rows 0-7 are the heads' first map and 8-15 the second, each multiplied with its own keys, so that one
 //                            product with the values serves both.  The weights enter that product as two bf16 parts (f32 up to rounding).
 //   GroupedAttentionGeneric  any size and type, plain FMA: the f32 path.
@@ -26,7 +29,7 @@ using tc::MbarWait;
 using tc::MbarWaitWarp;
 using tc::SmemAddr;
 
-constexpr int kGroup = 16, kWarps = 4, kMaxStages = 4;
+constexpr int kGroup = 16, kWarps = 4, kMaxHalves = 8;
 constexpr int kAtom = kGroup * 128;  // 16 rows x 64 channels
 constexpr int kMaxSmem = 227 * 1024;
 
@@ -38,7 +41,7 @@ struct GroupedArgs {
   const int *tables, *row_tables, *lens;
   float* records;
   int64_t pool_ld;
-  int T, heads, v_heads, maps, dim, vdim, v_first, num_blocks, block_size, max_blocks, num_tables, window, keep, slices, qtiles, stages;
+  int T, heads, v_heads, maps, dim, vdim, v_first, num_blocks, block_size, max_blocks, num_tables, window, keep, slices, qtiles, halves;  // halves: places of a warp's ring, a group's keys or its values
   float scale_log2;
 };
 
@@ -100,20 +103,20 @@ __device__ __forceinline__ void Split(float a, float b, uint32_t& hi, uint32_t& 
 
 // DK, NV: 16-channel steps of a key and a value head, in whole atoms of four.  What an atom holds past its head is multiplied with zero
 // queries (keys) or left out of the result (values).
-template <int DK, int NV>
+template <int DK, int NV, bool HALVES>
 __global__ void __launch_bounds__(kWarps * 32) GroupedAttentionMma(const __grid_constant__ CUtensorMap map, const __grid_constant__ GroupedArgs a)
 {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ alignas(8) uint64_t bars[kWarps * kMaxStages];
+  __shared__ alignas(8) uint64_t bars[kWarps * kMaxHalves];
   __shared__ uint32_t abort_store;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t base = (SmemAddr(smem_raw) + 1023u) & ~1023u;
   unsigned char* smem = smem_raw + (base - SmemAddr(smem_raw));
-  const uint32_t bar = SmemAddr(bars + warp * kMaxStages);
+  const uint32_t bar = SmemAddr(bars + warp * kMaxHalves);
   volatile uint32_t* abort_word = &abort_store;
   if (tid == 0) {
     abort_store = 0u;
-    for (int i = 0; i < kWarps * kMaxStages; ++i) MbarInit(SmemAddr(bars + i), 1);
+    for (int i = 0; i < kWarps * kMaxHalves; ++i) MbarInit(SmemAddr(bars + i), 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
@@ -149,40 +152,58 @@ __global__ void __launch_bounds__(kWarps * 32) GroupedAttentionMma(const __grid_
     return;
   }
 
-  // A stage: the atoms of every map's keys, then those of the values.  x is a multiple of 16 channels: a 16-byte boundary.
+  // The ring holds keys and values of this warp's groups in turn: the atoms of every map's keys, then those of the values.  An even number of places: pairs of
+  // them (a pair on one barrier, and filled again as one, unless HALVES); an odd one: places of the larger size.  x is a multiple of 16 channels: a 16-byte
+  // boundary.
   constexpr int k_atoms = DK / 4, v_atoms = NV / 4;
-  const int stage_bytes = (a.maps * k_atoms + v_atoms) * kAtom, stages = a.stages;
-  const uint32_t ring = base + warp * stages * stage_bytes;
+  const int k_bytes = a.maps * k_atoms * kAtom, v_bytes = v_atoms * kAtom, places = HALVES ? a.halves : a.halves >> 1;
+  const bool odd = HALVES && (places & 1) != 0;
+  const int place_bytes = odd ? max(k_bytes, v_bytes) : 0, pair_bytes = k_bytes + v_bytes;
+  const uint32_t ring = base + warp * (odd ? places * place_bytes : (HALVES ? places >> 1 : places) * pair_bytes);
+  auto place = [&](int i) {
+    if constexpr (!HALVES) return ring + i * pair_bytes;
+    else return ring + (odd ? i * place_bytes : (i >> 1) * pair_bytes + (i & 1) * k_bytes);
+  };
   const int k_col = vh * a.maps * a.dim, v_col = a.v_first + vh * a.vdim;
   const int steps = (g1 - g0 - warp + kWarps - 1) / kWarps;  // this warp's groups: g0 + warp, + kWarps, ..
   auto pool_row = [&](int i) {  // of the i-th group
     const int pos = position(g0 + warp + min(i, steps - 1) * kWarps), b = pos / a.block_size;
     return min(max(__ldg(table + b), 0), a.num_blocks - 1) * a.block_size + (pos - b * a.block_size);
   };
-  auto load = [&](int row, int stage) {
-    const uint32_t bar_s = bar + 8 * stage;
-    uint32_t dst = ring + stage * stage_bytes;
-    MbarExpectTx(bar_s, stage_bytes);
-    auto box = [&](int x) {
-      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-                   "l"(reinterpret_cast<uint64_t>(&map)), "r"(x), "r"(row), "r"(bar_s)
-                   : "memory");
-      dst += kAtom;
-    };
+  auto box = [&](uint32_t dst, int x, int row, uint32_t bar_s) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(&map)), "r"(x), "r"(row), "r"(bar_s)
+                 : "memory");
+  };
+  auto load_k = [&](int row, int at) {
+    const uint32_t bar_s = bar + 8 * at;
+    uint32_t dst = place(at);
+    MbarExpectTx(bar_s, HALVES ? k_bytes : k_bytes + v_bytes);
     for (int m = 0; m < a.maps; ++m)
 #pragma unroll
-      for (int c = 0; c < k_atoms; ++c) box(k_col + m * a.dim + c * 64);
+      for (int c = 0; c < k_atoms; ++c, dst += kAtom) box(dst, k_col + m * a.dim + c * 64, row, bar_s);
+  };
+  auto load_v = [&](int row, int at) {
+    const uint32_t bar_s = bar + 8 * at, dst = place(at) + (HALVES ? 0 : k_bytes);
+    if (HALVES) MbarExpectTx(bar_s, v_bytes);
 #pragma unroll
-    for (int c = 0; c < v_atoms; ++c) box(v_col + c * 64);
+    for (int c = 0; c < v_atoms; ++c) box(dst + c * kAtom, v_col + c * 64, row, bar_s);
   };
   if (steps > 0) {
-    for (int i = 0; i < min(steps, stages); ++i) {
-      const int row = pool_row(i);
-      if (lane == 0) load(row, i);
+    for (int i = 0; i < min(HALVES ? 2 * steps : steps, places); i += HALVES ? 2 : 1) {
+      const int row = pool_row(HALVES ? i >> 1 : i);
+      if (lane == 0) {
+        load_k(row, i);
+        if (!HALVES) load_v(row, i);
+        else if (i + 1 < places) load_v(row, i + 1);
+      }
       __syncwarp();
     }
   }
-  int next_row = steps > 0 ? pool_row(stages) : 0;  // looked up ahead of its request
+  // HALVES: the place of step i's keys is the next one to fill once its scores are there, that of its values after its product: with keys (even) or values (odd)
+  // of step i + places / 2, then with that step's values or the next one's keys.  Rows are looked up a step ahead.
+  const int ahead = HALVES ? places >> 1 : places;
+  int row_a = steps > 0 ? pool_row(ahead) : 0, row_b = HALVES && steps > 0 ? pool_row(ahead + 1) : 0;
 
   // Queries as A fragments: rows lane / 4 and lane / 4 + 8.
   uint32_t qa[DK][2], qb[DK][2];
@@ -219,19 +240,28 @@ __global__ void __launch_bounds__(kWarps * 32) GroupedAttentionMma(const __grid_
     k_off[k] = word((mat >> 1) * 8 + r8, 2 * k + (mat & 1));
     v_off[k] = word((mat & 1) * 8 + r8, 2 * k + (mat >> 1));
   }
-  int stage = 0, phase = 0;
+  int at_place = 0, phase = 0;
+  auto advance = [&]() {
+    if (++at_place == places) {
+      at_place = 0;
+      phase ^= 1;
+    }
+  };
   for (int i = 0; i < steps; ++i) {
     const int pos = position(g0 + warp + i * kWarps);
-    const uint32_t kt = ring + stage * stage_bytes, vt = kt + a.maps * k_atoms * kAtom;
-    ok = MbarWaitWarp(bar + 8 * stage, phase, lane, abort_word) && ok;
-    if (pos + kGroup > len) {  // rows past the end hold whatever the page did: 0 times it must stay 0
+    const uint32_t kt = place(at_place);
+    ok = MbarWaitWarp(bar + 8 * at_place, phase, lane, abort_word) && ok;
+    // Rows past the end hold whatever the page did: 0 times it must stay 0.
+    auto blank = [&](uint32_t values) {
+      if (pos + kGroup <= len) return;
       for (int r = len - pos; r < kGroup; ++r)
         for (int c = lane; c < v_atoms * 8; c += 32) {
-          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(vt + word(r, c)), "r"(0u) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(values + word(r, c)), "r"(0u) : "memory");
         }
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
-    }
+    };
+    if constexpr (!HALVES) blank(kt + k_bytes);
     float s[2][4] = {}, u[2][4] = {};
     {
       uint32_t at[4];
@@ -258,6 +288,14 @@ __global__ void __launch_bounds__(kWarps * 32) GroupedAttentionMma(const __grid_
           Mma(acc[1], qa[k][0], qb[k][0], qa[k][1], qb[k][1], b[2], b[3]);
         }
       }
+    }
+    if constexpr (HALVES) {
+      __syncwarp();  // the keys are read before their place is filled again
+      if (lane == 0 && i + ahead < steps) {
+        if (odd) load_v(row_a, at_place);
+        else load_k(row_a, at_place);
+      }
+      advance();
     }
     const int p0 = pos + (lane & 3) * 2;
     if (pos + kGroup > len || (pos < lo && pos + kGroup > keep)) {
@@ -310,6 +348,12 @@ __global__ void __launch_bounds__(kWarps * 32) GroupedAttentionMma(const __grid_
     Split(p[0][2], p[0][3], hi[1], low[1]);
     Split(p[1][0], p[1][1], hi[2], low[2]);
     Split(p[1][2], p[1][3], hi[3], low[3]);
+    uint32_t vt = kt + k_bytes;
+    if constexpr (HALVES) {
+      vt = place(at_place);
+      ok = MbarWaitWarp(bar + 8 * at_place, phase, lane, abort_word) && ok;
+      blank(vt);
+    }
     uint32_t at[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) at[k] = vt + v_off[k];
@@ -327,22 +371,33 @@ __global__ void __launch_bounds__(kWarps * 32) GroupedAttentionMma(const __grid_
       Mma(o[2 * j + 2], low[0], low[1], low[2], low[3], d[0], d[1]);
       Mma(o[2 * j + 3], low[0], low[1], low[2], low[3], d[2], d[3]);
     }
-    __syncwarp();  // the stage is read before it is filled again
-    if (i + stages < steps) {
-      if (lane == 0) load(next_row, stage);
-      next_row = pool_row(i + stages + 1);
-    }
-    if (++stage == stages) {
-      stage = 0;
-      phase ^= 1;
+    __syncwarp();  // the values (and the keys) are read before their place is filled again
+    if constexpr (HALVES) {
+      if (lane == 0) {
+        if (odd && i + ahead + 1 < steps) load_k(row_b, at_place);
+        if (!odd && i + ahead < steps) load_v(row_a, at_place);
+      }
+      advance();
+      row_a = row_b;
+      row_b = pool_row(i + ahead + 2);
+    } else {
+      if (i + ahead < steps) {
+        if (lane == 0) {
+          load_k(row_a, at_place);
+          load_v(row_a, at_place);
+        }
+        row_a = pool_row(i + ahead + 1);
+      }
+      advance();
     }
   }
   if (!ok) {
     // Given up: let the copies in flight land before the CTA's shared memory goes away.
     if (lane == 0) {
       volatile uint32_t never = 0;
-      for (int s = 0; s < stages; ++s)
-        if (steps > s) MbarWait(bar + 8 * s, ((steps - 1 - s) / stages) & 1, &never);
+      const int loads = HALVES ? 2 * steps : steps;
+      for (int s = 0; s < places; ++s)
+        if (loads > s) MbarWait(bar + 8 * s, ((loads - 1 - s) / places) & 1, &never);
       atomicExch(&g_grouped_status, 1);
     }
     __syncwarp();
@@ -470,20 +525,28 @@ __global__ void __launch_bounds__(kGenericThreads) GroupedAttentionGeneric(const
   }
 }
 
-// Stages of a warp's ring that fit beside the alignment slack; 0: none.
-int Stages(int maps, int dim, int vdim, size_t* smem)
+// Places (keys or values of a group) of a warp's ring; *smem what they take, *split whether keys and values travel on their own.  Groups of up to 8 KB: three of them,
+// and two CTAs an SM.  Larger ones in a grid of more CTAs than SMs (`many`): halves of two groups (up to 12 KB, 161 -> 139 us and the like) or three halves, if two CTAs then
+// fit an SM; 14 KB (128 + 128 + 192 channels) are better off with the four groups of one CTA (52.7 us, 61.2 in halves).  Else as many groups as one CTA has room for.
+int Halves(int maps, int dim, int vdim, bool many, size_t* smem, bool* split)
 {
-  const size_t stage = static_cast<size_t>(maps * ((dim + 63) / 64) + (vdim + 63) / 64) * kAtom;
+  const size_t keys = static_cast<size_t>(maps) * ((dim + 63) / 64) * kAtom, values = static_cast<size_t>((vdim + 63) / 64) * kAtom;
   const size_t merge = sizeof(float) * (kWarps * 32 + static_cast<size_t>(kWarps) * 16 * (vdim + 4));
-  int n = stage <= 8192 ? 3 : kMaxStages;  // small stages: two CTAs per SM
-  while (n > 0 && kWarps * n * stage + 1024 > kMaxSmem - 1024) --n;
-  if (smem != nullptr) *smem = (kWarps * n * stage > merge ? kWarps * n * stage : merge) + 1024;
+  constexpr size_t kHalfSm = 112 * 1024;  // dynamic shared memory of each of two CTAs, beside what each declares and the system keeps
+  auto ring = [&](int n) { return kWarps * (n % 2 != 0 ? n * (keys > values ? keys : values) : n / 2 * (keys + values)) + 1024; };
+  const int halves = keys + values > 8192 && merge + 1024 <= kHalfSm ? ring(4) <= kHalfSm ? 4 : keys == values && ring(3) <= kHalfSm ? 3 : 0 : 0;
+  *split = many && halves > 0;
+  int n = *split ? halves : keys + values <= 8192 ? 6 : kMaxHalves;
+  while (n > 0 && ring(n) > kMaxSmem - 1024) n -= 2;
+  *smem = ring(n) > merge + 1024 ? ring(n) : merge + 1024;
   return n;
 }
 bool MmaApplies(int maps, int dim, int vdim, int block_size, int dtype)
 {
+  size_t smem;
+  bool split;
   return dtype == TLALOC_B200_BF16 && (maps == 1 || maps == 2) && dim % 16 == 0 && vdim % 16 == 0 && dim <= 128 && vdim <= 256 && block_size % kGroup == 0 &&
-         Stages(maps, dim, vdim, nullptr) >= 2 && !OrderFaithful() && TensorMapEncoder() != nullptr;
+         Halves(maps, dim, vdim, false, &smem, &split) >= 4 && !OrderFaithful() && TensorMapEncoder() != nullptr;
 }
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -515,7 +578,8 @@ cudaError_t PrepareGrouped()
     TensorMapEncoder();
     cudaError_t e = cudaSuccess;
 #define TLALOC_OPT_IN(DK, NV) \
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(GroupedAttentionMma<DK, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - 1024);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(GroupedAttentionMma<DK, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - 1024); \
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(GroupedAttentionMma<DK, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - 1024);
     TLALOC_GROUPED_SIZES(TLALOC_OPT_IN)
 #undef TLALOC_OPT_IN
     return e;
@@ -603,12 +667,15 @@ extern "C" int tlaloc_b200_grouped_attention(const void* q, const void* pool, in
       return Fail(kInternal, "%s: the tensor map could not be encoded", op);
     }
     size_t smem = 0;
-    a.stages = Stages(maps, dim, vdim, &smem);
+    bool split = false;
     const dim3 grid(slices, v_heads * a.qtiles, num_tokens);
+    a.halves = Halves(maps, dim, vdim, static_cast<long long>(slices) * grid.y * num_tokens > 148, &smem, &split);
     const int dk = (dim + 63) / 64 * 4, nv = (vdim + 63) / 64 * 4;
     e = cudaErrorInvalidValue;
 #define TLALOC_LAUNCH(DK, NV) \
-  if (dk == DK && nv == NV) e = LaunchChained(GroupedAttentionMma<DK, NV>, grid, kWarps * 32, smem, st, map, a);
+  if (dk == DK && nv == NV)                                                                                              \
+    e = split ? LaunchChained(GroupedAttentionMma<DK, NV, true>, grid, kWarps * 32, smem, st, map, a)                    \
+              : LaunchChained(GroupedAttentionMma<DK, NV, false>, grid, kWarps * 32, smem, st, map, a);
     TLALOC_GROUPED_SIZES(TLALOC_LAUNCH)
 #undef TLALOC_LAUNCH
   } else {
