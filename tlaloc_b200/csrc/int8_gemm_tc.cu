@@ -427,8 +427,13 @@ void FillTcSlots(int device, int cls)
 
 // K slices (1..8) of a launch: the count with the lowest modelled time, in units of one 64-row block of one CTA:
 //   waves(ks) * (blocks per slice + fixed cost of a CTA [+ cost of the cluster reduction])
-// with waves = ceil(column tiles * ks / resident CTAs).  The constants come from timing the kernel at one full wave
-// over a range of K (fixed cost ~10 blocks) and from the reduction's traffic.  $TLALOC_B200_GEMM_KS overrides.
+// with waves = ceil(column tiles * ks / resident CTAs).  The constants come from timing the kernel at one full wave:
+// 40 rows x 4096 columns with k 14336 and 4096 take 100.9 and 31.6 us in one slice (0.43 us a block, 3.9 us fixed), 56.5
+// and 20.6 in two, 32.8 and 13.9 in four, 25.2 and 11.8 in six: the reduction adds the same with any number of slices.  It is
+// charged eight blocks, what it costs where 128 rows and more than 100 CTAs share the way (100 x 1024 x 14336: 13.6 us in one slice, 16.0 in two;
+// 100 x 1024 x 8192: 13.5 in one, 13.2 in four).  A charge that grew with the slices stayed below the best count: 40 x 1024 x 1024 11.4 us
+// in one slice, 8.2 in four; 40 x 2048 x 2048 10.2 in four, 8.2 in eight; 40 x 4096 x 4096 12.8 in five, 11.7 in six.
+// $TLALOC_B200_GEMM_KS overrides.
 int ChooseTcSlices(int k, int n, int mpad, double* cost_out = nullptr)
 {
   static const int forced = [] {
@@ -451,7 +456,7 @@ int ChooseTcSlices(int k, int n, int mpad, double* cost_out = nullptr)
     if (ks > 1 && nb / ks < 4) break;
     const int slots = g_tc_slots[device][cls][ks] > 0 ? g_tc_slots[device][cls][ks] : 148 / ks * ks;
     const int waves = (tiles * ks + slots - 1) / slots;
-    const double per_cta = (nb + ks - 1) / ks + 10.0 + (ks > 1 ? 8.0 + 1.5 * ks : 0.0);
+    const double per_cta = (nb + ks - 1) / ks + 10.0 + (ks > 1 ? 8.0 : 0.0);
     const double cost = waves * per_cta;
     if (cost < best_cost * 0.97) {  // prefer fewer slices unless the gain is real
       best_cost = cost;
@@ -512,11 +517,12 @@ cudaError_t LaunchInt8GemmTc(const __nv_bfloat16* x, const int8_t* codes, const 
     int rows = std::min(256, m - m0);
     if (rows > 128) {
       // Two accumulators share one pass over the weights but cannot split K; with few column tiles two passes of 128
-      // rows, each split over K, keep more SMs busy.
+      // rows, each split over K, keep more SMs busy.  A launch more is five blocks beside what a CTA's fixed cost says (200 rows x 1024 x 4096: 20.4 us
+      // in one pass, 23.5 in two of four slices; x 2048 x 4096: 24 in two).
       double c256 = 0.0, c128 = 0.0;
       ChooseTcSlices(k, n, 128, &c128);
       ChooseTcSlices(k, n, 256, &c256);
-      if (2.0 * c128 < c256) rows = 128;
+      if (2.0 * (c128 + 5.0) < c256) rows = 128;
     }
     const int mpad = rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256;
     p.ks = ChooseTcSlices(k, n, mpad);
