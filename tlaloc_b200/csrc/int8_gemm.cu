@@ -97,6 +97,8 @@ __device__ __forceinline__ uint32_t CodesToBf16x2(uint32_t w_lo_k, uint32_t w_hi
 
 // NT: n-tiles of eight activation rows.  S: stages of a warp.  Two are 37 KB a CTA, six an SM: where CTAs are many, more warps to hide the conversion behind are
 // worth more than a third stage (4096 x 28672 29.0 -> 27.1 us, 6144 10.5 -> 9.9); with one CTA an SM the loads in flight are (9 rows, 8192 x 1024 10.1, 10.3).
+// With 9 rows and more a stage's MMAs and strip are twice as many and three stages are better again (three layers of 6144 + 4096 + 28672 x 4096, 4096 x 14336 and a head,
+// 9, 12 and 16 rows: 359, 353, 376 us with two, 340, 343, 358 with three), but for short slices whose CTAs would then take a second wave (16 rows, 2048 x 8192 in eight slices: 11.7 and 17.4).
 template <int NT, int S>
 struct GvLayout {
   static constexpr int kRows = NT * 8;                     // activation rows a launch covers
@@ -422,7 +424,8 @@ template <int NT, typename YT>
 cudaError_t LaunchGemv(const GemmParams& p, cudaStream_t stream)
 {
   const int ctas = (p.N + kGvCols - 1) / kGvCols * p.ks;
-  return ctas <= kSms ? LaunchGemvStages<NT, 3, YT>(p, stream) : LaunchGemvStages<NT, 2, YT>(p, stream);
+  const int length = ((p.K + p.ks - 1) / p.ks + kGvStageK * kGvWarps - 1) / (kGvStageK * kGvWarps);  // stages of a warp's way through its slice
+  return ctas <= kSms || (NT > 1 && (ctas <= 3 * kSms || length >= 8)) ? LaunchGemvStages<NT, 3, YT>(p, stream) : LaunchGemvStages<NT, 2, YT>(p, stream);
 }
 
 // K slices for a shape, one to eight (the portable cluster sizes; not seven, which came out slower than six and eight wherever measured), each of at least one stage a warp.  What counts is how evenly the CTAs fall on the 148 SMs
