@@ -1,0 +1,30 @@
+"""What the Python layer refuses before a kernel is launched.  The library is a stand-in that counts calls: nothing here needs a GPU."""
+import pytest
+import torch
+
+from tlaloc_b200 import ops
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """The C functions that were called."""
+    seen = []
+
+    class Library:
+        def __getattr__(self, name):
+            return lambda *args: seen.append(name) or 0
+
+    monkeypatch.setattr(ops.N, "lib", lambda: Library())
+    return seen
+
+
+def test_rows_on_the_host_are_refused(calls, monkeypatch):
+    """latent_kv_write has no other look at where its rows lie than the stream of their device."""
+    monkeypatch.setattr(ops, "_dev", lambda *ts: None)  # the other operands are on the device
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 0, raising=False)
+    monkeypatch.setattr(ops, "_current_raw_stream", lambda device: 0, raising=False)
+    i32 = dict(dtype=torch.int32)
+    low, pool, table = torch.zeros(2, 12), torch.zeros(1, 16, 12), torch.zeros(3, 2)
+    with pytest.raises(ValueError, match="CUDA"):
+        ops.latent_kv_write(low, None, torch.ones(8), 1e-5, torch.zeros(2, **i32), table, table, torch.zeros(2, **i32), None, pool, q_rank=0, kv_rank=8, rot_dim=4, rot_dims=4)
+    assert calls == []

@@ -51,7 +51,10 @@ def _ptr(t):
 def _stream(t: torch.Tensor) -> int:
     """The current stream of the tensor's own device (not of whichever device happens to be current).  The handle alone: making a Stream
     object of it takes 4 us, more than a launch."""
-    return _current_raw_stream(t.get_device())
+    device = t.get_device()
+    if device < 0:  # the handle's getter takes it for "the current device", and the kernel would read a host address
+        raise ValueError(f"a CUDA tensor is needed, got one on {t.device}")
+    return _current_raw_stream(device)
 
 
 def init() -> None:
