@@ -1,4 +1,7 @@
 """What the Python layer refuses before a kernel is launched.  The library is a stand-in that counts calls: nothing here needs a GPU."""
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -22,9 +25,14 @@ def test_rows_on_the_host_are_refused(calls, monkeypatch):
     """latent_kv_write has no other look at where its rows lie than the stream of their device."""
     monkeypatch.setattr(ops, "_dev", lambda *ts: None)  # the other operands are on the device
     monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 0, raising=False)
-    monkeypatch.setattr(ops, "_current_raw_stream", lambda device: 0, raising=False)
     i32 = dict(dtype=torch.int32)
     low, pool, table = torch.zeros(2, 12), torch.zeros(1, 16, 12), torch.zeros(3, 2)
     with pytest.raises(ValueError, match="CUDA"):
         ops.latent_kv_write(low, None, torch.ones(8), 1e-5, torch.zeros(2, **i32), table, table, torch.zeros(2, **i32), None, pool, q_rank=0, kv_rank=8, rot_dim=4, rot_dims=4)
     assert calls == []
+
+
+def test_a_torch_without_cuda_imports_the_operators():
+    program = "import torch; del torch._C._cuda_getCurrentRawStream; import tlaloc_b200.ops, tlaloc_b200.decoder, tlaloc_b200.latent_decoder, tlaloc_b200.mixed_decoder"
+    done = subprocess.run([sys.executable, "-c", program], capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr

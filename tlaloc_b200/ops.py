@@ -13,7 +13,6 @@ import torch
 from . import _native as N
 from .attrs import PagedAttentionShape, parse_paged_attention
 
-_current_raw_stream = torch._C._cuda_getCurrentRawStream
 _DT = {torch.float32: N.F32, torch.bfloat16: N.BF16, torch.int8: N.S8, torch.int32: N.S32, torch.float8_e4m3fn: N.F8E4M3FN}
 
 
@@ -54,7 +53,7 @@ def _stream(t: torch.Tensor) -> int:
     device = t.get_device()
     if device < 0:  # the handle's getter takes it for "the current device", and the kernel would read a host address
         raise ValueError(f"a CUDA tensor is needed, got one on {t.device}")
-    return _current_raw_stream(device)
+    return torch._C._cuda_getCurrentRawStream(device)  # looked up here: a torch without CUDA does not have it, and imports this module
 
 
 def init() -> None:
