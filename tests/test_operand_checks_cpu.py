@@ -36,3 +36,20 @@ def test_a_torch_without_cuda_imports_the_operators():
     program = "import torch; del torch._C._cuda_getCurrentRawStream; import tlaloc_b200.ops, tlaloc_b200.decoder, tlaloc_b200.latent_decoder, tlaloc_b200.mixed_decoder"
     done = subprocess.run([sys.executable, "-c", program], capture_output=True, text=True)
     assert done.returncode == 0, done.stderr
+
+
+def on_the_device(*shape):
+    """A tensor that says it is on a CUDA device."""
+    class Tensor(torch.Tensor):
+        is_cuda = True
+
+    return torch.zeros(shape).as_subclass(Tensor)
+
+
+@pytest.mark.parametrize("name", ["x", "out", "residual"])
+@pytest.mark.parametrize("shape", [(), (4,), (1, 2, 4)])
+def test_a_projection_names_the_operand_of_another_rank(calls, name, shape):
+    operands = {n: on_the_device(2, 4) for n in ("x", "out", "residual")}
+    operands[name] = on_the_device(*shape)
+    with pytest.raises(ValueError, match=f"DENSE_PROJ {name}: a CUDA tensor of rank 2"):
+        ops.dense(operands["x"], on_the_device(4, 4), operands["out"], residual=operands["residual"])

@@ -278,10 +278,11 @@ def dense(x, w, out, *, bias=None, residual=None, act=N.ACT_NONE) -> N.DenseProb
     rank = len(ws)
     batched = rank == 3
     b, n, k = ws if batched else (1, *ws)
-    m, x_ld, out_ld = xs[-2], x.stride(), out.stride()
+    x_ld, out_ld = x.stride(), out.stride()
     for name, t, ld in (("x", x, x_ld), ("out", out, out_ld)) + ((("residual", residual, residual.stride()),) if residual is not None else ()):
-        if not t.is_cuda or ld[-1] != 1 or len(ld) != rank:
+        if not t.is_cuda or len(ld) != rank or ld[-1] != 1:
             raise ValueError(f"DENSE_PROJ {name}: a CUDA tensor of rank {rank} with a dense last dimension is needed")
+    m = xs[-2]
     _dev(w, bias)
     if xs[-1] != k or os[-2] != m or os[-1] != (n // 2 if act in GATED else n) or (batched and (xs[0] != b or os[0] != b)) or x.dtype != w.dtype:
         raise ValueError(f"DENSE_PROJ: x {tuple(x.shape)} {x.dtype}, w {tuple(w.shape)} {w.dtype}, out {tuple(out.shape)} do not fit")
