@@ -1,4 +1,5 @@
 """What the Python layer refuses before a kernel is launched.  The library is a stand-in that counts calls: nothing here needs a GPU."""
+import dataclasses
 import subprocess
 import sys
 
@@ -6,6 +7,7 @@ import pytest
 import torch
 
 from tlaloc_b200 import ops
+from tlaloc_b200.attrs import PagedAttentionShape, parse_paged_attention
 
 
 @pytest.fixture
@@ -53,3 +55,23 @@ def test_a_projection_names_the_operand_of_another_rank(calls, name, shape):
     operands[name] = on_the_device(*shape)
     with pytest.raises(ValueError, match=f"DENSE_PROJ {name}: a CUDA tensor of rank 2"):
         ops.dense(operands["x"], on_the_device(4, 4), operands["out"], residual=operands["residual"])
+
+
+def test_a_parsed_shape_comes_out_of_its_constructor(monkeypatch):
+    """All fields, in the constructor's hands: what it does not know is an error and not an attribute that is missing later."""
+    names = [f.name for f in dataclasses.fields(PagedAttentionShape)]
+    values = dict(zip(names, range(1, len(names) + 1)))
+    assert vars(PagedAttentionShape(*values.values())) == vars(PagedAttentionShape(**values)) == values
+    required = {f.name: 1 for f in dataclasses.fields(PagedAttentionShape) if f.default is dataclasses.MISSING}
+    assert vars(PagedAttentionShape(**required)) == {f.name: 1 if f.default is dataclasses.MISSING else f.default for f in dataclasses.fields(PagedAttentionShape)}
+    with pytest.raises(TypeError):
+        PagedAttentionShape(**values, block_table=1)
+    with pytest.raises(dataclasses.FrozenInstanceError):
+        PagedAttentionShape(**values).scale = 2.0
+    made = []
+    original = PagedAttentionShape.__init__
+    monkeypatch.setattr(PagedAttentionShape, "__init__", lambda self, *args, **kw: made.append(self) or original(self, *args, **kw))
+    i32 = dict(dtype=torch.int32)
+    parsed = parse_paged_attention(torch.zeros(4, 8, 16), torch.zeros(5, 2, 2, 16), torch.zeros(5, 2, 2, 16), torch.zeros(2, 6, **i32), torch.zeros(4, **i32), scale=0.25,
+                                   sliding_window=3, keep=torch.zeros(4, 4, **i32))
+    assert made == [parsed] and parsed == PagedAttentionShape(4, 8, 16, 5, 2, 2, 6, 0.25, 3, 2, 3, False)

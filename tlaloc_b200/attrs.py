@@ -14,7 +14,7 @@ from dataclasses import dataclass
 FORBIDDEN_ATTRS = ("block_size", "blockSize", "num_kv_heads", "numKvHeads")
 
 
-@dataclass(frozen=True)
+@dataclass(frozen=True, init=False)
 class PagedAttentionShape:
     """``PagedAttentionAttrs.Parsed`` (:79-138): every field derived or checked."""
 
@@ -30,6 +30,13 @@ class PagedAttentionShape:
     num_tables: int | None = None
     keep_chunk: int | None = None
     return_lse: bool = False
+
+    def __init__(self, num_seqs, num_heads, head_dim, num_blocks, block_size, num_kv_heads, max_blocks_per_seq, scale,
+                 sliding_window=None, num_tables=None, keep_chunk=None, return_lse=False):
+        # one update for all fields: the constructor that a frozen class gets sets them one by one, half a microsecond of each call
+        self.__dict__.update(num_seqs=num_seqs, num_heads=num_heads, head_dim=head_dim, num_blocks=num_blocks, block_size=block_size,
+                             num_kv_heads=num_kv_heads, max_blocks_per_seq=max_blocks_per_seq, scale=scale, sliding_window=sliding_window,
+                             num_tables=num_tables, keep_chunk=keep_chunk, return_lse=return_lse)
 
     @property
     def rows_per_table(self) -> int:
@@ -119,9 +126,5 @@ def parse_paged_attention(query, key_cache, value_cache, block_tables, seq_lens,
         if kt[1] < 1 or ctx % kt[1] != 0:
             raise ValueError(f"{layer}: PAGED_ATTENTION keep has {kt[1]} chunks, which do not divide the {ctx} positions")
         keep_chunk = ctx // kt[1]
-    # every field is checked by now; the frozen class's own constructor sets them one by one, 3 us of a 25 us call
-    out = object.__new__(PagedAttentionShape)
-    out.__dict__.update(num_seqs=num_seqs, num_heads=num_heads, head_dim=head_dim, num_blocks=num_blocks, block_size=block_size,
-                        num_kv_heads=num_kv_heads, max_blocks_per_seq=max_blocks, scale=float(scale), sliding_window=window,
-                        num_tables=num_tables, keep_chunk=keep_chunk, return_lse=bool(return_lse))
-    return out
+    return PagedAttentionShape(num_seqs, num_heads, head_dim, num_blocks, block_size, num_kv_heads, max_blocks,
+                               float(scale), window, num_tables, keep_chunk, bool(return_lse))
