@@ -50,6 +50,7 @@ struct PaParams {
   int R, H, Hkv, D, bs, M, Tb, P;
   int S;      // context slices in use
   int slice;  // positions per slice
+  int grid;   // slices of a table that are launched: S, or fewer from the window's first on (FirstSlice)
   int group, rpt, NQ;
   int window, keep_chunks, keep_chunk;
   int bs_shift;  // log2(bs) when bs is a power of two, else -1
@@ -57,6 +58,15 @@ struct PaParams {
 };
 
 __device__ __forceinline__ int ClampI(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
+
+// The slice of a CTA.  Where a table has one row and a window, only as many CTAs are launched as the window can touch slices, counted from the first it
+// touches: CTAs without a live position cost about 1 ns each, and a window of 1000 in tables of 64000 positions (32 rows, 8 KV heads, e4m3fn) leaves 249 of 250 slices of 256
+// positions without: 94 us with all of them.
+__device__ __forceinline__ int SliceOfCta(const PaParams& p, int table)
+{
+  if (p.grid == p.S) return blockIdx.x;
+  return max(0, ClampI(__ldg(p.lens + table), 0, p.M * p.bs) - p.window) / p.slice + blockIdx.x;
+}
 
 __device__ __forceinline__ bool Kept(const PaParams& p, int row, int pos)
 {
@@ -86,7 +96,7 @@ __global__ void __launch_bounds__(kGenThreads) PaSliceGeneric(PaParams p)
   __shared__ float m_s[kGenQ], l_s[kGenQ], alpha_s[kGenQ];
   __shared__ int len_s[kGenQ], first_s[kGenQ], row_s[kGenQ], head_s[kGenQ];
 
-  const int s = blockIdx.x, kv = blockIdx.y, tb = blockIdx.z;
+  const int kv = blockIdx.y, tb = blockIdx.z, s = SliceOfCta(p, tb);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int D = p.D, ctx = p.M * p.bs;
   const int c0 = s * p.slice;
@@ -339,7 +349,7 @@ __device__ __forceinline__ void PaSliceMmaBody(const PaParams& p, const CUtensor
   __shared__ __align__(8) unsigned long long tile_bars[kMmaWarps * NS];
   __shared__ uint32_t abort_word;
 
-  const int s = blockIdx.x, kv = blockIdx.y, tb = blockIdx.z;
+  const int kv = blockIdx.y, tb = blockIdx.z, s = SliceOfCta(p, tb);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
   const int ctx = p.M * p.bs;
@@ -751,7 +761,7 @@ __device__ __forceinline__ void PaSliceMmaF8Body(const PaParams& p, const CUtens
   __shared__ __align__(8) unsigned long long tile_bars[kMmaWarps * NS];
   __shared__ uint32_t abort_word;
 
-  const int s = blockIdx.x, kv = blockIdx.y, tb = blockIdx.z;
+  const int kv = blockIdx.y, tb = blockIdx.z, s = SliceOfCta(p, tb);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
   const int ctx = p.M * p.bs;
@@ -1358,7 +1368,7 @@ template <typename QT, int D, int NS>
 cudaError_t LaunchMmaNs(const PaParams& p, cudaStream_t stream)
 {
   const size_t smem = MmaLayout<D, NS>::Bytes(p.slice / p.bs + 2);
-  const dim3 grid(p.S, p.Hkv, p.Tb);
+  const dim3 grid(p.grid, p.Hkv, p.Tb);
   if (p.NQ <= 8) return LaunchChained(PaSliceMma<QT, D, NS, 1>, grid, kMmaThreads, smem, stream, p);
   return LaunchChained(PaSliceMma<QT, D, NS, 2>, grid, kMmaThreads, smem, stream, p);
 }
@@ -1395,7 +1405,7 @@ bool LaunchTma(const PaParams& p, cudaStream_t stream, cudaError_t* err)
   if (!EncodeKvPoolMap(&map_k, p.kc, D, p.Hkv, positions, 2) || !EncodeKvPoolMap(&map_v, p.vc, D, p.Hkv, positions, 2)) return false;
   const size_t smem = MmaLayout<D, 2>::Bytes(p.slice / p.bs + 2);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.S, p.Hkv, p.Tb);
+  cfg.gridDim = dim3(p.grid, p.Hkv, p.Tb);
   cfg.blockDim = dim3(kMmaThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -1454,7 +1464,7 @@ template <typename QT, int D, int NS>
 cudaError_t LaunchMmaF8Ns(const PaParams& p, cudaStream_t stream)
 {
   const size_t smem = MmaLayoutF8<D, NS>::Bytes(p.slice / p.bs + 2);
-  const dim3 grid(p.S, p.Hkv, p.Tb);
+  const dim3 grid(p.grid, p.Hkv, p.Tb);
   if (MmaTmaEnabled() && p.bs_shift >= 4) {  // a group of 16 positions lies inside one block: the tiles come as TMA boxes
     CUtensorMap map_k, map_v;
     const unsigned long long positions = static_cast<unsigned long long>(p.P) * p.bs;
@@ -1488,7 +1498,7 @@ template <typename QT, typename KVT>
 cudaError_t LaunchGeneric(const PaParams& p, cudaStream_t stream)
 {
   const size_t smem = sizeof(float) * (kGenQ * p.D + kGenQ * kGenTile) + sizeof(long long) * kGenTile;
-  return LaunchChained(PaSliceGeneric<QT, KVT>, dim3(p.S, p.Hkv, p.Tb), kGenThreads, smem, stream, p);
+  return LaunchChained(PaSliceGeneric<QT, KVT>, dim3(p.grid, p.Hkv, p.Tb), kGenThreads, smem, stream, p);
 }
 
 // Positions per slice of the tensor-core kernels when the scratch allows it, for `pairs` (table, KV head) pairs that see up to `seen` positions each;
@@ -1657,7 +1667,7 @@ extern "C" int tlaloc_b200_paged_attention(const void* query, int32_t q_dtype, c
       return Fail(kUnsupported, "%s: parity mode holds a row's scores on chip, at most %d positions (got %d)", op, kFaithfulMaxCtx, span);
     }
     p.slice = ctx;
-    p.S = 1;
+    p.S = p.grid = 1;
     cudaError_t fe;
     if (q_dtype == TLALOC_B200_F32 && kv_dtype == TLALOC_B200_F32) fe = LaunchFaithful<float, float>(p, out_dtype, span, st);
     else if (q_dtype == TLALOC_B200_F32 && kv_dtype == TLALOC_B200_BF16) fe = LaunchFaithful<float, __nv_bfloat16>(p, out_dtype, span, st);
@@ -1680,7 +1690,8 @@ extern "C" int tlaloc_b200_paged_attention(const void* query, int32_t q_dtype, c
   const bool mma = (kv_dtype == TLALOC_B200_BF16 || (f8 && !f8_generic)) && (head_dim == 64 || head_dim == 128) && p.NQ <= kMmaQ &&
                    keep == nullptr && (f8 ? block_size >= 16 : block_size >= 8) && Aligned16(key_cache) && Aligned16(value_cache);
   // Slice length: the preferred one (tensor-core kernel) or 256, stretched until `splits` slices cover the context.
-  const int seen = sliding_window > 0 ? std::min(sliding_window, ctx) : ctx;
+  const bool from_window = sliding_window > 0 && sliding_window < ctx && p.rpt == 1;  // rows that share a table have windows in different places: all slices are launched for them
+  const int seen = from_window ? sliding_window : ctx;
   int slice = mma ? PreferredSlice(seen, static_cast<long long>(num_tables) * num_kv_heads, f8) : 256;
   if (static_cast<int64_t>(slice) * splits < ctx) slice = (ctx + splits - 1) / splits;
   if (mma) slice = std::min((slice + 15) / 16 * 16, 8192);
@@ -1689,6 +1700,7 @@ extern "C" int tlaloc_b200_paged_attention(const void* query, int32_t q_dtype, c
   }
   p.slice = slice;
   p.S = (ctx + slice - 1) / slice;
+  p.grid = from_window ? std::min(p.S, (sliding_window + slice - 2) / slice + 1) : p.S;
 
   cudaError_t e = cudaSuccess;
   if (mma) {
