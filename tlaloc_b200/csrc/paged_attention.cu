@@ -50,7 +50,7 @@ struct PaParams {
   int R, H, Hkv, D, bs, M, Tb, P;
   int S;      // context slices in use
   int slice;  // positions per slice
-  int grid;   // slices of a table that are launched: S, or fewer from the window's first on (FirstSlice)
+  int grid;   // slices of a table that are launched: S, or fewer from the window's first on (SliceOfCta)
   int group, rpt, NQ;
   int window, keep_chunks, keep_chunk;
   int bs_shift;  // log2(bs) when bs is a power of two, else -1
@@ -1501,7 +1501,8 @@ cudaError_t LaunchGeneric(const PaParams& p, cudaStream_t stream)
   return LaunchChained(PaSliceGeneric<QT, KVT>, dim3(p.grid, p.Hkv, p.Tb), kGenThreads, smem, stream, p);
 }
 
-// Positions per slice of the tensor-core kernels when the scratch allows it, for `pairs` (table, KV head) pairs that see up to `seen` positions each;
+// Positions per slice of the tensor-core kernels when the scratch allows it, for `pairs` (table, KV head) pairs that see up to `seen` positions each, from the first
+// on or (from_window) from anywhere, which takes a slice more;
 // $TLALOC_B200_PA_SLICE overrides.
 // A CTA pays about 3 us of latency before its first position (lengths and table entries, then the first K/V rows)
 // and again to merge its warps and write its records, so slices should be as long as the grid can afford: 1024
@@ -1510,10 +1511,15 @@ cudaError_t LaunchGeneric(const PaParams& p, cudaStream_t stream)
 // contexts up to 16K): 0.718 -> 0.670 -> 0.661 ms per layer at 1024 / 2048 / 4096; 512 pairs: 382 / 374 / 372 us; 256
 // pairs: 203 / 200 / 222 us; 500 pairs of 64 channels 190 / 188 / 216; 128 pairs (one KV head per rank): 117 / 128 us.
 // e4m3fn rows are half as long and their CTAs (592 resident) wait less for memory than for their conversions, so an uneven last wave costs more: 320 pairs
-// at up to 16K 94 / 124 / 150 us, 500 pairs 139 / 158 / 199, 1024 pairs 435 / 408 / 422.
-// Few pairs, lengths spread up to the context, at 256 / 512 / 1024 us: 8 pairs of 16000 e4m3fn 9.4 / 11.9 / 17.2; 64 pairs of 2000 bf16 16.7 / 16.7 / 20.0, of 4000
-// 24.7 / 21.2 / 22.9, of 4000 e4m3fn 19.4 / 22.7 / 21.7; 256 pairs of 1000 e4m3fn 15.8 / 13.7 / 15.9.
-int PreferredSlice(int seen, long long pairs, bool f8)
+// at up to 16K 94 / 124 / 150 us, 500 pairs 139 / 158 / 199, 1024 pairs 435 / 408 / 422.  (Where tables are ten times as wide as the lengths need, those pools
+// would rather have the longer slices: 512 pairs of 700 positions in tables of 11264 29.2 / 26.6 / 24.8, and 128 pairs of 60000 215 / 200 / 194.)
+// Halving pays where it fills the wave; microseconds at 256 / 512 / 1024, lengths spread up to the context:
+//   few pairs       8 pairs of 4000 11.4 / 12.7 / 17.8; 64 of 2000 14.5 / 15.0 / 18.8, of 4000 24.5 / 20.0 / 22.0
+//   48 slices       the merge walks a row's records in one warp, eight at a time: one row of 16000 with 8 KV heads 28.8 / 20.5 / 20.5, of 60000 with one KV head 41.0 / 27.2 / 25.1
+//   past the wave   a second one has to be short and full: 16 pairs of 8191 22.6 / 18.1 / 19.0, of 16000 38.4 / 35.0 / 27.9; e4m3fn rather has it, 64 pairs of 8191 31.3 / 25.0 / 33.4,
+//                   but not for a remainder: 500 pairs of 701 17.8 / 21.8 / 17.0
+//   short contexts  a slice of 512 or less is hardly shorter by halves: 256 pairs of 300 14.0 / 12.9 / 13.1; with an SM for every CTA all the same, 8 pairs 8.7 / 9.4 / 9.4
+int PreferredSlice(int seen, bool from_window, long long pairs, bool f8)
 {
   static const int forced = [] {
     const char* e = std::getenv("TLALOC_B200_PA_SLICE");
@@ -1522,9 +1528,17 @@ int PreferredSlice(int seen, long long pairs, bool f8)
   }();
   if (forced > 0) return forced;
   int slice = 1024;
-  auto ctas = [&](int length) { return pairs * ((seen + length - 1) / length); };
+  const int wave = f8 ? 592 : 444;
+  auto count = [&](int length) { return from_window ? (seen + length - 2) / length + 1 : (seen + length - 1) / length; };
+  auto ctas = [&](int length) { return pairs * count(length); };
+  auto worth_halving = [&](int half) {
+    if (count(half) > 48) return false;
+    if (seen <= 512 && ctas(half) > 148) return false;
+    if (8 * ctas(half) <= 9 * wave) return true;
+    return (f8 || count(half) <= 8) && 4ll * count(half) * half <= 5ll * seen;
+  };
   while (slice < 4096 && ctas(2 * slice) >= (f8 ? 5000 : 2048)) slice *= 2;
-  while (slice > 256 && ctas(slice) < (f8 ? 592 : 444)) slice /= 2;
+  while (slice > 256 && ctas(slice) < wave && worth_halving(slice / 2)) slice /= 2;
   return slice;
 }
 
@@ -1692,7 +1706,7 @@ extern "C" int tlaloc_b200_paged_attention(const void* query, int32_t q_dtype, c
   // Slice length: the preferred one (tensor-core kernel) or 256, stretched until `splits` slices cover the context.
   const bool from_window = sliding_window > 0 && sliding_window < ctx && p.rpt == 1;  // rows that share a table have windows in different places: all slices are launched for them
   const int seen = from_window ? sliding_window : ctx;
-  int slice = mma ? PreferredSlice(seen, static_cast<long long>(num_tables) * num_kv_heads, f8) : 256;
+  int slice = mma ? PreferredSlice(seen, from_window, static_cast<long long>(num_tables) * num_kv_heads, f8) : 256;
   if (static_cast<int64_t>(slice) * splits < ctx) slice = (ctx + splits - 1) / splits;
   if (mma) slice = std::min((slice + 15) / 16 * 16, 8192);
   if (static_cast<int64_t>(slice) * splits < ctx) {
