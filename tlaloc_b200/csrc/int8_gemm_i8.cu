@@ -86,8 +86,9 @@ __device__ __forceinline__ float AsBf16Value<float>(float v) { return __bfloat16
 
 // One CTA per row: the row's largest magnitude, the power-of-two step s, then q = x / s (exact: a power of two) rounded
 // to the nearest integer and split as q = 256 hi + lo.  A row is bound by latency (128 rows of 28672 are 7 MB of L2 traffic), so up to WORDS
-// 16-byte words a thread are read once, all in flight together, and kept (128 rows of 8192 and of 28672 after one another in a step: 13.6 us by two passes of dependent loads, 6.2 so);
-// WORDS 0: rows that are longer or not whole aligned words, read twice.
+// 16-byte words a thread are read once, all in flight together, and kept (128 rows of 8192 and of 28672 after one another in a step: 13.6 us by two passes of dependent loads, 6.2 so).
+// Longer rows (WORDS 8 only) go by trips of WORDS words, the last of which is still there when the step is known and the others are read again.
+// WORDS 0: rows that are not whole aligned words, element by element and twice.
 constexpr int kQuantThreads = 512;
 template <typename XT, int WORDS>
 __global__ void __launch_bounds__(kQuantThreads) QuantizeRowsI8Kernel(const XT* x, int8_t* __restrict__ hi, int8_t* __restrict__ lo,
@@ -105,17 +106,24 @@ __global__ void __launch_bounds__(kQuantThreads) QuantizeRowsI8Kernel(const XT* 
     amax = fmaxf(amax, a);
   };
   uint4 u[WORDS > 0 ? WORDS : 1];
-  if constexpr (WORDS > 0) {
+  constexpr int kTrip = WORDS * kQuantThreads * kVec;  // elements
+  const int last = WORDS == 8 ? (K - 1) / kTrip * kTrip : 0;  // where the last trip begins
+  auto load = [&](int from) {
 #pragma unroll
     for (int w = 0; w < WORDS; ++w) {
-      const int i = (tid + w * kQuantThreads) * kVec;
+      const int i = from + (tid + w * kQuantThreads) * kVec;
       u[w] = i < K ? *reinterpret_cast<const uint4*>(row + i) : make_uint4(0u, 0u, 0u, 0u);
     }
+  };
+  if constexpr (WORDS > 0) {
+    for (int from = 0; from <= last; from += kTrip) {
+      load(from);
 #pragma unroll
-    for (int w = 0; w < WORDS; ++w) {
-      const XT* e = reinterpret_cast<const XT*>(&u[w]);
+      for (int w = 0; w < WORDS; ++w) {
+        const XT* e = reinterpret_cast<const XT*>(&u[w]);
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) see(AsBf16Value<XT>(e[j]));
+        for (int j = 0; j < kVec; ++j) see(AsBf16Value<XT>(e[j]));
+      }
     }
   } else {
     for (int i = tid; i < K; i += kQuantThreads) see(AsBf16Value<XT>(row[i]));
@@ -144,22 +152,25 @@ __global__ void __launch_bounds__(kQuantThreads) QuantizeRowsI8Kernel(const XT* 
   int8_t* hrow = hi + static_cast<size_t>(m) * K;
   int8_t* lrow = lo + static_cast<size_t>(m) * K;
   if constexpr (WORDS > 0) {
+    for (int from = last; from >= 0; from -= kTrip) {
+      if (from != last) load(from);
 #pragma unroll
-    for (int w = 0; w < WORDS; ++w) {
-      const int i = (tid + w * kQuantThreads) * kVec;
-      if (i >= K) break;
-      const XT* e = reinterpret_cast<const XT*>(&u[w]);
-      uint32_t h[kVec / 4], l[kVec / 4];
+      for (int w = 0; w < WORDS; ++w) {
+        const int i = from + (tid + w * kQuantThreads) * kVec;
+        if (i >= K) break;
+        const XT* e = reinterpret_cast<const XT*>(&u[w]);
+        uint32_t h[kVec / 4], l[kVec / 4];
 #pragma unroll
-      for (int j = 0; j < kVec; j += 4) {
-        I8Split4(AsBf16Value<XT>(e[j]), AsBf16Value<XT>(e[j + 1]), AsBf16Value<XT>(e[j + 2]), AsBf16Value<XT>(e[j + 3]), inv, h[j / 4], l[j / 4]);
-      }
-      if constexpr (kVec == 8) {
-        *reinterpret_cast<uint2*>(hrow + i) = make_uint2(h[0], h[1]);
-        *reinterpret_cast<uint2*>(lrow + i) = make_uint2(l[0], l[1]);
-      } else {
-        *reinterpret_cast<uint32_t*>(hrow + i) = h[0];
-        *reinterpret_cast<uint32_t*>(lrow + i) = l[0];
+        for (int j = 0; j < kVec; j += 4) {
+          I8Split4(AsBf16Value<XT>(e[j]), AsBf16Value<XT>(e[j + 1]), AsBf16Value<XT>(e[j + 2]), AsBf16Value<XT>(e[j + 3]), inv, h[j / 4], l[j / 4]);
+        }
+        if constexpr (kVec == 8) {
+          *reinterpret_cast<uint2*>(hrow + i) = make_uint2(h[0], h[1]);
+          *reinterpret_cast<uint2*>(lrow + i) = make_uint2(l[0], l[1]);
+        } else {
+          *reinterpret_cast<uint32_t*>(hrow + i) = h[0];
+          *reinterpret_cast<uint32_t*>(lrow + i) = l[0];
+        }
       }
     }
   } else {
@@ -594,10 +605,10 @@ cudaError_t LaunchQuantize(const XT* x, int8_t* planes, int m, int k, cudaStream
   float* row_scale = reinterpret_cast<float*>(lo + static_cast<size_t>(m) * k);
   constexpr int kVec = 16 / sizeof(XT);
   const int words = (k + kQuantThreads * kVec - 1) / (kQuantThreads * kVec);
-  auto kernel = k % kVec != 0 || !Aligned16(x) || words > 8 ? QuantizeRowsI8Kernel<XT, 0>
-                : words <= 2                                ? QuantizeRowsI8Kernel<XT, 2>
-                : words <= 4                                ? QuantizeRowsI8Kernel<XT, 4>
-                                                            : QuantizeRowsI8Kernel<XT, 8>;
+  auto kernel = k % kVec != 0 || !Aligned16(x) ? QuantizeRowsI8Kernel<XT, 0>
+                : words <= 2                 ? QuantizeRowsI8Kernel<XT, 2>
+                : words <= 4                 ? QuantizeRowsI8Kernel<XT, 4>
+                                             : QuantizeRowsI8Kernel<XT, 8>;
   return LaunchChained(kernel, static_cast<unsigned>(m), kQuantThreads, 0, st, x, hi, lo, row_scale, k);
 }
 
