@@ -7,7 +7,7 @@
 //                    128 output columns and one slice of K; each of its four warps is an independent cp.async
 //                    pipeline over its own 32-row stages (a 32 x 128 int8 weight tile plus the matching 32-wide
 //                    strip of the bf16 activations, XOR-swizzled in shared memory), so there is no CTA-wide barrier
-//                    in the loop and six CTAs fit an SM.  The MMA runs transposed: the 16 output columns a lane
+//                    in the loop and five CTAs fit an SM (one n-tile).  The MMA runs transposed: the 16 output columns a lane
 //                    pair-set owns are the M dimension and the (<= 8 per n-tile) activation rows the N dimension, so
 //                    one 16-row step costs 8 mma.sync m16n8k16 per n-tile.  The int8 codes become exact bf16 pairs in
 //                    registers (one byte-permute, two logic ops and one packed bf16 add per pair); products are
@@ -18,7 +18,7 @@
 //                    Bound at one row by the issue of the conversion (ncu, 4096 x 28672: ALU pipe 57 %, issue slots 50 % busy, 3.3 warps a scheduler)
 //                    and by the SMs that idle at its ends (22 % of the time).  4096 x 28672 with a norm in front: 34.3 us with two slices and a division
 //                    per stage for the ring's place, 31.0 with three slices, 30.1 with places and sources that move on by themselves, 29.0 with the ranks' sums in flight together,
-//                    27.1 with two stages a warp and six CTAs an SM in place of three and four.
+//                    27.1 with two stages a warp and five CTAs an SM in place of three and four.
 //   GemmExactKernel  the interpreter's MATMUL order (DxirInterpreter.kt:739-765): f32, k ascending, separate
 //                    multiply and add, zero activations skipped.  Bit-identical to the CPU oracle; slow.
 #include <cooperative_groups.h>
@@ -95,10 +95,9 @@ __device__ __forceinline__ uint32_t CodesToBf16x2(uint32_t w_lo_k, uint32_t w_hi
   return r;
 }
 
-// NT: n-tiles of eight activation rows.  S: stages of a warp.  Two are 37 KB a CTA, six an SM: where CTAs are many, more warps to hide the conversion behind are
-// worth more than a third stage (4096 x 28672 29.0 -> 27.1 us, 6144 10.5 -> 9.9); with one CTA an SM the loads in flight are (9 rows, 8192 x 1024 10.1, 10.3).
-// With 9 rows and more a stage's MMAs and strip are twice as many and three stages are better again (three layers of 6144 + 4096 + 28672 x 4096, 4096 x 14336 and a head,
-// 9, 12 and 16 rows: 359, 353, 376 us with two, 340, 343, 358 with three), but for short slices whose CTAs would then take a second wave (16 rows, 2048 x 8192 in eight slices: 11.7 and 17.4).
+// NT: n-tiles of eight activation rows.  S: stages of a warp.  Registers allow five CTAs an SM with one n-tile (96 a thread) and four with two (126); three stages leave room in
+// shared memory for four and three.  (Six CTAs, by a bound of 80 registers and 16 bytes of spills: 4096 x 14336 at one row 16.4 -> 20.0 us, 4096 x 4096 6.6 -> 7.0.)
+// LaunchGemv says which is taken where.
 template <int NT, int S>
 struct GvLayout {
   static constexpr int kRows = NT * 8;                     // activation rows a launch covers
@@ -424,18 +423,30 @@ template <int NT, typename YT>
 cudaError_t LaunchGemv(const GemmParams& p, cudaStream_t stream)
 {
   const int ctas = (p.N + kGvCols - 1) / kGvCols * p.ks;
-  const int length = ((p.K + p.ks - 1) / p.ks + kGvStageK * kGvWarps - 1) / (kGvStageK * kGvWarps);  // stages of a warp's way through its slice
-  return ctas <= kSms || (NT > 1 && (ctas <= 3 * kSms || length >= 8)) ? LaunchGemvStages<NT, 3, YT>(p, stream) : LaunchGemvStages<NT, 2, YT>(p, stream);
+  const int slice = (p.K + p.ks - 1) / p.ks;
+  constexpr int kUnit = kGvStageK * kGvWarps;
+  // Three stages where a third hides more than a fifth (NT 2: a fourth) CTA an SM would, us with two and three:
+  //   NT 1  one CTA an SM: 1 row of 8192 x 1024 6.6, 6.2.  A full SM of long slices: 4096 x 32768 (512 CTAs of 2048 k) 29.9, 25.0, 28672 x 8192 50.2, 41.3, either the
+  //         same behind a norm.  Not shorter ones: 2048 x 8192 (512 of 256 k) behind a norm 7.8, 8.9; nor between: 5120 x 5120 (320) 8.6, 9.9; nor more CTAs: 4096 x 28672 (672) 22.5, 24.8.
+  //   NT 2  up to what three CTAs an SM hold in one wave of clusters: 9 rows of 4096 x 6144 (384) 10.7, 9.4, 5120 x 5120 (320) 12.2, 10.5, a step of 12 rows through three 8B-shape layers
+  //         403, 390; but 2560 x 11008 in 430 11.0, 13.8, 28672 x 8192 in 512 49.2, 60.8, 12 rows through two 70B-shape layers 594 with three there, 551 with two.
+  //         Far more CTAs of long slices again: the same 8B-shape step, its 4096 x 28672 (672 of 1366 k) with two 399, with three 389.
+  const bool three = NT == 1 ? ctas <= kSms || (ctas > 3 * kSms && ctas <= 4 * kSms && slice >= 16 * kUnit)
+                             : 5 * ctas <= 13 * kSms || (ctas > 4 * kSms && slice >= 10 * kUnit);
+  return three ? LaunchGemvStages<NT, 3, YT>(p, stream) : LaunchGemvStages<NT, 2, YT>(p, stream);
 }
 
-// K slices for a shape, one to eight (the portable cluster sizes; not seven, which came out slower than six and eight wherever measured), each of at least one stage a warp.  What counts is how evenly the CTAs fall on the 148 SMs
-// and that there are about three an SM, so that loads in flight cover the way to HBM, and how much of the longest slice the average one has; more slices
+// K slices for a shape, one to eight (the portable cluster sizes; not seven, which came out slower than six and eight wherever measured).  What counts is how evenly
+// the CTAs fall on the 148 SMs and that there are about three an SM, so that loads in flight cover the way to HBM, and how much of the longest slice the average one has; more slices
 // than that have to be worth a seventh.  Columns that are cut
 // evenly over all SMs instead (112 or 96 a CTA) lose more to rows of codes that start within a 128-byte line than the last wave costs.
 // Microseconds at one row with a norm in front, slices 2 / 3 / 4 of 4096 x 28672: 30.1 / 27.4 / 30.5; 4 / 5 / 6 of 5120 x 14336: 21.2 / 19.0 / 20.0;
-// 4 / 6 / 8 of 14336 x 4096: 20.9 / 19.8 / 16.5.
+// 4 / 6 / 8 of 14336 x 4096: 20.9 / 19.8 / 16.5.  Not taken are
+//   a slice without rows (2560 in eight is seven of 384: 2560 x 8192 at one row 8.5, 7.0 in four),
+//   beyond two CTAs an SM a slice of less than four stages a warp, whose beginning and end outweigh it (2048 x 8192 at 8 rows 8.0 in eight, 7.1 in four), unless k has no more to begin with,
+//   a second wave (five CTAs an SM up to 8 rows, four from 9 on) of less than nine (4096 x 11008 in eight: 1 row 11.0, 9 rows 17.1, in six 13.6, 14.4).
 // $TLALOC_B200_GEMV_KS overrides.
-int ChooseSlices(int k, int n)
+int ChooseSlices(int k, int n, int rows)
 {
   static const int forced = [] {
     const char* e = std::getenv("TLALOC_B200_GEMV_KS");
@@ -451,6 +462,9 @@ int ChooseSlices(int k, int n)
     if (ks == 7) continue;
     const int items = tiles * ks, share = (items + kSms - 1) / kSms;
     const int unit = kGvStageK * kGvWarps, slice = ((k + ks - 1) / ks + unit - 1) / unit * unit;
+    if (ks > 1 && slice * (ks - 1) >= k) continue;
+    if (ks > 1 && items > 2 * kSms && slice < 4 * unit && k >= 4 * unit) continue;
+    if (ks > 1 && items > (rows > 8 ? 4 : 5) * kSms && slice <= 8 * unit) continue;
     const double score = static_cast<double>(items) / (share * kSms) * std::min(1.0, static_cast<double>(items) / kWanted) * k / (static_cast<double>(ks) * slice);
     if (score > best_score * (tiles * best < kWanted ? 1.08 : 1.15)) {
       best_score = score;
@@ -599,7 +613,7 @@ extern "C" int tlaloc_b200_int8_gemm(const void* x, int32_t x_dtype, const int8_
   p.scales = scales;
   p.K = k;
   p.N = n;
-  p.ks = ChooseSlices(k, n);
+  p.ks = ChooseSlices(k, n, m);
   p.weights_const = (flags & TLALOC_B200_GEMM_WEIGHTS_CONST) != 0 ? 1 : 0;
   const int per = (k + p.ks - 1) / p.ks;
   const int unit = kGvStageK * kGvWarps;
