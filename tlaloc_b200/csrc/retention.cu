@@ -230,11 +230,11 @@ extern "C" int tlaloc_b200_retention_step(const float* in, int64_t ld, const int
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int vp = (vdim + 3) / 4 * 4;
   // Ranks: where heads and rows alone leave SMs idle, as long as each has at least 32 columns (a whole 128-byte line of a state row) and 32 KB of state;
-  // a CTA's beginning and the cluster's meeting cost about as much as that.  Microseconds with one rank and split, head x dim x vdim of rows:
+  // a CTA's beginning and the cluster's meeting cost about as much as that, and heads of less than 96 KB have nothing to gain (8 heads of 128 x 128, 15 rows: 4.6 us, 5.9 in two).  Microseconds with one rank and split, head x dim x vdim of rows:
   // 8 x 256 x 512 of 15 31.0 -> 25.6 (two ranks) and 35 (eight), of 1 21.4 -> 6.6; 16 x 128 x 256 of 1 7.8 -> 5.2; 20 x 64 x 128 of 3 4.1 -> 4.9 (not split).
   const size_t bytes = sizeof(float) * dim * vp;
   int ranks = 1;
-  while (ranks < kMostRanks && static_cast<long long>(heads) * rows * ranks < kWantedCtas && vp / (2 * ranks) >= 32 && bytes / (2 * ranks) >= 32 * 1024) ranks *= 2;
+  while (bytes >= 96 * 1024 && ranks < kMostRanks && static_cast<long long>(heads) * rows * ranks < kWantedCtas && vp / (2 * ranks) >= 32 && bytes / (2 * ranks) >= 32 * 1024) ranks *= 2;
   const int cols = (vp / 4 + ranks - 1) / ranks;
   const bool deep = dim > kThreads / cols * kAhead && static_cast<long long>(heads) * rows * ranks <= 2 * 148;  // two places an SM are enough
   const size_t smem = sizeof(float) * (2 * ((dim + 3) / 4 * 4) + 4 * static_cast<size_t>(kThreads));
