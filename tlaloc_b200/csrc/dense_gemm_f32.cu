@@ -509,17 +509,33 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int q = 0; q < 3; ++q) TcSt4(w_to + ((it & 1) != 0 ? L::PlaneColumn(1, q) : L::PlaneColumn(0, q)), part[q]);
         }
+        if constexpr (BT <= 64) {
+          // Few rows: half a group a warp, so that all sixteen have some (64 rows, n 32768, k 2048: 127.6 us with whole groups for half of the warps, 124.4 so; one row 105.7, 102.3). A
+          // lane has four k, and the two rows of sixteen lanes lie in different halves of their lines.
+          const int row = (sw >> 1) * 8 + 2 * (sw & 1) + ((lane & 8) >> 1) + (lane >> 4), word = lane & 7;
+          if ((sw >> 1) < groups) {
+            uint64_t v[2];
+            uint32_t part[3][2];
+            asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v[0]), "=l"(v[1]) : "r"(base + L::kRaw + s * L::kStage + (kBN + row) * 128 + ((word ^ (row & 7)) << 4)));
 #pragma unroll
-        for (int i = 0; i < BT / 8; i += kSplitWarps) {
-          const int g = i + sw;
-          if (g >= groups) break;
-          uint32_t part[3][4];
-          split(from + g * 1024, part);
+            for (int e = 0; e < 2; ++e) Split2(v[e], part[0][e], part[1][e], part[2][e]);
+            const uint32_t at = (base + row * 128 + (((word >> 1) ^ (row & 7)) << 4) + (word & 1) * 8) ^ ((it & 1) << 6);
 #pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(to + g * 1024 + q * L::kPlane), "r"(part[q][0]), "r"(part[q][1]),
-                         "r"(part[q][2]), "r"(part[q][3])
-                         : "memory");
+            for (int q = 0; q < 3; ++q) asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(at + q * L::kPlane), "r"(part[q][0]), "r"(part[q][1]) : "memory");
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < BT / 8; i += kSplitWarps) {
+            const int g = i + sw;
+            if (g >= groups) break;
+            uint32_t part[3][4];
+            split(from + g * 1024, part);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(to + g * 1024 + q * L::kPlane), "r"(part[q][0]), "r"(part[q][1]),
+                           "r"(part[q][2]), "r"(part[q][3])
+                           : "memory");
+            }
           }
         }
         asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
