@@ -1,4 +1,4 @@
-"""Attention over grouped heads in grids of more CTAs than SMs, where large groups' keys and values travel on their own (three halves, or two of each), against f64."""
+"""Attention over grouped heads in grids of more CTAs than SMs, where large groups' keys and values travel on their own (three halves, or two of each) and others as one, against f64."""
 import pytest
 import torch
 
@@ -17,9 +17,10 @@ def no_wait_runs_out():
     assert _native.lib().tlaloc_b200_device_status() == 0
 
 
-# heads of queries (with maps), value heads, maps, dim, vdim: halves of 8 + 8 KB, of 4 + 8 (two maps of 64, one of 128), 8 + 4, 4 + 6, 2 + 8 (too small: whole groups)
+# heads of queries (with maps), value heads, maps, dim, vdim.  Keys and values on their own: 8 + 8 KB, 8 + 8 of which 240 channels are used, 4 + 8 (two maps of 64, one of 128), 8 + 4,
+# 4 + 6, 2 + 8; whole groups in as large a grid: 4 + 4 (small enough as they are), 8 + 6 (halves of two do not leave room for a second CTA)
 @pytest.mark.parametrize("heads,groups,maps,dim,vdim", [(16, 4, 2, 128, 256), (8, 4, 2, 128, 240), (16, 4, 2, 64, 256), (8, 4, 1, 128, 256), (16, 4, 2, 112, 128), (8, 4, 2, 48, 192),
-                                                        (16, 4, 1, 64, 256)])
+                                                        (16, 4, 1, 64, 256), (16, 4, 2, 64, 128), (16, 4, 2, 128, 192)])
 @pytest.mark.parametrize("window,keep,slices", [(0, 0, 1), (70, 0, 1), (70, 9, 1), (33, 40, 2), (0, 0, 3)])
 def test_more_ctas_than_sms(heads, groups, maps, dim, vdim, window, keep, slices):
     lens = [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 80, 95, 96, 97, 111, 112, 127, 128, 129, 143, 144, 145, 159, 160, 200, 255, 256, 257, 300, 319, 320, 321, 350, 383, 384,
