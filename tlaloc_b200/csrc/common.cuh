@@ -78,11 +78,13 @@ void CountLaunches(int n);
 // the programmatic-serialization attribute and starts with GridDependencySync(): the kernel may be scheduled (and run
 // whatever comes before that call: shared-memory carve-up, mbarrier and TMEM setup) while its predecessor drains, and
 // the call then waits until the predecessor grid has COMPLETED and its writes are visible.  So no global memory is
-// read or written before it, and correctness is exactly that of plain stream order.  The one exception, taken only
-// when the caller states that the weights are constant (TLALOC_B200_GEMM_WEIGHTS_CONST): the projection kernels fetch
-// their first stages of codes ahead of the call, since no kernel in flight can be writing them.  The trigger for the kernel's
-// own successors is issued right after the wait, never before it, so at most one kernel is ever waiting behind a
-// running one.  A launch without the attribute (another library's kernel, $TLALOC_B200_PDL=0) makes the call a no-op.
+// read or written before it, and correctness is exactly that of plain stream order.  The one exception: the projection kernels fetch
+// their first stages of codes (and their scales) ahead of the call where no kernel in flight can be writing them, that is
+//   - the caller states that the weights are constant (TLALOC_B200_GEMM_WEIGHTS_CONST), or
+//   - the kernel right in front is this call's own QuantizeRowsI8Kernel, which writes no weights: a kernel starts only once every CTA of the one before it has
+//     triggered (or ended), the quantizer triggers behind its own wait, and so whatever wrote the codes has completed.
+// The trigger for the kernel's own successors is issued right after the wait, never before it: at most one kernel is ever waiting behind a
+// running one, and the second case above rests on it.  A launch without the attribute (another library's kernel, $TLALOC_B200_PDL=0) makes the call a no-op.
 __device__ __forceinline__ void GridDependencySync()
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");

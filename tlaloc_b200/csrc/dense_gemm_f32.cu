@@ -25,7 +25,7 @@
 // Bound at 208 rows by the split and the six products, which run side by side (203 rows, n 18944, k 2048: 106 us with the weights' planes in shared memory too, where
 // each of the two alone took about 100; 92 us now, the split first: its warps wait for one another's latencies, with 40 registers there is one group of words at a time),
 // at few rows by the way of a chunk through the three kinds of warps (0.8 us each).  203 rows, n 2048, k 10304: 77 us, 1414 us with plain FMAs; one
-// row, n 32768, k 2048: 106 us, 443 us.  Every mbarrier wait is bounded.  Sums computed again: 203 rows, n 18944, k 2048 with one row of NaN 0.26 ms, all
+// row, n 32768, k 2048: 102 us, 443 us.  (72 registers a thread at launch: the 208-row form spills 92 bytes, the two smallest 16; none did with the planes in shared memory but the 64-row form, 8.)  Every mbarrier wait is bounded.  Sums computed again: 203 rows, n 18944, k 2048 with one row of NaN 0.26 ms, all
 // infinite 2.2 ms (DenseGemmTiled 0.85 ms); n 2048, k 10304: 0.80, 2.3 (1.4) ms.
 #include <cuda.h>
 
@@ -727,8 +727,8 @@ int ReadF32Status()
 }
 KernelSetup g_setup(PrepareDenseF32, ReadF32Status);
 
-// K slices (1..8) of tiles with k of nb times 64, in microseconds: 64 k take 3.6 us at 208 rows and 1.7 us at
-// few; a tile's start and end cost about 3 us, a cluster's sum 2 us and more with its ranks.
+// K slices (1..8) of tiles with k of nb times 64, in microseconds: 64 k took 3.6 us at 208 rows and 1.7 us at
+// few with all planes in shared memory, which is what the counts were fitted to (2.9 and 1.6 since the weights' are in TMEM); a tile's start and end cost about 3 us, a cluster's sum 2 us and more with its ranks.
 int ChooseSlices(long long tiles, int nb, int bt)
 {
   int device = 0;

@@ -10,7 +10,8 @@
 //                            swizzle) by TMA; no CTA-wide barrier in the loop.  A warp's chain of products and exponentials is what a step takes, so two
 //                            CTAs an SM are worth more than the deeper rings of one; where a group is too large for that (HALVES), its keys and values
 //                            travel on their own, and the keys' place is free again once the scores are there.  64 rows of 4 value heads, two maps of
-//                            128, values of 256 channels, up to 4160 positions: 161 us with one CTA an SM and three groups a warp, 139 with two CTAs and three halves.  Query heads are the rows of mma.m16n8k16; with two maps the
+//                            128, values of 256 channels, up to 4160 positions: 161 us with one CTA an SM and three groups a warp, 139 with two CTAs and three halves.  Registers (255 with values of
+//                            256 channels: 136 to 160 bytes of spills with keys of 128, 28 to 32 with keys of 64) allow no third.  Query heads are the rows of mma.m16n8k16; with two maps the
 //                            rows 0-7 are the heads' first map and 8-15 the second, each multiplied with its own keys, so that one
 //                            product with the values serves both.  The weights enter that product as two bf16 parts (f32 up to rounding).
 //   GroupedAttentionGeneric  any size and type, plain FMA: the f32 path.

@@ -94,7 +94,7 @@ template <typename XT, int WORDS>
 __global__ void __launch_bounds__(kQuantThreads) QuantizeRowsI8Kernel(const XT* x, int8_t* __restrict__ hi, int8_t* __restrict__ lo,
                                                                       float* __restrict__ row_scale, int K)
 {
-  GridDependencySync();
+  GridDependencySync();  // the projection behind this kernel reads its codes as soon as every CTA has passed here: its trigger must not move ahead of its wait
   const int m = blockIdx.x, tid = threadIdx.x;
   const XT* row = x + static_cast<size_t>(m) * K;
   constexpr int kVec = 16 / sizeof(XT);  // elements per 16-byte load

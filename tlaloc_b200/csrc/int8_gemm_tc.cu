@@ -517,8 +517,8 @@ cudaError_t LaunchInt8GemmTc(const __nv_bfloat16* x, const int8_t* codes, const 
     int rows = std::min(256, m - m0);
     if (rows > 128) {
       // Two accumulators share one pass over the weights but cannot split K; with few column tiles two passes of 128
-      // rows, each split over K, keep more SMs busy.  A launch more is five blocks beside what a CTA's fixed cost says (200 rows x 1024 x 4096: 20.4 us
-      // in one pass, 23.5 in two of four slices; x 2048 x 4096: 24 in two).
+      // rows, each split over K, keep more SMs busy.  Each of the two launches is charged five blocks beside what a CTA's fixed cost says, the second launch ten in all (200 rows
+      // x 1024 x 4096: 20.4 us in one pass, 23.5 in two of four slices; x 2048 x 4096: 24 in two).
       double c256 = 0.0, c128 = 0.0;
       ChooseTcSlices(k, n, 128, &c128);
       ChooseTcSlices(k, n, 256, &c256);
