@@ -90,8 +90,9 @@ __device__ __forceinline__ float2 Rotate(float u, float v, float c, float s)
 
 // One CTA per token: two norms, one rotation, one cache row.  VEC: q_rank up to 2048, kv_rank up to 1024, both and rot_dim multiples of 4, and everything
 // aligned: the row is read once, by 16-byte words.  2048 tokens of 1536 + 576 values: 11.1 us element by element (bound by their instructions), 6.4 so.
+// Element by element the registers are bound, so that an SM holds eight CTAs: 2048 tokens of 2052 + 72 values 12.4 us with six, 10.5 with eight (700 tokens 5.7, 6.3).
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256) LatentKvWriteKernel(const float* in, int64_t ld, const float* q_gain, const float* kv_gain, float eps,
+__global__ void __launch_bounds__(256, VEC ? 4 : 8) LatentKvWriteKernel(const float* in, int64_t ld, const float* q_gain, const float* kv_gain, float eps,
                                                            const int* positions, const float* cos_t, const float* sin_t, const int* slots,
                                                            T* cq, T* pool, int64_t pool_ld, int q_rank, int kv_rank, int rot_dim,
                                                            int rot_dims, int num_slots, int max_pos)
