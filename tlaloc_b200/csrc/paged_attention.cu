@@ -1501,8 +1501,8 @@ cudaError_t LaunchGeneric(const PaParams& p, cudaStream_t stream)
   return LaunchChained(PaSliceGeneric<QT, KVT>, dim3(p.grid, p.Hkv, p.Tb), kGenThreads, smem, stream, p);
 }
 
-// Positions per slice of the tensor-core kernels when the scratch allows it, for `pairs` (table, KV head) pairs that see up to `seen` positions each, from the first
-// on or (from_window) from anywhere, which takes a slice more;
+// Positions per slice of the tensor-core kernels when the scratch allows it, for the pairs of `tables` tables and `kv_heads` KV heads, which see up to `seen` positions each, from the first
+// on or (from_window) from anywhere;
 // $TLALOC_B200_PA_SLICE overrides.
 // A CTA pays about 3 us of latency before its first position (lengths and table entries, then the first K/V rows)
 // and again to merge its warps and write its records, so slices should be as long as the grid can afford: 1024
@@ -1516,10 +1516,13 @@ cudaError_t LaunchGeneric(const PaParams& p, cudaStream_t stream)
 // Halving pays where it fills the wave; microseconds at 256 / 512 / 1024, lengths spread up to the context:
 //   few pairs       8 pairs of 4000 11.4 / 12.7 / 17.8; 64 of 2000 14.5 / 15.0 / 18.8, of 4000 24.5 / 20.0 / 22.0
 //   48 slices       the merge walks a row's records in one warp, eight at a time: one row of 16000 with 8 KV heads 28.8 / 20.5 / 20.5, of 60000 with one KV head 41.0 / 27.2 / 25.1
-//   past the wave   a second one has to be short and full: 16 pairs of 8191 22.6 / 18.1 / 19.0, of 16000 38.4 / 35.0 / 27.9; e4m3fn rather has it, 64 pairs of 8191 31.3 / 25.0 / 33.4,
-//                   but not for a remainder: 500 pairs of 701 17.8 / 21.8 / 17.0
+//   past the wave   one sequence may fill its table, and then a second wave has to be short: 16 KV heads of one row of 8191 22.6 / 18.1 / 19.0, of 16000 38.4 / 35.0 / 27.9.  Lengths of
+//                   several differ, and less than all CTAs live (32 rows of up to 1500 in tables of 12032, one KV head: - / 15.7 / 19.5); e4m3fn has the second wave anyway, 64 pairs of
+//                   8191 31.3 / 25.0 / 33.4.  Neither for a remainder: 500 pairs of 701 17.8 / 21.8 / 17.0
+//   windows         reach into a slice more than their length says, and most rows' are full: counted with it, as one sequence's (64 pairs of 4096 in 16000: - / 36.9 / 30.5).  e4m3fn without:
+//                   500 pairs of 1000 in 2000 - / 26.4 / 33.1
 //   short contexts  a slice of 512 or less is hardly shorter by halves: 256 pairs of 300 14.0 / 12.9 / 13.1; with an SM for every CTA all the same, 8 pairs 8.7 / 9.4 / 9.4
-int PreferredSlice(int seen, bool from_window, long long pairs, bool f8)
+int PreferredSlice(int seen, bool from_window, int tables, int kv_heads, bool f8)
 {
   static const int forced = [] {
     const char* e = std::getenv("TLALOC_B200_PA_SLICE");
@@ -1529,13 +1532,13 @@ int PreferredSlice(int seen, bool from_window, long long pairs, bool f8)
   if (forced > 0) return forced;
   int slice = 1024;
   const int wave = f8 ? 592 : 444;
-  auto count = [&](int length) { return from_window ? (seen + length - 2) / length + 1 : (seen + length - 1) / length; };
-  auto ctas = [&](int length) { return pairs * count(length); };
+  auto count = [&](int length) { return from_window && !f8 ? (seen + length - 2) / length + 1 : (seen + length - 1) / length; };
+  auto ctas = [&](int length) { return static_cast<long long>(tables) * kv_heads * count(length); };
   auto worth_halving = [&](int half) {
     if (count(half) > 48) return false;
     if (seen <= 512 && ctas(half) > 148) return false;
     if (8 * ctas(half) <= 9 * wave) return true;
-    return (f8 || count(half) <= 8) && 4ll * count(half) * half <= 5ll * seen;
+    return (f8 || (tables > 1 && !from_window) || count(half) <= 8) && 4ll * count(half) * half <= 5ll * seen;
   };
   while (slice < 4096 && ctas(2 * slice) >= (f8 ? 5000 : 2048)) slice *= 2;
   while (slice > 256 && ctas(slice) < wave && worth_halving(slice / 2)) slice /= 2;
@@ -1706,7 +1709,7 @@ extern "C" int tlaloc_b200_paged_attention(const void* query, int32_t q_dtype, c
   // Slice length: the preferred one (tensor-core kernel) or 256, stretched until `splits` slices cover the context.
   const bool from_window = sliding_window > 0 && sliding_window < ctx && p.rpt == 1;  // rows that share a table have windows in different places: all slices are launched for them
   const int seen = from_window ? sliding_window : ctx;
-  int slice = mma ? PreferredSlice(seen, from_window, static_cast<long long>(num_tables) * num_kv_heads, f8) : 256;
+  int slice = mma ? PreferredSlice(seen, from_window, num_tables, num_kv_heads, f8) : 256;
   if (static_cast<int64_t>(slice) * splits < ctx) slice = (ctx + splits - 1) / splits;
   if (mma) slice = std::min((slice + 15) / 16 * 16, 8192);
   if (static_cast<int64_t>(slice) * splits < ctx) {
